@@ -67,4 +67,12 @@ static __device__ __forceinline__ void nb_axial_setup(const nb_ray &R, float atn
   }
 }
 
+// The first plane boundary (0 .. 127) an oblique ray of ring pair R reaches on its way up from
+// the LOR's entry point tp.
+static __device__ __forceinline__ int nb_first_plane(const nb_ray &R, float atn, float tp) {
+  const float az_atn = __fdiv_rn(__fsub_rn(R.r1z, R.r0z), atn);
+  const float pz = __double2float_rn(__dadd_rn((double)R.r0z, 0.5 * (double)NB_RING));
+  return (int)ceilf(nb_zpos(__fmaf_rn(az_atn, tp, pz)));
+}
+
 static __device__ __forceinline__ int nb_clampz(int w) { return w < 0 ? 0 : (w > 127 ? 127 : w); }

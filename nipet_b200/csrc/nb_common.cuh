@@ -19,6 +19,7 @@
 #define NB_NSN11 837
 #define NB_SEG0 127
 #define NB_NCRS 504
+#define NB_MAXRD 60 // largest ring difference
 #define NB_IMX 320
 #define NB_IMY 320
 #define NB_IMZ 127

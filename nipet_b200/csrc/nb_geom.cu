@@ -16,7 +16,6 @@
 
 #include "nb_axial.cuh"
 #include "nb_internal.cuh"
-#include "nb_project.cuh"
 
 // ---------------------------------------------------------------------------------------
 // One thread per LOR: tt[10] and the crossing sequence tv[1807] (reference layout).
@@ -193,20 +192,159 @@ __global__ void k_expand_steps(const float *__restrict__ tt, const unsigned char
   hdr[idx] = make_float4(t[5], t[7], t[6], __int_as_float(n));
 }
 
-// longest walk segment (tn - tp) of every LOR, as float bits (segments are >= 0)
-__global__ void k_maxseg(const float4 *__restrict__ hdr, const float *__restrict__ st, int naw,
-                         unsigned *out) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= naw) return;
-  const float4 h = hdr[idx];
+// Walks every ray of every LOR once at geometry creation and counts axial positions outside
+// [0, 127]: the projector indexes shared memory by the plane without clamping.  z = 127 is one
+// plane above the image; it maps to a column's zero padding slot (reads 0, back projections
+// into it are discarded).  In the mMR geometry exactly one ray step reaches it (the last step
+// of rings 59->63 on LOR 24839).  One block per LOR.
+__global__ void k_check_walk(const float4 *__restrict__ hdr, const float *__restrict__ st,
+                             const nb_ray *__restrict__ rays, int naw, int *bad) {
+  const int lor = blockIdx.x;
+  if (lor >= naw) return;
+  const float4 h = hdr[lor];
   const int n = __float_as_int(h.w);
-  float tp = h.x, m = 0.f;
-  for (int k = 0; k < n; k++) {
-    const float tn = st[(size_t)idx * NB_STEP_STRIDE + k];
-    m = fmaxf(m, fabsf(__fsub_rn(tn, tp)));
-    tp = tn;
+  int nbad = 0;
+  for (int ray = threadIdx.x; ray < NB_NRAYS; ray += blockDim.x) {
+    nb_axial A;
+    nb_axial_setup(rays[ray], h.y, h.x, h.z, A);
+    int w = A.w;
+    float tzc = A.tzc;
+    if (w < 0 || w > NB_IMZ) nbad++;
+    for (int k = 0; k < n; k++) {
+      if (st[(size_t)lor * NB_STEP_STRIDE + k] > tzc) {
+        w += A.dir;
+        tzc = __fadd_rn(tzc, A.dtz);
+        if (w < 0 || w > NB_IMZ) nbad++;
+      }
+    }
   }
-  atomicMax(out, __float_as_uint(m));
+  if (nbad) atomicAdd(bad, nbad);
+}
+
+// ---------------------------------------------------------------------------------------
+// Crossing schedules (layout: nb_internal.cuh).  Rays of one ring difference d start two
+// planes apart per ring and their crossing parameters are the same floats (ring positions and
+// planes are exact multiples of 13/128 cm), so one ray of a difference stands for all: the
+// schedule is that ray's own walk (prjf.cu:164-190: at most one crossing a step, the crossing
+// parameter advanced by float additions).  What differs between the rays of a difference is
+// the start plane where it rounds across a plane boundary (~700 of 2.8e8 rays); those are
+// listed with their offset.  A first boundary that rounds to the next one is the same walk
+// with a segment of ~1e-6 cm moved between neighbouring planes, so only the start plane at the
+// group's own first crossing matters.
+//
+// One block of 64 threads per LOR, thread d for difference d.  FILL = false counts: sizes[lor]
+// in 16-byte units; FILL = true writes the records.  err: a schedule or list over capacity.
+// ---------------------------------------------------------------------------------------
+static __device__ __forceinline__ nb_ray ring_pair(int r0, int d, int kind) {
+  nb_ray R;
+  R.r0z = __fmul_rn((float)(r0 - NB_NRINGS / 2), NB_RING);
+  R.r1z = __fmul_rn((float)(r0 + d - NB_NRINGS / 2), NB_RING);
+  R.kind = (int8_t)kind;
+  return R;
+}
+
+template <bool FILL>
+__global__ void k_sched(const float4 *__restrict__ hdr, const float *__restrict__ st,
+                        uint32_t *__restrict__ sizes, const uint32_t *__restrict__ rec_off,
+                        unsigned char *__restrict__ rec, int *err) {
+  const int lor = blockIdx.x, d = threadIdx.x;
+  __shared__ int scnt[64], soff[64], nirr, big;
+  const float4 h = hdr[lor];
+  const int n = __float_as_int(h.w);
+  const float *t = st + (size_t)lor * NB_STEP_STRIDE;
+  unsigned char *out = FILL ? rec + (size_t)rec_off[lor] * 16 : nullptr;
+  if (d == 0) nirr = big = 0;
+  int m = 1, rc = 0;
+  const bool live = d >= 1 && d <= NB_MAXRD && n > 0;
+  if (live) {
+    // the first boundary (relative to 2 r0) that most rays of the difference have
+    int lo = 1 << 20, clo = 0, rlo = 0, rhi = 0;
+    for (int r0 = 0; r0 + d < NB_NRINGS; r0++) {
+      const int k = nb_first_plane(ring_pair(r0, d, 1), h.y, h.x) - 2 * r0;
+      if (k < lo) {
+        rhi = rlo;
+        lo = k;
+        clo = 0;
+        rlo = r0;
+      } else if (k > lo) {
+        rhi = r0;
+      }
+      clo += k == lo;
+    }
+    const bool up = 2 * clo < NB_NRINGS - d;   // the other value is in the majority
+    rc = up ? rhi : rlo;
+    m = nb_first_plane(ring_pair(rc, d, 1), h.y, h.x) - 2 * rc;
+  }
+  nb_axial A;
+  A.tzc = A.dtz = 0.f;
+  if (live) nb_axial_setup(ring_pair(rc, d, 1), h.y, h.x, h.z, A);
+  auto walk = [&](bool fill, int base) {
+    int k = 0;
+    float tp = h.x, tzc = A.tzc;
+    for (int s = 0; s < n; s++) {
+      const float tn = t[s];
+      if (live && tn > tzc) {
+        if (fill) {
+          const float lt = __fsub_rn(tn, tp);
+          const float f = lt > 0.f ? __fdiv_rn(__fsub_rn(tzc, tp), lt) : 0.f;
+          if (fabsf(f) > 1.f) big = 1;
+          *reinterpret_cast<uint2 *>(out + NB_REC_ENT + 8 * (size_t)(base + k)) =
+              make_uint2((uint32_t)s, __float_as_uint(f));
+        }
+        k++;
+        tzc = __fadd_rn(tzc, A.dtz);
+      }
+      tp = tn;
+      if (fill && ((s & 7) == 7 || s == n - 1)) out[NB_REC_KEND + (s >> 3) * 64 + d] = (uint8_t)k;
+    }
+    if (fill)
+      for (int r = (n + 7) >> 3; r < NB_STEP_STRIDE / 8; r++)
+        out[NB_REC_KEND + r * 64 + d] = (uint8_t)k;
+    return k;
+  };
+  scnt[d] = walk(false, 0);
+  __syncthreads();
+  if (d == 0) {
+    int tot = 0;
+    for (int x = 0; x < 64; x++) {
+      soff[x] = tot;
+      tot += scnt[x];
+      if (scnt[x] > 255) atomicOr(err, 1);
+    }
+    if (tot > NB_REC_MAXENT) atomicOr(err, 1);
+    if (!FILL) sizes[lor] = (uint32_t)(NB_REC_ENT + ((tot + 1) & ~1) * 8) / 16;
+  }
+  __syncthreads();
+  if (!FILL) return;
+  walk(true, soff[d]);
+  out[NB_REC_M + d] = (uint8_t)m;
+  reinterpret_cast<uint16_t *>(out + NB_REC_OFF)[d] = (uint16_t)soff[d];
+  if (live && (m < 1 || m > 255)) atomicOr(err, 1);
+  if (live)
+    for (int r0 = 0; r0 + d < NB_NRINGS; r0++) {
+      nb_axial U, D;
+      nb_axial_setup(ring_pair(r0, d, 1), h.y, h.x, h.z, U);
+      nb_axial_setup(ring_pair(r0, d, 2), h.y, h.x, h.z, D);
+      // start planes at the group's own first crossing: one that is reached earlier (later)
+      // than the group's has moved the ray one plane on (back) by then
+      const int k = nb_first_plane(ring_pair(r0, d, 1), h.y, h.x) - 2 * r0 - m;
+      const int bu = U.w - k - (2 * r0 + m - 1), bd = D.w + k - (2 * (r0 + d) - m + 1);
+      for (int dir = 0; dir < 2; dir++) {
+        const int b = dir ? bd : bu;
+        if (b == 0) continue;
+        if (b < -7 || b > 7) atomicOr(err, 2);
+        const int i = atomicAdd(&nirr, 1);
+        if (i < NB_REC_MAXIRR)
+          reinterpret_cast<uchar4 *>(out + NB_REC_IRR)[i] =
+              make_uchar4((uint8_t)d, (uint8_t)r0, (uint8_t)dir, (uint8_t)(int8_t)b);
+      }
+    }
+  __syncthreads();
+  if (d == 0) {
+    if (nirr > NB_REC_MAXIRR) atomicOr(err, 2);
+    reinterpret_cast<uint16_t *>(out + NB_REC_META)[0] = (uint16_t)nirr;
+    reinterpret_cast<uint16_t *>(out + NB_REC_META)[1] = (uint16_t)big;
+  }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -219,8 +357,10 @@ static void nb_geom_free(nb_geom *g) {
   cudaFree(g->d_hdr);
   cudaFree(g->d_tt);
   cudaFree(g->d_rays);
+  cudaFree(g->d_rec);
+  cudaFree(g->d_rec_off);
+  cudaFree(g->d_slots);
   cudaFree(g->d_bin11);
-  cudaFree(g->d_bin1);
   cudaFree(g->d_scratch128);
   cudaFree(g->d_err);
   cudaFree(g->d_one);
@@ -250,6 +390,66 @@ static int run_tables(nb_geom *g, const float *crs_h, const int16_t *s2c_h, floa
   cudaFree(d_crs);
   cudaFree(d_s2c);
   return st;
+}
+
+// Ring of a ring front edge z (cm): ring i starts at (i - 32) * AXR (mmraux.py:365-370)
+static int ring_of(float z) {
+  const double r = (double)z / (double)NB_RING + 0.5 * NB_NRINGS;
+  const long i = lrint(r);
+  return fabs(r - (double)i) < 1e-4 ? (int)i : -1;
+}
+
+// Slots of a set of rays (those of all ring pairs, or of a reduced range): the direct planes
+// two to a slot, then the pairs by ring difference and ring.  False if the rays are not ring
+// pairs of the mMR's rings with both directions, once each.
+static bool make_slots(const std::vector<nb_ray> &rays, std::vector<nb_slot> &slots) {
+  std::map<std::pair<int, int>, nb_slot> pair;  // (d, r0)
+  std::map<int, const nb_ray *> direct;
+  std::map<std::pair<int, int>, int> seen;
+  for (const nb_ray &R : rays) {
+    const int r0 = ring_of(R.r0z), r1 = ring_of(R.r1z);
+    if (r0 < 0 || r0 >= NB_NRINGS || R.r0z != (float)(r0 - NB_NRINGS / 2) * NB_RING) return false;
+    if (R.kind == 0) {
+      if (direct.count(r0)) return false;
+      direct[r0] = &R;
+      continue;
+    }
+    if (r1 <= r0 || r1 >= NB_NRINGS || r1 - r0 > NB_MAXRD ||
+        R.r1z != (float)(r1 - NB_NRINGS / 2) * NB_RING)
+      return false;
+    const auto key = std::make_pair(r1 - r0, r0);
+    nb_slot &S = pair[key];
+    if (seen[key] & R.kind) return false;
+    seen[key] |= R.kind;
+    S.zA = (int16_t)(2 * r0);
+    S.zB = (int16_t)(2 * r1);
+    S.d = (uint8_t)(r1 - r0);
+    S.pad = 0;
+    (R.kind == 1 ? S.o11A : S.o11B) = R.out11;
+    (R.kind == 1 ? S.o1A : S.o1B) = R.out1;
+    (R.kind == 1 ? S.nosA : S.nosB) = (uint8_t)R.nos;
+  }
+  for (const auto &kv : seen)
+    if (kv.second != 3) return false;
+  std::vector<const nb_ray *> dir;
+  for (const auto &kv : direct) dir.push_back(kv.second);
+  const size_t half = (dir.size() + 1) / 2;
+  slots.clear();
+  for (size_t i = 0; i < half; i++) {
+    nb_slot S{};
+    const nb_ray *A = dir[i], *B = half + i < dir.size() ? dir[half + i] : nullptr;
+    S.zA = (int16_t)(2 * ring_of(A->r0z));
+    S.o11A = A->out11;
+    S.o1A = A->out1;
+    S.nosA = (uint8_t)A->nos;
+    S.zB = B ? (int16_t)(2 * ring_of(B->r0z)) : 0;
+    S.o11B = B ? B->out11 : -1;
+    S.o1B = B ? B->out1 : -1;
+    S.nosB = B ? (uint8_t)B->nos : 1;
+    slots.push_back(S);
+  }
+  for (const auto &kv : pair) slots.push_back(kv.second);
+  return slots.size() <= NB_NSLOT;
 }
 
 extern "C" int nb_geom_create(int device, const float *crs, int ncrs, const int16_t *s2c,
@@ -314,74 +514,31 @@ extern "C" int nb_geom_create(int device, const float *crs, int ncrs, const int1
     }
     rays[r] = R;
   }
-  // Warp-friendly ray order: the kernels give thread t the rays t, t+NT, ... so every
-  // 32-aligned block of ray indices is the lane set of one warp.  Rays of one ring
-  // difference d and direction (a "group", 64-|d| rays) sit 2 voxels apart and cross z
-  // planes at the same steps; a warp drawn from one group reads consecutive shared-memory
-  // banks and takes its crossings together.  Order: every group's first 32 rays (groups
-  // of 32 or more), then warps that pair the rest of group d (32-d rays) with all of group
-  // 64-d (d rays) -- exactly 32, at most two groups per warp -- and last the rest of
-  // groups 1..3, which have no partner.  Any ray not placed by these rules (none for the
-  // mMR's 64 rings and maximum ring difference 60) is appended at the end.
-  {
-    const std::vector<nb_ray> canon = rays;
-    std::map<int, std::vector<int>> grp;  // (kind, d) -> canonical rays in ring order
-    auto key = [&](int r) {
-      return canon[r].kind * 1000 + (int)lrintf((canon[r].r1z - canon[r].r0z) / NB_RING);
-    };
-    for (int r = 0; r < NB_NRAYS; r++) grp[key(r)].push_back(r);
-    std::vector<int> order;
-    std::vector<char> used(NB_NRAYS, 0);
-    auto take = [&](int k, size_t from, size_t to) {
-      auto it = grp.find(k);
-      if (it == grp.end()) return;
-      for (size_t i = from; i < to && i < it->second.size(); i++) {
-        const int r = it->second[i];
-        if (!used[r]) {
-          used[r] = 1;
-          order.push_back(r);
-        }
-      }
-    };
-    auto size_of = [&](int k) -> size_t {
-      auto it = grp.find(k);
-      return it == grp.end() ? 0 : it->second.size();
-    };
-    for (auto &kv : grp)  // full first blocks (direct planes: both of theirs)
-      for (size_t f = 0; f + 32 <= kv.second.size(); f += 32)
-        if (kv.first / 1000 == 0 || f == 0) take(kv.first, f, f + 32);
-    for (int kind = 1; kind <= 2; kind++)
-      for (int d = 4; d <= 31; d++) {
-        const int ka = kind * 1000 + d, kb = kind * 1000 + (64 - d);
-        if (size_of(ka) == (size_t)(64 - d) && size_of(kb) == (size_t)d) {
-          take(ka, 32, size_of(ka));
-          take(kb, 0, size_of(kb));
-        }
-      }
-    for (int kind = 1; kind <= 2; kind++)
-      for (int d = 1; d <= 3; d++) take(kind * 1000 + d, 32, size_of(kind * 1000 + d));
-    for (int r = 0; r < NB_NRAYS; r++)
-      if (!used[r]) order.push_back(r);
-    for (int r = 0; r < NB_NRAYS; r++) rays[r] = canon[order[r]];
+  std::vector<nb_slot> slots;
+  if (!make_slots(rays, slots)) {
+    free(g->h_s2c);
+    free(g);
+    nb_set_error_msg("nb_geom_create: li2rng is not the mMR's ring pairs (ring fronts at "
+                     "(i - 32) * 0.40625 cm, differences 1 .. %d, each pair once)", NB_MAXRD);
+    return NB_ERR_ARG;
   }
-  std::vector<int16_t> bin11(NB_NSN11 * 8, -1), bin1(NB_NSN1, -1);
-  std::vector<int> cnt11(NB_NSN11, 0);
-  for (int r = 0; r < NB_NRAYS; r++) {
-    int o = rays[r].out11;
-    if (cnt11[o] >= 8) {
+  g->nslots = (int)slots.size();
+  std::vector<int16_t> bin11(NB_NSN11 * 8, -1);
+  std::vector<int> cnt11(NB_NSN11, 0), cnt1(NB_NSN1, 0);
+  for (int r = 0; r < 2 * g->nslots; r++) {
+    const nb_slot &S = slots[r / 2];
+    const int o = r & 1 ? S.o11B : S.o11A, o1 = r & 1 ? S.o1B : S.o1A;
+    if (o < 0) continue;
+    if (cnt11[o] >= 8 || cnt1[o1]++) {
       free(g->h_s2c);
       free(g);
-      nb_set_error_msg("nb_geom_create: more than 8 span-1 planes in span-11 sinogram %d", o);
+      if (cnt11[o] >= 8)
+        nb_set_error_msg("nb_geom_create: more than 8 span-1 planes in span-11 sinogram %d", o);
+      else
+        nb_set_error_msg("nb_geom_create: span-1 sinogram %d mapped twice", o1);
       return NB_ERR_ARG;
     }
     bin11[o * 8 + cnt11[o]++] = (int16_t)r;
-    if (bin1[rays[r].out1] != -1) {
-      free(g->h_s2c);
-      free(g);
-      nb_set_error_msg("nb_geom_create: span-1 sinogram %d mapped twice", rays[r].out1);
-      return NB_ERR_ARG;
-    }
-    bin1[rays[r].out1] = (int16_t)r;
   }
 
   int st = NB_OK;
@@ -408,7 +565,8 @@ extern "C" int nb_geom_create(int device, const float *crs, int ncrs, const int1
   ALLOC(g->d_tt, sizeof(float) * NB_N_TT * (size_t)naw);
   ALLOC(g->d_rays, sizeof(nb_ray) * NB_NRAYS);
   ALLOC(g->d_bin11, sizeof(int16_t) * NB_NSN11 * 8);
-  ALLOC(g->d_bin1, sizeof(int16_t) * NB_NSN1);
+  ALLOC(g->d_slots, sizeof(nb_slot) * g->nslots);
+  ALLOC(g->d_rec_off, sizeof(uint32_t) * (naw + 1));
   ALLOC(g->d_scratch128, sizeof(float) * NB_IMG_COL128);
   ALLOC(g->d_err, sizeof(int));
   ALLOC(g->d_one, sizeof(float));
@@ -430,8 +588,8 @@ extern "C" int nb_geom_create(int device, const float *crs, int ncrs, const int1
           cudaSuccess ||
       cudaMemcpy(g->d_bin11, bin11.data(), sizeof(int16_t) * NB_NSN11 * 8,
                  cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(g->d_bin1, bin1.data(), sizeof(int16_t) * NB_NSN1, cudaMemcpyHostToDevice) !=
-          cudaSuccess) {
+      cudaMemcpy(g->d_slots, slots.data(), sizeof(nb_slot) * g->nslots,
+                 cudaMemcpyHostToDevice) != cudaSuccess) {
     st = nb_cuda_fail(cudaGetLastError(), "nb_geom_create upload", __FILE__, __LINE__);
     goto fail;
   }
@@ -451,41 +609,56 @@ extern "C" int nb_geom_create(int device, const float *crs, int ncrs, const int1
       st = NB_ERR_DEVICE;
       goto fail;
     }
-    // Walk checks: every ray stays inside z in [0, 127) (the projector kernels index
-    // shared memory by it) and the longest segment sets the fixed-point headroom of the
-    // back projector (242 overlapping rays per column slot at most).
+    // walk check (the projector indexes shared memory by the plane), then the schedules:
+    // count, place, fill
     cudaMemset(g->d_err, 0, sizeof(int));
-    unsigned *d_seg = (unsigned *)d_tv;  // reuse the table buffer
-    cudaMemset(d_seg, 0, sizeof(unsigned));
-    nbk::k_check_walk<<<naw, 256>>>(g->d_hdr, g->d_st, g->d_rays, naw, g->d_err, d_seg);
-    k_maxseg<<<(naw + 255) / 256, 256>>>(g->d_hdr, g->d_st, naw, d_seg);
-    unsigned segbits = 0;
+    k_check_walk<<<naw, 256>>>(g->d_hdr, g->d_st, g->d_rays, naw, g->d_err);
     int nbad = 0;
     cudaError_t e = cudaMemcpy(&nbad, g->d_err, sizeof(int), cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess) e = cudaMemcpy(&segbits, d_seg, sizeof(unsigned), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) {
-      st = nb_cuda_fail(e, "nb_geom_create walk check", __FILE__, __LINE__);
-      goto fail;
-    }
-    cudaMemset(g->d_err, 0, sizeof(int));
-    if (nbad) {
+    if (e == cudaSuccess && nbad) {
       nb_set_error_msg("nb_geom_create: %d ray positions leave the axial FOV", nbad);
       st = NB_ERR_DATA;
       goto fail;
     }
-    memcpy(&g->maxseg, &segbits, sizeof(float));
-    // maxseg: the largest weight one ray gives one voxel in one step (the longest step, or
-    // a late crossing's |tzc - tp|).  Slot sums stay below 2^31 (242 rays per slot at
-    // most), and every contribution below 2^22, the range in which the back projectors
-    // round w * value to an integer with one fused multiply-add (nb_fx_round).
-    const double seg = g->maxseg > 0.f ? (double)g->maxseg : 1.0;
-    int lb = (int)ceil(log2(242.0 * seg));
-    g->fxbits = 31 - lb;
-    int fm = (int)floor(log2(4194304.0 / seg));
-    while (fm > 0 && ldexp(seg, fm) >= 4194304.0) fm--;
-    if (fm < g->fxbits) g->fxbits = fm;
-    if (g->fxbits < 16) {
-      nb_set_error_msg("nb_geom_create: walk segments too long (%g cm)", (double)g->maxseg);
+    std::vector<uint32_t> off(naw + 1);
+    if (e == cudaSuccess) {
+      k_sched<false><<<naw, 64>>>(g->d_hdr, g->d_st, g->d_rec_off, nullptr, nullptr, g->d_err);
+      e = cudaMemcpy(off.data(), g->d_rec_off, sizeof(uint32_t) * naw, cudaMemcpyDeviceToHost);
+    }
+    if (e == cudaSuccess) {
+      uint64_t tot = 0;  // 16-byte units: 1.2e8 for the mMR
+      for (int i = 0; i <= naw; i++) {
+        const uint32_t sz = i < naw ? off[i] : 0;
+        off[i] = (uint32_t)tot;
+        tot += sz;
+      }
+      if (tot > 0xffffffffull) {
+        nb_set_error_msg("nb_geom_create: crossing schedules too large");
+        st = NB_ERR_DATA;
+        goto fail;
+      }
+      if (cudaMalloc((void **)&g->d_rec, (size_t)tot * 16) != cudaSuccess) {
+        cudaGetLastError();
+        nb_set_error_msg("nb_geom_create: cudaMalloc of %zu bytes failed", (size_t)tot * 16);
+        st = NB_ERR_NOMEM;
+        goto fail;
+      }
+      e = cudaMemset(g->d_rec, 0, (size_t)tot * 16);
+      if (e == cudaSuccess)
+        e = cudaMemcpy(g->d_rec_off, off.data(), sizeof(uint32_t) * (naw + 1),
+                       cudaMemcpyHostToDevice);
+    }
+    if (e == cudaSuccess) {
+      k_sched<true><<<naw, 64>>>(g->d_hdr, g->d_st, nullptr, g->d_rec_off, g->d_rec, g->d_err);
+      e = cudaMemcpy(&herr, g->d_err, sizeof(int), cudaMemcpyDeviceToHost);
+    }
+    if (e == cudaSuccess) e = cudaMemset(g->d_err, 0, sizeof(int));
+    if (e != cudaSuccess) {
+      st = nb_cuda_fail(e, "nb_geom_create walk check and schedules", __FILE__, __LINE__);
+      goto fail;
+    }
+    if (herr) {
+      nb_set_error_msg("nb_geom_create: crossing schedules over capacity (%d)", herr);
       st = NB_ERR_DATA;
       goto fail;
     }
@@ -499,13 +672,6 @@ fail:
   return st;
 }
 
-// Ring of a ring front edge z (cm): ring i starts at (i - 32) * AXR (mmraux.py:365-370)
-static int ring_of(float z) {
-  const double r = (double)z / (double)NB_RING + 0.5 * NB_NRINGS;
-  const long i = lrint(r);
-  return fabs(r - (double)i) < 1e-4 ? (int)i : -1;
-}
-
 // Rays of the ring range [rs, re) from the range's axial LUTs, as mmraux.axial_lut builds
 // them after mmraux.reduce_rings: li2rng / li2sn1 [nli2r][2], the first re - rs entries
 // the direct planes (prjf.cu:33-95 runs them as fprj_drct), the others the oblique pairs,
@@ -514,7 +680,7 @@ static int ring_of(float z) {
 // range, and the rays must fill the range's (re - rs)^2 sinograms (4084 for all 64 rings)
 // once each; anything else is NB_ERR_ARG (the reference's LUTs of 62- and 63-ring ranges,
 // whose ring differences exceed the maximum of 60 without the full-ring correction, end in
-// zero entries and fail this check).  The rays keep the geometry's warp-friendly order.
+// zero entries and fail this check).
 extern "C" int nb_rings_create(nb_geom *g, int rs, int re, const float *li2rng,
                                const int16_t *li2sn1, int nli2r, nb_rings **out) {
   NB_REQUIRE(out != nullptr, "nb_rings_create: out is NULL");
@@ -539,7 +705,7 @@ extern "C" int nb_rings_create(nb_geom *g, int rs, int re, const float *li2rng,
     memcpy(&b, &R.r1z, 4);
     pos[std::make_tuple((int)R.kind, a, b)] = r;
   }
-  std::vector<std::pair<int, nb_ray>> sel;  // (position in the geometry's order, ray)
+  std::vector<nb_ray> sel;
   sel.reserve(nsino);
   for (int li = 0; li < nli2r; li++) {
     const float z0 = li2rng[2 * li], z1 = li2rng[2 * li + 1];
@@ -564,28 +730,26 @@ extern "C" int nb_rings_create(nb_geom *g, int rs, int re, const float *li2rng,
       nb_ray R = g->h_rays[it->second];
       R.out1 = li2sn1[2 * li + k];
       R.out11 = 0;  // span 11 does not exist for a reduced range
-      sel.emplace_back(it->second, R);
+      sel.push_back(R);
     }
   }
   if ((int)sel.size() != nsino) {
     nb_set_error_msg("nb_rings_create: %zu rays for %d sinograms", sel.size(), nsino);
     return NB_ERR_ARG;
   }
-  std::sort(sel.begin(), sel.end(),
-            [](const std::pair<int, nb_ray> &x, const std::pair<int, nb_ray> &y) {
-              return x.first < y.first;
-            });
-  std::vector<nb_ray> rays(nsino);
-  std::vector<int16_t> bin1(nsino, -1);
-  for (int r = 0; r < nsino; r++) {
-    rays[r] = sel[r].second;
-    const int o = rays[r].out1;
-    if (o < 0 || o >= nsino || bin1[o] != -1) {
+  std::vector<char> used(nsino, 0);
+  for (const nb_ray &R : sel) {
+    if (R.out1 < 0 || R.out1 >= nsino || used[R.out1]) {
       nb_set_error_msg("nb_rings_create: sinogram %d of the range is out of [0, %d) or mapped "
-                       "twice", o, nsino);
+                       "twice", (int)R.out1, nsino);
       return NB_ERR_ARG;
     }
-    bin1[o] = (int16_t)r;
+    used[R.out1] = 1;
+  }
+  std::vector<nb_slot> slots;
+  if (!make_slots(sel, slots)) {
+    nb_set_error_msg("nb_rings_create: the ring pairs are not distinct pairs of both directions");
+    return NB_ERR_ARG;
   }
   NB_CUDA(cudaSetDevice(g->device));
   nb_rings *rr = (nb_rings *)calloc(1, sizeof(nb_rings));
@@ -596,15 +760,13 @@ extern "C" int nb_rings_create(nb_geom *g, int rs, int re, const float *li2rng,
   rr->nrays = nsino;
   rr->vz0 = 2 * rs;
   rr->nvz = 2 * n - 1;
-  cudaError_t e = cudaMalloc(&rr->d_rays, sizeof(nb_ray) * nsino);
-  if (e == cudaSuccess) e = cudaMalloc(&rr->d_bin1, sizeof(int16_t) * nsino);
+  rr->nslots = (int)slots.size();
+  cudaError_t e = cudaMalloc(&rr->d_slots, sizeof(nb_slot) * slots.size());
   if (e == cudaSuccess)
-    e = cudaMemcpy(rr->d_rays, rays.data(), sizeof(nb_ray) * nsino, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess)
-    e = cudaMemcpy(rr->d_bin1, bin1.data(), sizeof(int16_t) * nsino, cudaMemcpyHostToDevice);
+    e = cudaMemcpy(rr->d_slots, slots.data(), sizeof(nb_slot) * slots.size(),
+                   cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
-    cudaFree(rr->d_rays);
-    cudaFree(rr->d_bin1);
+    cudaFree(rr->d_slots);
     free(rr);
     return nb_cuda_fail(e, "nb_rings_create upload", __FILE__, __LINE__);
   }
@@ -615,8 +777,7 @@ extern "C" int nb_rings_create(nb_geom *g, int rs, int re, const float *li2rng,
 extern "C" int nb_rings_destroy(nb_rings *rr) {
   if (!rr) return NB_OK;
   cudaSetDevice(rr->device);
-  cudaFree(rr->d_rays);
-  cudaFree(rr->d_bin1);
+  cudaFree(rr->d_slots);
   free(rr);
   return NB_OK;
 }

@@ -21,6 +21,35 @@ struct nb_ray {
   int16_t li;
 };
 
+// A ray pair of the projector kernels (one per thread and turn): ring pair (r0, r0 + d) with
+// its upward ray A (r0 -> r1) and downward ray B (r1 -> r0), or for d = 0 two direct planes.
+// Slots are ordered by d, so the lanes of a warp make about equally many plane crossings.
+struct nb_slot {
+  int16_t zA, zB;      // voxel plane of ring r0 (2 r0) and of ring r1 (direct: of each plane)
+  int16_t o11A, o11B;  // span-11 sinogram of each ray, -1: no such ray
+  int16_t o1A, o1B;    // span-1 sinogram (a reduced range's own numbers in nb_rings)
+  uint8_t d, nosA, nosB, pad;
+};
+#define NB_NSLOT 2048  // slot table capacity: 32 for the direct planes, 2010 pairs, padding
+
+// Crossing schedule of a LOR (k_sched, nb_geom.cu), 16-byte aligned:
+//   kend[52][64]  crossings of difference d up to and including the steps of 8-step row r
+//   m[64]         first plane boundary the upward ray crosses, relative to its ring's 2 r0
+//   off[64]       first entry of difference d (uint16)
+//   meta          uint16 count of irregular rays, uint16 "some fraction lies outside [-1, 1]"
+//   irr[96]       {d, r0, 0 up / 1 down, start plane offset}: rays whose start plane rounds
+//                 away from their group's
+//   entries       {int32 step, float32 fraction of the step before the crossing}
+#define NB_REC_KEND 0
+#define NB_REC_M 3328
+#define NB_REC_OFF 3392
+#define NB_REC_META 3520
+#define NB_REC_IRR 3536
+#define NB_REC_MAXIRR 96
+#define NB_REC_ENT 3920
+#define NB_REC_MAXENT 3392
+#define NB_REC_MAX (NB_REC_ENT + 8 * NB_REC_MAXENT)
+
 struct nb_geom {
   int device;
   int nsm;
@@ -31,17 +60,18 @@ struct nb_geom {
   float4 *d_hdr;     // per LOR: (t entry of step 0, atn, t2, nsteps as int bits)
   float *d_tt;       // reference-layout tt [naw][10]
   nb_ray *d_rays;    // [4084]
-  int16_t *d_bin11;  // [837][8] rays summed into each span-11 sinogram (-1 padded)
-  int16_t *d_bin1;   // [4084] ray of each span-1 sinogram
+  unsigned char *d_rec;  // crossing schedules of all LORs
+  uint32_t *d_rec_off;   // [naw + 1] start of a LOR's record, in 16-byte units
+  nb_slot *d_slots;      // [nslots] ray pairs
+  int nslots;
+  int16_t *d_bin11;  // [837][8] rays (2 slot + direction) of each span-11 sinogram (-1 padded)
   float *d_scratch128;   // one col128 image (reference-layout entry points)
-  float maxseg;          // longest walk segment of the geometry (cm)
-  int fxbits;            // fixed-point headroom of the backward accumulators
   int *d_err;            // device error flag
   float *d_one;          // the constant 1.0f (randoms factor of a single-image batch)
   // host copies of the LUTs (for nb_geom_tables) and of the ray table (for nb_rings_create)
   float h_crs[504 * 4];
   int16_t *h_s2c;
-  nb_ray *h_rays;    // [4084], the order of d_rays
+  nb_ray *h_rays;    // [4084], as d_rays
 };
 
 // The rays of a reduced axial ring range [rs, re) (span 1 only): the reference's
@@ -55,8 +85,8 @@ struct nb_rings {
   int rs, re;
   int nrays;         // rays of the range = its span-1 sinograms
   int vz0, nvz;
-  nb_ray *d_rays;    // [nrays], out1 = the range's sinogram of the ray
-  int16_t *d_bin1;   // [nrays] ray of each of the range's sinograms
+  nb_slot *d_slots;  // [nslots] the range's ray pairs, o1A / o1B the range's sinograms
+  int nslots;
 };
 
 // ---- tracing: an NVTX range around a C-ABI call (header-only NVTX3: without a profiler

@@ -1,16 +1,12 @@
 // nb_prj.cu -- projector entry points, layout conversion, OSEM element-wise kernels and
-// the sinogram gap kernels.  The projector kernel itself is in nb_project.cuh.
+// the sinogram gap kernels.  The projector kernel itself is in nb_walk.cuh.
 #include <math.h>
-
-#include <atomic>
 
 #include "nb_axial.cuh"
 #include "nb_internal.cuh"
-#include "nb_project.cuh"
+#include "nb_walk.cuh"
 
 namespace {
-
-using namespace nbk;
 
 // ---------------------------------------------------------------------------------------
 // layout conversion and element-wise kernels
@@ -124,47 +120,6 @@ __global__ void k_count_reads(const float4 *__restrict__ hdr, const float *__res
   atomicAdd(per_lor + lor, tot);
 }
 
-template <int MODE, int CH>
-int launch_project(nb_geom *g, const PrjArgs &a, cudaStream_t stream) {
-  const size_t smem = Smem<MODE, CH>::total;
-  // set once per device and kernel shape; atomics, since host threads may launch at once
-  static std::atomic<bool> attr_set[64];
-  if (!attr_set[g->device & 63].load(std::memory_order_acquire)) {
-    NB_CUDA(cudaFuncSetAttribute(k_project<MODE, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
-    attr_set[g->device & 63].store(true, std::memory_order_release);
-  }
-  if (a.nprj <= 0) return NB_OK;
-  const int grid = a.nprj < g->nsm ? a.nprj : g->nsm;
-  k_project<MODE, CH><<<grid, NT, smem, stream>>>(a);
-  NB_CUDA(cudaGetLastError());
-  return NB_OK;
-}
-
-// columns per shared-memory chunk: the forward kernel double-buffers 2 x 64 KB of
-// columns; the backward/OSEM kernels also hold the int32 accumulators
-constexpr int CH_FWD = 128;
-constexpr int CH_BWD = 64;
-
-PrjArgs base_args(nb_geom *g, const int32_t *subs, int nprj, int span) {
-  PrjArgs a{};
-  a.scol = g->d_scol;
-  a.st = g->d_st;
-  a.hdr = g->d_hdr;
-  a.rays = g->d_rays;
-  a.bin11 = g->d_bin11;
-  a.bin1 = g->d_bin1;
-  a.subs = subs;
-  a.nprj = subs ? nprj : g->naw;
-  a.naw = g->naw;
-  a.nrays = NB_NRAYS;
-  a.nout = span == 11 ? NB_NSN11 : NB_NSN1;
-  a.span = span;
-  a.fxbits = g->fxbits;
-  a.err = g->d_err;
-  return a;
-}
-
 int check_common(nb_geom *g, int nprj, const int32_t *subs, int span) {
   NB_REQUIRE(g != nullptr, "NULL geometry handle");
   NB_REQUIRE(span == 1 || span == 11, "span must be 1 or 11");
@@ -201,11 +156,11 @@ extern "C" int nb_fprj_col128(nb_geom *g, float *sino, const float *im128, const
   if (st) return st;
   NB_REQUIRE(sino && im128, "nb_fprj_col128: NULL sino or image");
   NB_REQUIRE(att == 0 || att == 1, "att must be 0 or 1");
-  PrjArgs a = base_args(g, subs, nprj, span);
+  nbw::WalkArgs a = nb_walk_args(g, subs, nprj, span, 1, 1);
   a.att = att;
   a.img = im128;
   a.sino = sino;
-  return launch_project<MODE_FWD, CH_FWD>(g, a, (cudaStream_t)stream);
+  return nb_walk_launch(g, a, nbw::MODE_FWD, 1, 0, (cudaStream_t)stream);
 }
 
 extern "C" int nb_bprj_col128(nb_geom *g, float *im128, const float *sino, const int32_t *subs,
@@ -214,10 +169,10 @@ extern "C" int nb_bprj_col128(nb_geom *g, float *im128, const float *sino, const
   int st = check_common(g, nprj, subs, span);
   if (st) return st;
   NB_REQUIRE(sino && im128, "nb_bprj_col128: NULL sino or image");
-  PrjArgs a = base_args(g, subs, nprj, span);
+  nbw::WalkArgs a = nb_walk_args(g, subs, nprj, span, 1, 1);
   a.bimg = im128;
   a.sino_in = sino;
-  return launch_project<MODE_BWD, CH_BWD>(g, a, (cudaStream_t)stream);
+  return nb_walk_launch(g, a, nbw::MODE_BWD, 1, 0, (cudaStream_t)stream);
 }
 
 extern "C" int nb_sens_col128(nb_geom *g, float *sens128, const float *an, const int32_t *subs,
@@ -227,11 +182,11 @@ extern "C" int nb_sens_col128(nb_geom *g, float *sens128, const float *an, const
   if (st) return st;
   NB_REQUIRE(sens128 && an, "nb_sens_col128: NULL image or sinogram");
   NB_CUDA(cudaMemsetAsync(sens128, 0, sizeof(float) * NB_IMG_COL128, (cudaStream_t)stream));
-  PrjArgs a = base_args(g, subs, nprj, span);
+  nbw::WalkArgs a = nb_walk_args(g, subs, nprj, span, 1, 1);
   a.bimg = sens128;
   a.sino_in = an;
   a.in_by_lor = 1;
-  return launch_project<MODE_BWD, CH_BWD>(g, a, (cudaStream_t)stream);
+  return nb_walk_launch(g, a, nbw::MODE_BWD, 1, 0, (cudaStream_t)stream);
 }
 
 extern "C" int nb_fprj(nb_geom *g, float *sino, const float *im, const int32_t *subs, int nprj,
@@ -282,15 +237,14 @@ extern "C" int nb_fprj_rings(nb_geom *g, const nb_rings *rr, float *sino, const 
   k_slab_to_col128<<<(NB_NCOL * 32 + 255) / 256, 256, 0, s>>>(g->d_scratch128, im, rr->nvz,
                                                                rr->vz0);
   NB_CUDA(cudaGetLastError());
-  PrjArgs a = base_args(g, subs, nprj, 1);
-  a.rays = rr->d_rays;
-  a.bin1 = rr->d_bin1;
-  a.nrays = rr->nrays;
+  nbw::WalkArgs a = nb_walk_args(g, subs, nprj, 1, 1, 1);
+  a.slots = rr->d_slots;
+  a.nslots = rr->nslots;
   a.nout = rr->nrays;
   a.att = att;
   a.img = g->d_scratch128;
   a.sino = sino;
-  return launch_project<MODE_FWD, CH_FWD>(g, a, s);
+  return nb_walk_launch(g, a, nbw::MODE_FWD, 1, 0, s);
 }
 
 extern "C" int nb_bprj_rings(nb_geom *g, const nb_rings *rr, float *im, const float *sino,
@@ -303,14 +257,13 @@ extern "C" int nb_bprj_rings(nb_geom *g, const nb_rings *rr, float *im, const fl
   NB_REQUIRE(sino && im, "nb_bprj_rings: NULL sino or image");
   cudaStream_t s = (cudaStream_t)stream;
   NB_CUDA(cudaMemsetAsync(g->d_scratch128, 0, sizeof(float) * NB_IMG_COL128, s));
-  PrjArgs a = base_args(g, subs, nprj, 1);
-  a.rays = rr->d_rays;
-  a.bin1 = rr->d_bin1;
-  a.nrays = rr->nrays;
+  nbw::WalkArgs a = nb_walk_args(g, subs, nprj, 1, 1, 1);
+  a.slots = rr->d_slots;
+  a.nslots = rr->nslots;
   a.nout = rr->nrays;
   a.bimg = g->d_scratch128;
   a.sino_in = sino;
-  st = launch_project<MODE_BWD, CH_BWD>(g, a, s);
+  st = nb_walk_launch(g, a, nbw::MODE_BWD, 1, 0, s);
   if (st) return st;
   k_col128_to_slab<<<(NB_NCOL * 32 + 255) / 256, 256, 0, s>>>(im, g->d_scratch128, rr->nvz,
                                                                rr->vz0);
@@ -337,12 +290,12 @@ extern "C" int nb_osem_subset(nb_geom *g, float *img128, float *bimg128, const f
              "nb_osem_subset: NULL argument");
   cudaStream_t s = (cudaStream_t)stream;
   NB_CUDA(cudaMemsetAsync(bimg128, 0, sizeof(float) * NB_IMG_COL128, s));
-  PrjArgs a = base_args(g, subs, nprj, 11);
+  nbw::WalkArgs a = nb_walk_args(g, subs, nprj, 11, 1, 1);
   a.img = img128;
   a.bimg = bimg128;
   a.psng = psng;
   a.rs = rs;
-  st = launch_project<MODE_OSEM, CH_BWD>(g, a, s);
+  st = nb_walk_launch(g, a, nbw::MODE_OSEM, 1, 0, s);
   if (st) return st;
   const size_t n4 = NB_IMG_COL128 / 4;
   k_osem_update<<<g->nsm * 8, 256, 0, s>>>((float4 *)img128, (float4 *)bimg128,
@@ -372,12 +325,12 @@ extern "C" int nb_osem_subset_psf(nb_geom *g, float *img128, float *bimg128,
   st = nb_psf_col128(rm, img128, krnl, tmp, stream);
   if (st) return st;
   NB_CUDA(cudaMemsetAsync(bimg128, 0, sizeof(float) * NB_IMG_COL128, s));
-  PrjArgs a = base_args(g, subs, nprj, 11);
+  nbw::WalkArgs a = nb_walk_args(g, subs, nprj, 11, 1, 1);
   a.img = rm;
   a.bimg = bimg128;
   a.psng = psng;
   a.rs = rs;
-  st = launch_project<MODE_OSEM, CH_BWD>(g, a, s);
+  st = nb_walk_launch(g, a, nbw::MODE_OSEM, 1, 0, s);
   if (st) return st;
   st = nb_psf_col128(rm, bimg128, krnl, tmp, stream);  // rm: the convolved back projection
   if (st) return st;

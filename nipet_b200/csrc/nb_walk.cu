@@ -1,0 +1,71 @@
+// nb_walk.cu -- launches of the projector kernel (nb_walk.cuh).
+#include <atomic>
+
+#include "nb_walk.cuh"
+
+namespace {
+
+template <int BS, int VB, int CH, int NT, int MODE, int MINB>
+int launch(nb_geom *g, const nbw::WalkArgs &a, cudaStream_t s) {
+  constexpr int NSEG = NT * VB / (64 * BS);
+  constexpr size_t smem = nbw::WSmem<BS, CH, NSEG>::total;
+  static_assert(smem * MINB + 1024 * MINB <= 228 * 1024, "too much shared memory per SM");
+  auto *k = nbw::k_walk<BS, VB, CH, NT, MODE, MINB>;
+  // the shared-memory opt-in is set once per device and kernel shape; host threads may
+  // launch concurrently, so the flags are atomics (setting the attribute twice is harmless)
+  static std::atomic<bool> set[64];
+  if (!set[g->device & 63].load(std::memory_order_acquire)) {
+    NB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    set[g->device & 63].store(true, std::memory_order_release);
+  }
+  const long jobs = (long)a.nprj * a.ngroups;
+  const long grid = jobs < (long)g->nsm * MINB ? jobs : (long)g->nsm * MINB;
+  if (grid <= 0) return NB_OK;
+  k<<<(int)grid, NT, smem, s>>>(a);
+  NB_CUDA(cudaGetLastError());
+  return NB_OK;
+}
+
+template <int MODE> int launch_default(nb_geom *g, const nbw::WalkArgs &a, int bs, cudaStream_t s) {
+  if (bs == 4) return launch<4, 2, 32, 1024, MODE, 1>(g, a, s);
+  if (bs == 2) return launch<2, 2, 24, 512, MODE, 2>(g, a, s);
+  return launch<1, 1, 32, 512, MODE, 2>(g, a, s);
+}
+
+}  // namespace
+
+int nb_walk_launch(nb_geom *g, const nbw::WalkArgs &a, int mode, int bs, int tile,
+                   cudaStream_t s) {
+  if (mode == nbw::MODE_FWD) return launch_default<nbw::MODE_FWD>(g, a, bs, s);
+  if (mode == nbw::MODE_BWD) return launch_default<nbw::MODE_BWD>(g, a, bs, s);
+  constexpr int M = nbw::MODE_OSEM;
+  if (tile == 0) return launch_default<M>(g, a, bs, s);
+  if (bs == 4)
+    return tile == 1 ? launch<4, 2, 16, 1024, M, 1>(g, a, s) : launch<4, 4, 32, 512, M, 1>(g, a, s);
+  if (bs == 2)
+    return tile == 1 ? launch<2, 2, 16, 512, M, 2>(g, a, s) : launch<2, 2, 32, 1024, M, 1>(g, a, s);
+  return tile == 1 ? launch<1, 1, 16, 512, M, 2>(g, a, s) : launch<1, 1, 64, 1024, M, 1>(g, a, s);
+}
+
+nbw::WalkArgs nb_walk_args(const nb_geom *g, const int32_t *subs, int nprj, int span, int nrep,
+                           int bs) {
+  nbw::WalkArgs a{};
+  a.scol = g->d_scol;
+  a.st = g->d_st;
+  a.hdr = g->d_hdr;
+  a.rec = g->d_rec;
+  a.rec_off = g->d_rec_off;
+  a.slots = g->d_slots;
+  a.nslots = g->nslots;
+  a.bin11 = g->d_bin11;
+  a.subs = subs;
+  a.nprj = subs ? nprj : g->naw;
+  a.naw = g->naw;
+  a.ngroups = (nrep + bs - 1) / bs;
+  a.nrep = nrep;
+  a.nout = span == 11 ? NB_NSN11 : NB_NSN1;
+  a.span = span;
+  a.rscale = g->d_one;
+  a.err = g->d_err;
+  return a;
+}

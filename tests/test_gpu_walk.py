@@ -1,0 +1,115 @@
+"""The projector kernel at the sizes where its chunks, schedules and fixed-point scales can go
+wrong, against the FP64 oracle.
+
+Bars: forward, a ray's fraction terms are float32 (relative 2^-24 each, up to ~35 of them and
+one conversion per chunk) and its integer part is good to 2^-29 of its chunk's integral, so
+1e-6 relative L2 per projection, 1e-5 per bin above 1e-3 of the maximum, and exact zeros where
+the oracle has zeros; backward, values are rounded to 2^-23 of the LOR's largest: 1e-6."""
+import numpy as np
+import pytest
+import torch
+
+from nipet_b200 import diffprj, geometry, petprj
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope='module')
+def env():
+    p = geometry.get_mmrparams()
+    tt, _ = O.siddon_tables(p['txLUT'])
+    n = tt.reshape(-1, 10)[:, 9].astype(int) - 3       # steps of each LOR
+    order = np.argsort(n, kind='stable')
+    pick = [order[0], order[-1],                       # shortest and longest walk
+            24839,                                     # a ray reaches the plane above the image
+            254, 48, 47,                               # second crossings taken a step late
+            42285]                                     # a walk starting on a plane boundary
+    for ch in (16, 24, 32, 64, 128):                   # chunk edges: 1, ch - 1 or 0 steps left
+        for rest in (0, 1, ch - 1):
+            m = np.flatnonzero((n % ch == rest) & (n > ch))
+            pick += [m[m.size // 3], m[m.size // 2]]
+    subs = np.unique(np.asarray(pick)).astype(np.int32)
+    return {'p': p, 'orc': O.Oracle(p), 'subs': subs}
+
+
+def _cnt(env, span):
+    return dict(env['p']['Cnt'], SPN=span)
+
+
+def _image(seed):
+    """Positive with empty planes and columns, values over four decades."""
+    r = np.random.default_rng(seed)
+    im = r.uniform(0.0, 1.0, (320, 320, 127)).astype(np.float32) ** 8
+    im[:, :, 40:47] = 0
+    im[100:130, 90:200] = 0
+    return im
+
+
+def _check_fwd(got, want):
+    assert np.linalg.norm(got - want) <= 1e-6 * np.linalg.norm(want)
+    big = want >= 1e-3 * want.max()
+    assert (np.abs(got - want)[big] / want[big]).max() <= 1e-5
+    assert not got[want == 0].any()
+
+
+@pytest.mark.parametrize('span', [11, 1])
+@pytest.mark.parametrize('nimg', [1, 2, 3, 4])
+def test_walk_edges(env, span, nimg):
+    p, orc, subs = env['p'], env['orc'], env['subs']
+    prj = diffprj.MMRProjector(p, span=span, subs=subs)
+    ims = np.stack([_image(7 * nimg + i) * 10.0 ** (-2 * i) for i in range(nimg)])
+    got = prj.project(torch.from_numpy(ims).cuda()).cpu().numpy().astype(np.float64)
+    r = np.random.default_rng(nimg)
+    si = r.exponential(1.0, got.shape).astype(np.float32) * 10.0 ** (2 * np.arange(nimg))[:, None, None]
+    si = si.astype(np.float32)
+    si[:, 3] = 0
+    back = prj.backproject(torch.from_numpy(si).cuda()).cpu().numpy().astype(np.float64)
+    prj.check()
+    for i in range(nimg):
+        _check_fwd(got[i], orc.fprj(ims[i], subs, span=span))
+        want = orc.bprj(si[i], subs, span=span)
+        assert np.linalg.norm(back[i] - want) <= 1e-6 * np.linalg.norm(want)
+        assert not back[i][want == 0].any()
+
+
+@pytest.mark.parametrize('value', [np.inf, -np.inf, np.nan, 1e35])
+def test_walk_non_finite_voxel(env, value):
+    """A voxel without a fixed-point scale reaches the rays that meet it and no others."""
+    p, subs, Cnt = env['p'], env['subs'], _cnt(env, 1)
+    im = _image(1)
+    vox = (160, 150, 63)
+    im[vox] = 0
+    one = np.zeros_like(im)
+    one[vox] = 1
+    run = lambda x: _project(p, Cnt, x, subs)  # noqa: E731
+    ref, hit = run(im), run(one) != 0
+    im[vox] = value
+    got = run(im)
+    assert hit.any() and np.allclose(got[~hit], ref[~hit], rtol=1e-5, atol=1e-6 * ref.max())
+    if np.isfinite(value):
+        assert (got[hit] > 1e28).all()
+    else:
+        assert not np.isfinite(got[hit]).any()
+
+
+def _project(p, Cnt, im, subs):
+    out = torch.zeros((subs.size, 4084 if Cnt['SPN'] == 1 else 837), device='cuda')
+    petprj.fprj(out, torch.from_numpy(im).cuda(), p['txLUT'], p['axLUT'], subs, Cnt, 0)
+    return out.cpu().numpy().astype(np.float64)
+
+
+@pytest.mark.parametrize('scale', [1e-30, 1e-15, 1e20])
+def test_walk_scales(env, scale):
+    """Results scale with their inputs, also where values are near the ends of float32."""
+    p, orc, subs, Cnt = env['p'], env['orc'], env['subs'], _cnt(env, 11)
+    im = _image(2)
+    want = orc.fprj(im, subs)
+    got = _project(p, Cnt, im * np.float32(scale), subs) / scale
+    assert np.linalg.norm(got - want) <= 2e-6 * np.linalg.norm(want)
+    si = np.random.default_rng(3).exponential(1.0, (subs.size, 837)).astype(np.float32)
+    b = torch.zeros((320, 320, 127), device='cuda')
+    petprj.bprj(b, torch.from_numpy(si * np.float32(scale)).cuda(), p['txLUT'], p['axLUT'], subs, Cnt)
+    want = orc.bprj(si, subs)
+    got = b.cpu().numpy().astype(np.float64) / scale
+    assert np.linalg.norm(got - want) <= 2e-6 * np.linalg.norm(want)
