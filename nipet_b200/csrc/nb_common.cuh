@@ -139,6 +139,33 @@ static __device__ __forceinline__ void nb_fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// Cluster launch control (sm_100): a running block takes over the work of a block of its own
+// grid that has not started yet.  The request completes on `bar` (16 bytes) and leaves its
+// answer in `resp` (16-byte aligned shared memory).
+static __device__ __forceinline__ void nb_clc_request(void *resp, uint64_t *bar) {
+  nb_mbar_arrive_expect_tx(bar, 16);
+  asm volatile(
+      "clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 "
+      "[%0], [%1];" ::"r"(nb_smem_u32(resp)),
+      "r"(nb_smem_u32(bar))
+      : "memory");
+}
+// blockIdx.x of the block taken over, or -1: none was left (no further request may follow)
+static __device__ __forceinline__ int nb_clc_answer(const void *resp) {
+  uint32_t got, x;
+  asm volatile(
+      "{\n\t.reg .b128 r;\n\t.reg .pred p;\n\t.reg .b32 y, z, w;\n\t"
+      "ld.shared.b128 r, [%2];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "mov.u32 %1, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, y, z, w}, r;\n\t}"
+      : "=r"(got), "=r"(x)
+      : "r"(nb_smem_u32(resp))
+      : "memory");
+  return got ? (int)x : -1;
+}
+
 // device-side error reporting: the first error code wins
 static __device__ __forceinline__ void nb_set_error(int *flag, int code) {
   if (flag) atomicCAS(flag, 0, code);

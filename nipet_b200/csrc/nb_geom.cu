@@ -248,12 +248,12 @@ __global__ void k_sched(const float4 *__restrict__ hdr, const float *__restrict_
                         uint32_t *__restrict__ sizes, const uint32_t *__restrict__ rec_off,
                         unsigned char *__restrict__ rec, int *err) {
   const int lor = blockIdx.x, d = threadIdx.x;
-  __shared__ int scnt[64], soff[64], nirr, big;
+  __shared__ int scnt[64], soff[64], nirr;
   const float4 h = hdr[lor];
   const int n = __float_as_int(h.w);
   const float *t = st + (size_t)lor * NB_STEP_STRIDE;
   unsigned char *out = FILL ? rec + (size_t)rec_off[lor] * 16 : nullptr;
-  if (d == 0) nirr = big = 0;
+  if (d == 0) nirr = 0;
   int m = 1, rc = 0;
   const bool live = d >= 1 && d <= NB_MAXRD && n > 0;
   if (live) {
@@ -287,9 +287,9 @@ __global__ void k_sched(const float4 *__restrict__ hdr, const float *__restrict_
         if (fill) {
           const float lt = __fsub_rn(tn, tp);
           const float f = lt > 0.f ? __fdiv_rn(__fsub_rn(tzc, tp), lt) : 0.f;
-          if (fabsf(f) > 1.f) big = 1;
-          *reinterpret_cast<uint2 *>(out + NB_REC_ENT + 8 * (size_t)(base + k)) =
-              make_uint2((uint32_t)s, __float_as_uint(f));
+          if (!(fabsf(f) < 32.f)) atomicOr(err, 4);  // the fixed-point range
+          *reinterpret_cast<int2 *>(out + NB_REC_ENT + 8 * (size_t)(base + k)) =
+              make_int2(s, __float2int_rn(ldexpf(f, NB_REC_QBITS)));
         }
         k++;
         tzc = __fadd_rn(tzc, A.dtz);
@@ -342,8 +342,7 @@ __global__ void k_sched(const float4 *__restrict__ hdr, const float *__restrict_
   __syncthreads();
   if (d == 0) {
     if (nirr > NB_REC_MAXIRR) atomicOr(err, 2);
-    reinterpret_cast<uint16_t *>(out + NB_REC_META)[0] = (uint16_t)nirr;
-    reinterpret_cast<uint16_t *>(out + NB_REC_META)[1] = (uint16_t)big;
+    *reinterpret_cast<uint16_t *>(out + NB_REC_META) = (uint16_t)nirr;
   }
 }
 

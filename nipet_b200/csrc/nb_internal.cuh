@@ -36,10 +36,10 @@ struct nb_slot {
 //   kend[52][64]  crossings of difference d up to and including the steps of 8-step row r
 //   m[64]         first plane boundary the upward ray crosses, relative to its ring's 2 r0
 //   off[64]       first entry of difference d (uint16)
-//   meta          uint16 count of irregular rays, uint16 "some fraction lies outside [-1, 1]"
+//   meta          uint16 count of irregular rays
 //   irr[96]       {d, r0, 0 up / 1 down, start plane offset}: rays whose start plane rounds
 //                 away from their group's
-//   entries       {int32 step, float32 fraction of the step before the crossing}
+//   entries       {int32 step, int32 fraction of the step before the crossing (2^26 = 1)}
 #define NB_REC_KEND 0
 #define NB_REC_M 3328
 #define NB_REC_OFF 3392
@@ -48,6 +48,7 @@ struct nb_slot {
 #define NB_REC_MAXIRR 96
 #define NB_REC_ENT 3920
 #define NB_REC_MAXENT 3392
+#define NB_REC_QBITS 26
 #define NB_REC_MAX (NB_REC_ENT + 8 * NB_REC_MAXENT)
 
 struct nb_geom {

@@ -19,9 +19,9 @@ int launch(nb_geom *g, const nbw::WalkArgs &a, cudaStream_t s) {
     set[g->device & 63].store(true, std::memory_order_release);
   }
   const long jobs = (long)a.nprj * a.ngroups;
-  const long grid = jobs < (long)g->nsm * MINB ? jobs : (long)g->nsm * MINB;
-  if (grid <= 0) return NB_OK;
-  k<<<(int)grid, NT, smem, s>>>(a);
+  if (jobs <= 0) return NB_OK;
+  NB_REQUIRE(jobs <= 0x7fffffff, "too many LORs times images for one launch");
+  k<<<(int)jobs, NT, smem, s>>>(a);
   NB_CUDA(cudaGetLastError());
   return NB_OK;
 }
@@ -29,7 +29,7 @@ int launch(nb_geom *g, const nbw::WalkArgs &a, cudaStream_t s) {
 template <int MODE> int launch_default(nb_geom *g, const nbw::WalkArgs &a, int bs, cudaStream_t s) {
   if (bs == 4) return launch<4, 2, 32, 1024, MODE, 1>(g, a, s);
   if (bs == 2) return launch<2, 2, 24, 512, MODE, 2>(g, a, s);
-  return launch<1, 1, 32, 512, MODE, 2>(g, a, s);
+  return launch<1, 1, 64, 512, MODE, 2>(g, a, s);
 }
 
 }  // namespace
@@ -44,7 +44,7 @@ int nb_walk_launch(nb_geom *g, const nbw::WalkArgs &a, int mode, int bs, int til
     return tile == 1 ? launch<4, 2, 16, 1024, M, 1>(g, a, s) : launch<4, 4, 32, 512, M, 1>(g, a, s);
   if (bs == 2)
     return tile == 1 ? launch<2, 2, 16, 512, M, 2>(g, a, s) : launch<2, 2, 32, 1024, M, 1>(g, a, s);
-  return tile == 1 ? launch<1, 1, 16, 512, M, 2>(g, a, s) : launch<1, 1, 64, 1024, M, 1>(g, a, s);
+  return tile == 1 ? launch<1, 1, 32, 512, M, 2>(g, a, s) : launch<1, 1, 64, 1024, M, 1>(g, a, s);
 }
 
 nbw::WalkArgs nb_walk_args(const nb_geom *g, const int32_t *subs, int nprj, int span, int nrep,

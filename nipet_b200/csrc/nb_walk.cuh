@@ -31,14 +31,22 @@
 // denormal-small) value is walked step by step in float32 instead, which keeps the value in
 // the rays that meet it.
 //
+// Jobs.  One block per (LOR, image group); a finished block takes over a block that has not
+// started (cluster launch control), so LORs of 10 to 404 steps even out over the SMs and the
+// next LOR's copies are in flight while one ends (a fixed stride over the LORs left the last
+// wave 9% of the SMs' time idle at 4894 LORs).
+//
 // Measured (B200, 1965 MHz; per call, against the step-by-step walk it replaces): attenuation
 // factors of all LORs at span 11 28.0 -> 4.0 ms (chunks without any value are skipped), a
-// 4894-LOR emission projection 2.16 -> 0.38 ms, a 5003-LOR span-1 back projection 2.60 ->
-// 1.08 ms, a drop-in OSEM iteration 64.5 -> 29.4 ms, 9 images batched 341 -> 250 ms.  Against
-// the FP64 oracle the error halves (forward 1.2e-7 -> 5e-8, back 1.5e-7 -> 7e-8 relative L2).
-// What bounds it: instruction issue (65% active) and the shared-memory pipe (54 .. 60%); per
-// LOR and image ~150k warp instructions, of which the crossings are 40%, the rest the running
-// sums and each chunk's set-up of the 2042 ray pairs.
+// 4894-LOR emission projection 2.16 -> 0.36 ms, a 5003-LOR span-1 back projection 2.58 ->
+// 0.84 ms, a drop-in OSEM iteration 64.5 -> 23.2 ms, 9 images batched 341 -> 215 ms.  Against
+// the FP64 oracle the error halves (forward 1.2e-7 -> 5e-8, back 1.5e-7 -> 6e-8 relative L2).
+// What bounds it: the shared-memory (LSU) pipe at 79 .. 81% of its wavefronts, half of them the
+// crossings' (a warp of 32 pairs spans up to 8 ring differences, whose lanes share banks: 3.1
+// wavefronts per 8-byte read where 2 would do); per LOR and image ~100k warp instructions, the
+// crossings 30%, running sums 21%, each chunk's set-up of the pairs 21% (64-step chunks in
+// place of 32 took 30% off).  Aligning differences to half-warps saved 20% of the crossings'
+// wavefronts and lost more to 20% more sets (0.77 -> 0.85 ms).
 #pragma once
 #include "nb_axial.cuh"
 #include "nb_internal.cuh"
@@ -47,7 +55,8 @@ namespace nbw {
 
 constexpr uint32_t WAIT_POLLS = 1u << 20;
 enum { MODE_FWD = 0, MODE_BWD = 1, MODE_OSEM = 2 };
-constexpr int FXBITS = 22;    // back projection: |V| <= 2^22 (see the file comment)
+constexpr int FXBITS = 23;    // back projection: |V| <= 2^23 (see the file comment)
+constexpr int QBITS = NB_REC_QBITS;  // crossing fractions are int32 with this many fraction bits
 
 struct WalkArgs {
   const int32_t *scol;
@@ -87,8 +96,8 @@ template <int BS, int CH, int NSEG> struct WSmem {
   static constexpr size_t region = cmax(cmax(tab, 4096ull * 4 * BS), align128(gacc) + stage);
   static constexpr size_t stg_off = align128(gacc);
   static constexpr size_t seg_off = align128(region);                       // [NSEG][128][BS]
-  static constexpr size_t oc_off = align128(seg_off + 512ull * NSEG * BS);  // [CH][BS] x 2
-  static constexpr size_t run_off = align128(oc_off + 8ull * CH * BS);      // [2][128][BS]
+  static constexpr size_t oc_off = align128(seg_off + 512ull * NSEG * BS);  // [NSEG][steps + 1][BS]
+  static constexpr size_t run_off = align128(oc_off + 4ull * (CH + NSEG) * BS);      // [2][128][BS]
   static constexpr size_t rec_off = align128(run_off + 1024ull * BS);
   static constexpr size_t cs_off = align128(rec_off + NB_REC_MAX);          // [2][2][stride]
   static constexpr size_t rat_off = align128(cs_off + 16ull * NB_STEP_STRIDE);
@@ -134,35 +143,30 @@ template <int N> __device__ __forceinline__ void sti(int *p, const int *v) {
 }
 
 // shared-memory accessors on 32-bit shared-window addresses
-static __device__ __forceinline__ void lds_ent(uint32_t addr, uint32_t &i, float &f) {
-  asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(i), "=f"(f) : "r"(addr));
+static __device__ __forceinline__ void lds_ent(uint32_t addr, int &i, int &f) {
+  asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(i), "=r"(f) : "r"(addr));
 }
 static __device__ __forceinline__ void reds_add_s32(uint32_t addr, int v) {
   asm volatile("red.shared.add.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
-// {D, dX} of BS images at a table address: 8 bytes (BS 1), 16 (BS 2: D0 D1 dX0 dX1), or two
+// {D, dD} of BS images at a table address: 8 bytes (BS 1), 16 (BS 2: D0 D1 dD0 dD1), or two
 // 16-byte rows 2 KB apart (BS 4), so that the lanes of a warp read consecutive banks
 template <int BS>
-static __device__ __forceinline__ void lds_tab(uint32_t addr, int *D, float *X) {
+static __device__ __forceinline__ void lds_tab(uint32_t addr, int *D, int *X) {
   if (BS == 1) {
-    asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(D[0]), "=f"(X[0]) : "r"(addr));
+    asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(D[0]), "=r"(X[0]) : "r"(addr));
   } else if (BS == 2) {
     asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(D[0]), "=r"(D[1]), "=f"(X[0]), "=f"(X[1])
+                 : "=r"(D[0]), "=r"(D[1]), "=r"(X[0]), "=r"(X[1])
                  : "r"(addr));
   } else {
     asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(D[0]), "=r"(D[1]), "=r"(D[2]), "=r"(D[3])
                  : "r"(addr));
     asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];"
-                 : "=f"(X[0]), "=f"(X[1]), "=f"(X[2]), "=f"(X[3])
+                 : "=r"(X[0]), "=r"(X[1]), "=r"(X[2]), "=r"(X[3])
                  : "r"(addr + 2048u));
   }
-}
-// round(x * y) to the nearest integer (ties to even) for |x * y| < 2^22 on the FMA pipe:
-// adding 1.5 * 2^23 inside the fused multiply-add leaves the integer in the low mantissa bits
-static __device__ __forceinline__ int fx_round(float x, float y) {
-  return __float_as_int(__fmaf_rn(x, y, 12582912.0f)) - 0x4B400000;
 }
 
 // byte offset of a plane in a row whose planes are `unit` bytes wide (even planes first)
@@ -173,9 +177,6 @@ static __device__ __forceinline__ float oblique_s(int d, float atn) {
   if (d == 0) return 1.f;
   const float az_atn = __fdiv_rn((float)d * NB_RING, atn);
   return __fsqrt_rn(__fmaf_rn(az_atn, az_atn, 1.0f));
-}
-static __device__ __forceinline__ int bias_of(uint32_t bias, int k) {
-  return (int)(bias << (28 - 4 * k)) >> 28;
 }
 
 // One ray over steps [s0, s1) of a chunk, step by step in float32 (chunks whose values have
@@ -190,7 +191,7 @@ static __device__ __noinline__ void slow_ray(const float *gimg, const int32_t *c
     tp = tn;
     const float *p0 = c + nb_zi(z) * BS;
     if (cnt > 0 && (int)ent->x == s) {
-      const float f = __uint_as_float(ent->y);
+      const float f = (float)(int)ent->y * (1.f / (1 << QBITS));
       z += dir;
       const float *p1 = c + nb_zi(z) * BS;
       for (int k = 0; k < BS; k++)
@@ -213,7 +214,6 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
   constexpr int LOGR = BS == 1 ? 10 : (BS == 2 ? 11 : 12);   // table row bytes
   constexpr int LOGG = LOGR - 1;                             // accumulator row bytes
   static_assert(CH % 8 == 0 && CH % NSEG == 0 && SEGL >= 1, "chunk shape");
-  static_assert(SPT * 8 <= 32, "bias bits");
   using L = WSmem<BS, CH, NSEG>;
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char *tab = smem;
@@ -222,13 +222,15 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
   float *vals = reinterpret_cast<float *>(smem);                     // [4096][BS]
   int *sseg = reinterpret_cast<int *>(smem + L::seg_off);
   int *soc = reinterpret_cast<int *>(smem + L::oc_off);              // prefixes of voxel 63
-  float *sxo = reinterpret_cast<float *>(smem + L::oc_off) + CH * BS;  // its values
   int *srun = reinterpret_cast<int *>(smem + L::run_off);
   unsigned char *rec = smem + L::rec_off;
   float *rat = reinterpret_cast<float *>(smem + L::rat_off);
   unsigned char *misc = smem + L::misc_off;
   uint64_t *bar = reinterpret_cast<uint64_t *>(misc);
-  int *sflag = reinterpret_cast<int *>(misc + 8);
+  uint64_t *bar2 = reinterpret_cast<uint64_t *>(misc + 8);
+  void *clc = misc + 16;                                             // launch control's answer
+  int *sflag = reinterpret_cast<int *>(misc + 32);
+  int *snext = reinterpret_cast<int *>(misc + 36);
   unsigned *smax = reinterpret_cast<unsigned *>(smem + L::max_off);  // forward bounds
   unsigned *smaxb = reinterpret_cast<unsigned *>(misc + 64);         // [2][BS] backward
 
@@ -236,11 +238,11 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
   const int s = tid & 63;                     // scan: this thread's planes 2 s and 2 s + 1
   const int seg = (tid >> 6) % NSEG, iv = ((tid >> 6) / NSEG) * VB;
   const uint32_t tab_u = nb_smem_u32(tab), rec_u = nb_smem_u32(rec);
-  const long jobs = (long)a.nprj * a.ngroups;
   const bool span11 = a.span == 11;
 
   if (tid == 0) {
     nb_mbar_init(bar, 1);
+    nb_mbar_init(bar2, 1);
     *sflag = 0;
     for (int k = 0; k < 3 * NSEG * BS; k++) smax[k] = 0u;
     for (int k = 0; k < 2 * BS; k++) smaxb[k] = 0u;
@@ -251,8 +253,8 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
   __syncthreads();
 
   // one thread: the record, columns and exit parameters of job q into shared memory
-  auto issue = [&](long q, int buf) {
-    const int p = (int)(q / a.ngroups);
+  auto issue = [&](int q, int buf) {
+    const int p = q / a.ngroups;
     int lor = a.subs ? a.subs[p] : p;
     if (lor < 0 || lor >= a.naw) {
       nb_set_error(a.err, NB_DEVERR_BAD_LOR);
@@ -267,11 +269,25 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
     nb_bulk_g2s(cs, a.scol + (size_t)lor * NB_STEP_STRIDE, cb, bar);
     nb_bulk_g2s(cs + 4 * NB_STEP_STRIDE, a.st + (size_t)lor * NB_STEP_STRIDE, cb, bar);
   };
-  if (tid == 0 && blockIdx.x < jobs) issue(blockIdx.x, 0);
+  // The grid has one block per job (LOR, image group); a block that has finished takes over
+  // a job whose block has not started, so that long and short LORs even out over the SMs and
+  // the next LOR's copies are in flight while this one ends.
+  auto next_job = [&](int job) {
+    int q = -1;
+    if (nb_mbar_wait(bar2, (uint32_t)(job & 1), WAIT_POLLS)) {
+      q = nb_clc_answer(clc);
+      nb_fence_proxy_async_smem();   // the answer is read before the next request rewrites it
+    } else {
+      nb_set_error(a.err, NB_DEVERR_MBAR_TIMEOUT);
+    }
+    *snext = q;
+    if (q >= 0) issue(q, (job + 1) & 1);
+  };
+  if (tid == 0) issue(blockIdx.x, 0);
 
-  int job = 0, mrot = 0;
-  for (long q = blockIdx.x; q < jobs; q += gridDim.x, job++) {
-    const int p = (int)(q / a.ngroups), g = (int)(q - (long)p * a.ngroups);
+  int mrot = 0, q = blockIdx.x;
+  for (int job = 0; q >= 0; job++) {
+    const int p = q / a.ngroups, g = q - p * a.ngroups;
     const int lor0 = a.subs ? a.subs[p] : p;
     const bool badlor = lor0 < 0 || lor0 >= a.naw;
     const int lor = badlor ? 0 : lor0;
@@ -287,24 +303,29 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
     if (MODE != MODE_FWD && warp == 0) nb_bulk_wait_read<0>();   // staging region reusable
     __syncthreads();
     if (*sflag) break;
+    if (tid == 0) nb_clc_request(clc, bar2);
 
     auto slot_of = [&](int j) { return ((j & 1) ? (j + 1) * W - 1 - warp : j * W + warp) * 32 + lane; };
-    // the few rays whose start plane rounds away from their group's
-    uint32_t bias = 0;
+    // this thread's slots: start planes of the two rays (8 bits each) and ring difference;
+    // the few rays whose start plane rounds away from their group's are listed in the record
+    uint32_t zzd[SPT];
     const int nirr = *reinterpret_cast<const uint16_t *>(rec + NB_REC_META);
-    const bool bigf = *reinterpret_cast<const uint16_t *>(rec + NB_REC_META + 2) != 0;
-    if (nirr) {
 #pragma unroll
-      for (int j = 0; j < SPT; j++) {
-        const int sl = slot_of(j);
-        if (sl >= a.nslots) continue;
-        const nb_slot S = a.slots[sl];
-        for (int x = 0; x < nirr; x++) {
-          const uchar4 e = reinterpret_cast<const uchar4 *>(rec + NB_REC_IRR)[x];
-          if (e.x == S.d && 2 * (int)e.y == S.zA)
-            bias |= ((uint32_t)e.w & 15u) << (4 * (2 * j + e.z));
+    for (int j = 0; j < SPT; j++) {
+      const int sl = slot_of(j);
+      zzd[j] = 0u;
+      if (sl >= a.nslots) continue;
+      const nb_slot S = a.slots[sl];
+      const int m = rec[NB_REC_M + S.d];
+      int zA = S.zA + m - 1, zB = S.zB - m + 1;
+      for (int x = 0; x < nirr; x++) {
+        const char4 e = reinterpret_cast<const char4 *>(rec + NB_REC_IRR)[x];
+        if (e.x == S.d && 2 * (int)e.y == S.zA) {
+          zA += e.z ? 0 : e.w;
+          zB += e.z ? e.w : 0;
         }
       }
+      zzd[j] = (uint32_t)zA | (uint32_t)zB << 8 | (uint32_t)S.d << 16;
     }
 
     float FA[SPT][BS], FB[SPT][BS];           // forward: line integrals
@@ -400,12 +421,9 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
               tE[v] += __float2int_rn(E[j][v] * w);
               tO[v] += __float2int_rn(O[j][v] * w);
             }
-            if (s == 31) {
-              sti<VB>(soc + (seg * SEGL + j) * BS + iv, cO[j]);
-#pragma unroll
-              for (int v = 0; v < VB; v++) sxo[(seg * SEGL + j) * BS + iv + v] = O[j][v];
-            }
+            if (s == 31) sti<VB>(soc + (seg * (SEGL + 1) + j) * BS + iv, cO[j]);
           }
+          if (s == 31) sti<VB>(soc + (seg * (SEGL + 1) + SEGL) * BS + iv, tO);
           sti<VB>(sseg + (seg * 128 + s) * BS + iv, tE);
           sti<VB>(sseg + (seg * 128 + 64 + s) * BS + iv, tO);
           __syncthreads();
@@ -425,49 +443,46 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
             }
           }
           if (seg == NSEG - 1) {              // the chunk's whole integral per plane
+            int u[VB], w[VB];
 #pragma unroll
-            for (int v = 0; v < VB; v++) tE[v] += bE[v], tO[v] += bO[v];
-            sti<VB>(srun + s * BS + iv, tE);
-            sti<VB>(srun + (64 + s) * BS + iv, tO);
+            for (int v = 0; v < VB; v++) u[v] = tE[v] + bE[v], w[v] = tO[v] + bO[v];
+            sti<VB>(srun + s * BS + iv, u);
+            sti<VB>(srun + (64 + s) * BS + iv, w);
           }
+          // D at the start of each step and its change over the step
+          int De[VB], Do[VB];
 #pragma unroll
-          for (int j = 0; j < SEGL; j++) {
-            int De[VB], Do[VB];
-            float Xe[VB], Xo[VB];
-            const int row = seg * SEGL + j;
+          for (int j = SEGL; j >= 0; j--) {
+            int ne[VB], no[VB];               // D at the end of step j
 #pragma unroll
             for (int v = 0; v < VB; v++) {
-              const int ce = cE[j][v] + bE[v], co = cO[j][v] + bO[v];
+              ne[v] = De[v];
+              no[v] = Do[v];
+              const int ce = (j < SEGL ? cE[j < SEGL ? j : 0][v] : tE[v]) + bE[v];
+              const int co = (j < SEGL ? cO[j < SEGL ? j : 0][v] : tO[v]) + bO[v];
               int cp = __shfl_up_sync(0xffffffffu, co, 1);      // plane 2 s - 1
-              float xp = __shfl_up_sync(0xffffffffu, O[j][v], 1);
               if (lane == 0) {
-                cp = s ? bP[v] + soc[row * BS + iv + v] : ce;
-                xp = s ? sxo[row * BS + iv + v] : E[j][v];
+                const int o = (seg * (SEGL + 1) + j) * BS + iv + v;
+                cp = s ? bP[v] + soc[o] : ce;
               }
               De[v] = cp - ce;
               Do[v] = ce - co;
-              Xe[v] = lt[j] * (xp - E[j][v]);
-              Xo[v] = lt[j] * (E[j][v] - O[j][v]);
+              ne[v] -= De[v];
+              no[v] -= Do[v];
             }
-            unsigned char *r = tab + ((size_t)row << LOGR) + s * UNIT;
+            if (j == SEGL) continue;
+            unsigned char *r = tab + ((size_t)(seg * SEGL + j) << LOGR) + s * UNIT;
             if (BS == 1) {
-              *reinterpret_cast<float2 *>(r) = make_float2(__int_as_float(De[0]), Xe[0]);
-              *reinterpret_cast<float2 *>(r + 64 * UNIT) = make_float2(__int_as_float(Do[0]), Xo[0]);
+              *reinterpret_cast<int2 *>(r) = make_int2(De[0], ne[0]);
+              *reinterpret_cast<int2 *>(r + 64 * UNIT) = make_int2(Do[0], no[0]);
             } else if (BS == 2 && VB == 2) {
-              *reinterpret_cast<float4 *>(r) =
-                  make_float4(__int_as_float(De[0]), __int_as_float(De[VB - 1]), Xe[0], Xe[VB - 1]);
-              *reinterpret_cast<float4 *>(r + 64 * UNIT) =
-                  make_float4(__int_as_float(Do[0]), __int_as_float(Do[VB - 1]), Xo[0], Xo[VB - 1]);
+              *reinterpret_cast<int4 *>(r) = make_int4(De[0], De[VB - 1], ne[0], ne[VB - 1]);
+              *reinterpret_cast<int4 *>(r + 64 * UNIT) = make_int4(Do[0], Do[VB - 1], no[0], no[VB - 1]);
             } else {
               sti<VB>(reinterpret_cast<int *>(r) + iv, De);
               sti<VB>(reinterpret_cast<int *>(r + 64 * UNIT) + iv, Do);
-#pragma unroll
-              for (int v = 0; v < VB; v++) {
-                De[v] = __float_as_int(Xe[v]);
-                Do[v] = __float_as_int(Xo[v]);
-              }
-              sti<VB>(reinterpret_cast<int *>(r + 2048) + iv, De);
-              sti<VB>(reinterpret_cast<int *>(r + 2048 + 64 * UNIT) + iv, Do);
+              sti<VB>(reinterpret_cast<int *>(r + 2048) + iv, ne);
+              sti<VB>(reinterpret_cast<int *>(r + 2048 + 64 * UNIT) + iv, no);
             }
           }
           __syncthreads();
@@ -478,16 +493,11 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
         const int krow0 = c * (CH / 8) - 1, krow1 = (s1 - 1) >> 3;
 #pragma unroll
         for (int j = 0; j < SPT; j++) {
-          const int sl = slot_of(j);
-          if (sl >= a.nslots) continue;
-          const nb_slot S = a.slots[sl];
-          const int d = S.d;
-          const int ka = c ? kend[krow0 * 64 + d] : 0, kb = kend[krow1 * 64 + d];
-          const int m = rec[NB_REC_M + d];
+          const int zz = (int)zzd[j], d = zz >> 16;
+          const int ka = c ? kend[krow0 * 64 + d] : 0;
+          int cnt = kend[krow1 * 64 + d] - ka;
           const int e0 = reinterpret_cast<const uint16_t *>(rec + NB_REC_OFF)[d] + ka;
-          int cnt = kb - ka;
-          const int zA = S.zA + m - 1 + ka + bias_of(bias, 2 * j);
-          const int zB = S.zB - m + 1 - ka + bias_of(bias, 2 * j + 1);
+          const int zA = (zz & 255) + ka, zB = ((zz >> 8) & 255) - ka;
           if (slow) {
             const uint2 *ent = reinterpret_cast<const uint2 *>(rec + NB_REC_ENT) + e0;
             slow_ray<BS>(gimg, scol, sst, t0, s0, s1, zA, 1, ent, cnt, FA[j]);
@@ -501,67 +511,59 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
           const uint32_t base = tab_u - ((uint32_t)s0 << LOGR);
           uint32_t cA0 = base + plane_off(zA + 1, UNIT), cA1 = base + plane_off(zA + 2, UNIT);
           uint32_t cB0 = base + plane_off(zB, UNIT), cB1 = base + plane_off(zB - 1, UNIT);
+          // sums of D and of dD * fraction (64 bits: 2^30 by 2^31, up to ~100 of them)
           int iA[BS], iB[BS];
+          long long xA[BS], xB[BS];
 #pragma unroll
-          for (int k = 0; k < BS; k++) iA[k] = iB[k] = 0;
+          for (int k = 0; k < BS; k++) {
+            iA[k] = iB[k] = 0;
+            xA[k] = xB[k] = 0;
+          }
+          auto cross = [&](int f, uint32_t rA, uint32_t rB) {
+            int D[BS], X[BS];
+            lds_tab<BS>(rA, D, X);
+#pragma unroll
+            for (int k = 0; k < BS; k++) {
+              iA[k] += D[k];
+              xA[k] += (long long)X[k] * f;
+            }
+            lds_tab<BS>(rB, D, X);
+#pragma unroll
+            for (int k = 0; k < BS; k++) {
+              iB[k] += D[k];
+              xB[k] += (long long)X[k] * f;
+            }
+          };
           for (; cnt >= 2; cnt -= 2) {
-            uint32_t i0, i1;
-            float f0, f1;
-            int D[BS], D2[BS];
-            float X[BS], X2[BS];
+            int i0, i1, f0, f1;
             lds_ent(ep, i0, f0);
             lds_ent(ep + 8, i1, f1);
             ep += 16;
-            lds_tab<BS>(cA0 + (i0 << LOGR), D, X);
-            lds_tab<BS>(cB0 + (i0 << LOGR), D2, X2);
-#pragma unroll
-            for (int k = 0; k < BS; k++) {
-              iA[k] += D[k];
-              FA[j][k] = fmaf(f0, X[k], FA[j][k]);
-              iB[k] -= D2[k];
-              FB[j][k] = fmaf(-f0, X2[k], FB[j][k]);
-            }
-            lds_tab<BS>(cA1 + (i1 << LOGR), D, X);
-            lds_tab<BS>(cB1 + (i1 << LOGR), D2, X2);
-#pragma unroll
-            for (int k = 0; k < BS; k++) {
-              iA[k] += D[k];
-              FA[j][k] = fmaf(f1, X[k], FA[j][k]);
-              iB[k] -= D2[k];
-              FB[j][k] = fmaf(-f1, X2[k], FB[j][k]);
-            }
+            cross(f0, cA0 + (i0 << LOGR), cB0 + (i0 << LOGR));
+            cross(f1, cA1 + (i1 << LOGR), cB1 + (i1 << LOGR));
             cA0 += UNIT;
             cA1 += UNIT;
             cB0 -= UNIT;
             cB1 -= UNIT;
           }
           if (cnt) {
-            uint32_t i0;
-            float f0;
-            int D[BS], D2[BS];
-            float X[BS], X2[BS];
+            int i0, f0;
             lds_ent(ep, i0, f0);
-            lds_tab<BS>(cA0 + (i0 << LOGR), D, X);
-            lds_tab<BS>(cB0 + (i0 << LOGR), D2, X2);
-#pragma unroll
-            for (int k = 0; k < BS; k++) {
-              iA[k] += D[k];
-              FA[j][k] = fmaf(f0, X[k], FA[j][k]);
-              iB[k] -= D2[k];
-              FB[j][k] = fmaf(-f0, X2[k], FB[j][k]);
-            }
+            cross(f0, cA0 + (i0 << LOGR), cB0 + (i0 << LOGR));
           }
-          int u[BS];
+          // the down-going ray leaves C[P] for C[P-1]: its differences count negative
+          int u[BS], w[BS];
           ldi<BS>(srun + nb_zi(endA) * BS, u);
+          ldi<BS>(srun + nb_zi(endB) * BS, w);
 #pragma unroll
-          for (int k = 0; k < BS; k++) FA[j][k] = fmaf((float)(iA[k] + u[k]), inv[k], FA[j][k]);
-          ldi<BS>(srun + nb_zi(endB) * BS, u);
-#pragma unroll
-          for (int k = 0; k < BS; k++) FB[j][k] = fmaf((float)(iB[k] + u[k]), inv[k], FB[j][k]);
+          for (int k = 0; k < BS; k++) {
+            FA[j][k] = fmaf((float)(u[k] + iA[k] + (int)(xA[k] >> QBITS)), inv[k], FA[j][k]);
+            FB[j][k] = fmaf((float)(w[k] - iB[k] - (int)(xB[k] >> QBITS)), inv[k], FB[j][k]);
+          }
         }
       }
       __syncthreads();   // the walk is done: the table region and the record are free
-      if (MODE == MODE_FWD && tid == 0 && q + gridDim.x < jobs) issue(q + gridDim.x, (job + 1) & 1);
+      if (MODE == MODE_FWD && tid == 0) next_job(job);
 
       // ratio of a bin (recon.cu:459-470): y / (Ax + rscale (r+s)/(an)), 0 where |.| < 1e-6
       auto ratio = [&](float v, int o, int k) {
@@ -636,7 +638,11 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
 #pragma unroll
       for (int j = 0; j < SPT; j++) {
         const int sl = slot_of(j);
-        if (sl >= a.nslots) continue;
+        if (sl >= a.nslots) {                 // lanes without a pair have walked plane 0
+#pragma unroll
+          for (int k = 0; k < BS; k++) FA[j][k] = FB[j][k] = 0.f;
+          continue;
+        }
         const nb_slot S = a.slots[sl];
         const float so = oblique_s(S.d, h.y);
         const int oA = span11 ? S.o11A : S.o1A, oB = span11 ? S.o11B : S.o1B;
@@ -668,6 +674,7 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
       for (int i = tid; i < 128 * BS; i += NT) srun[i] = 0;
       __syncthreads();
       float inv[BS];
+      int VA[SPT][BS], VB_[SPT][BS];          // the rays' values, integers
       unsigned any = 0u;
 #pragma unroll
       for (int k = 0; k < BS; k++) {
@@ -682,97 +689,79 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
         }
 #pragma unroll
         for (int j = 0; j < SPT; j++) {
-          // through int: a NaN, or an infinity (scale 0), becomes 0
-          FA[j][k] = (float)__float2int_rn(FA[j][k] * sc);
-          FB[j][k] = (float)__float2int_rn(FB[j][k] * sc);
+          // a NaN, or an infinity (scale 0), becomes 0
+          VA[j][k] = __float2int_rn(FA[j][k] * sc);
+          VB_[j][k] = __float2int_rn(FB[j][k] * sc);
         }
       }
       if (tid < BS) smaxb[(par ^ 1) * BS + tid] = 0u;
-      if (any == 0u || nch == 0) {            // nothing to spread
+      const int nchb = any ? nch : 0;         // 0: nothing to spread
+      if (nchb == 0) {
         __syncthreads();
-        if (tid == 0 && q + gridDim.x < jobs) issue(q + gridDim.x, (job + 1) & 1);
-        continue;
+        if (tid == 0) next_job(job);
       }
       const uint32_t g_u = nb_smem_u32(gacc), run_u = nb_smem_u32(srun);
 #pragma unroll
-      for (int j = 0; j < SPT; j++) {
-        const int sl = slot_of(j);
-        if (sl >= a.nslots) continue;
-        const nb_slot S = a.slots[sl];
-        const int m = rec[NB_REC_M + S.d];
-        const int zA = S.zA + m - 1 + bias_of(bias, 2 * j);
-        const int zB = S.zB - m + 1 + bias_of(bias, 2 * j + 1);
+      for (int j = 0; j < SPT && nchb; j++) {
+        const int zA = zzd[j] & 255, zB = (zzd[j] >> 8) & 255;
 #pragma unroll
         for (int k = 0; k < BS; k++) {
-          const int vA = __float2int_rn(FA[j][k]), vB = __float2int_rn(FB[j][k]);
+          const int vA = VA[j][k], vB = VB_[j][k];
           if (vA) reds_add_s32(run_u + (nb_zi(zA) * BS + k) * 4, vA);
           if (vB) reds_add_s32(run_u + (nb_zi(zB) * BS + k) * 4, vB);
         }
       }
       float *gb = a.bimg + (size_t)g * NB_IMG_COL128 * BS;
-      for (int c = 0; c < nch; c++) {
+      for (int c = 0; c < nchb; c++) {
         const int s0 = c * CH, s1 = min(n, s0 + CH);
         const unsigned char *kend = rec + NB_REC_KEND;
         const int krow0 = c * (CH / 8) - 1, krow1 = (s1 - 1) >> 3;
 #pragma unroll
         for (int j = 0; j < SPT; j++) {
-          const int sl = slot_of(j);
-          if (sl >= a.nslots) continue;
-          const nb_slot S = a.slots[sl];
-          const int d = S.d;
-          const int ka = c ? kend[krow0 * 64 + d] : 0, kb = kend[krow1 * 64 + d];
-          const int m = rec[NB_REC_M + d];
+          const int zz = (int)zzd[j], d = zz >> 16;
+          const int ka = c ? kend[krow0 * 64 + d] : 0;
+          int cnt = kend[krow1 * 64 + d] - ka;
           const int e0 = reinterpret_cast<const uint16_t *>(rec + NB_REC_OFF)[d] + ka;
-          int cnt = kb - ka;
-          const int zA = S.zA + m - 1 + ka + bias_of(bias, 2 * j);
-          const int zB = S.zB - m + 1 - ka + bias_of(bias, 2 * j + 1);
+          const int zA = (zz & 255) + ka, zB = ((zz >> 8) & 255) - ka;
           uint32_t ep = rec_u + NB_REC_ENT + e0 * 8;
           const uint32_t base = g_u - ((uint32_t)s0 << LOGG);
           uint32_t cA0 = base + plane_off(zA + 1, 4), cA1 = base + plane_off(zA + 2, 4);
           uint32_t cB0 = base + plane_off(zB, 4), cB1 = base + plane_off(zB - 1, 4);
-          int vA[BS], vB[BS];
-#pragma unroll
-          for (int k = 0; k < BS; k++) {
-            vA[k] = __float2int_rn(FA[j][k]);
-            vB[k] = __float2int_rn(FB[j][k]);
-          }
-          // upward flow over a plane boundary is positive; image k of a row is k * 512 bytes on
-          auto cross = [&](uint32_t i, float f, uint32_t cA, uint32_t cB) {
-            const uint32_t rA = cA + (i << LOGG), rB = cB + (i << LOGG);
+          // upward flow over a plane boundary is positive; image k of a row is k * 512 bytes on.
+          // q = floor(f V) = high word of f 2^26 by V 2^6
+          auto cross = [&](int f, uint32_t rA, uint32_t rB) {
 #pragma unroll
             for (int k = 0; k < BS; k++) {
-              const int qA = bigf ? __float2int_rn(f * FA[j][k]) : fx_round(f, FA[j][k]);
-              const int qB = bigf ? __float2int_rn(f * FB[j][k]) : fx_round(f, FB[j][k]);
-              reds_add_s32(rA + 512u * k, vA[k] - qA);
+              const int qA = __mulhi(VA[j][k] << (32 - QBITS), f);
+              const int qB = __mulhi(VB_[j][k] << (32 - QBITS), f);
+              reds_add_s32(rA + 512u * k, VA[j][k] - qA);
               reds_add_s32(rA + 512u * k + (1u << LOGG), qA);
-              reds_add_s32(rB + 512u * k, qB - vB[k]);
+              reds_add_s32(rB + 512u * k, qB - VB_[j][k]);
               reds_add_s32(rB + 512u * k + (1u << LOGG), -qB);
             }
           };
           for (; cnt >= 2; cnt -= 2) {
-            uint32_t i0, i1;
-            float f0, f1;
+            int i0, i1, f0, f1;
             lds_ent(ep, i0, f0);
             lds_ent(ep + 8, i1, f1);
             ep += 16;
-            cross(i0, f0, cA0, cB0);
-            cross(i1, f1, cA1, cB1);
+            cross(f0, cA0 + (i0 << LOGG), cB0 + (i0 << LOGG));
+            cross(f1, cA1 + (i1 << LOGG), cB1 + (i1 << LOGG));
             cA0 += 4;
             cA1 += 4;
             cB0 -= 4;
             cB1 -= 4;
           }
           if (cnt) {
-            uint32_t i0;
-            float f0;
+            int i0, f0;
             lds_ent(ep, i0, f0);
-            cross(i0, f0, cA0, cB0);
+            cross(f0, cA0 + (i0 << LOGG), cB0 + (i0 << LOGG));
           }
         }
         if (warp == 0) nb_bulk_wait_read<0>();
         __syncthreads();
         const bool last = c == nch - 1;
-        if (last && tid == 0 && q + gridDim.x < jobs) issue(q + gridDim.x, (job + 1) & 1);
+        if (last && tid == 0) next_job(job);
         // flows -> running sums: this thread's planes z = 2 s and 2 s + 1, SEGL steps
         int rE[SEGL][VB], rO[SEGL][VB], cy[2][VB];
 #pragma unroll
@@ -856,6 +845,8 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
         }
       }
     }
+    __syncthreads();
+    q = *snext;
   }
   if (*sflag && tid == 0) nb_set_error(a.err, NB_DEVERR_MBAR_TIMEOUT);
   if (MODE != MODE_FWD && warp == 0) nb_bulk_wait_all<0>();
