@@ -227,7 +227,8 @@ def autotune(rec: BatchRecon, candidates=None, repeats: int = 2):
     timing `repeats` sub-iterations per candidate after one warm-up.  Returns (bs, tile);
     results are cached in memory and in `~/.cache/nipet_b200/autotune.json`."""
     name = torch.cuda.get_device_name(rec.device)
-    key = f'{name}|span{rec.span}|n{rec.nrep}'
+    # (the kernel's name: choices stored for another kernel say nothing about this one)
+    key = f'{name}|k_walk|span{rec.span}|n{rec.nrep}'
     if key in _TUNE_CACHE:
         return _TUNE_CACHE[key]
     disk = {}
@@ -243,7 +244,8 @@ def autotune(rec: BatchRecon, candidates=None, repeats: int = 2):
     if candidates is None:
         widths = [1, 2, 4]
         widths = [w for w in widths if w <= max(1, rec.nrep) or w == 1]
-        candidates = [(w, t) for w in widths for t in TILES]
+        # one image per walk has one kernel shape
+        candidates = [(w, t) for w in widths for t in (TILES if w > 1 else TILES[:1])]
     best, best_t = candidates[0], float('inf')
     rec.sens128.fill_(1.0)
     for bs, tile in candidates:

@@ -420,13 +420,10 @@ static bool make_slots(const std::vector<nb_ray> &rays, std::vector<nb_slot> &sl
     nb_slot &S = pair[key];
     if (seen[key] & R.kind) return false;
     seen[key] |= R.kind;
-    S.zA = (int16_t)(2 * r0);
-    S.zB = (int16_t)(2 * r1);
-    S.d = (uint8_t)(r1 - r0);
-    S.pad = 0;
+    S.zzd = (uint32_t)(2 * r0) | (uint32_t)(2 * r1) << 8 | (uint32_t)(r1 - r0) << 16;
     (R.kind == 1 ? S.o11A : S.o11B) = R.out11;
     (R.kind == 1 ? S.o1A : S.o1B) = R.out1;
-    (R.kind == 1 ? S.nosA : S.nosB) = (uint8_t)R.nos;
+    (R.kind == 1 ? S.nosA : S.nosB) = R.nos;
   }
   for (const auto &kv : seen)
     if (kv.second != 3) return false;
@@ -437,14 +434,13 @@ static bool make_slots(const std::vector<nb_ray> &rays, std::vector<nb_slot> &sl
   for (size_t i = 0; i < half; i++) {
     nb_slot S{};
     const nb_ray *A = dir[i], *B = half + i < dir.size() ? dir[half + i] : nullptr;
-    S.zA = (int16_t)(2 * ring_of(A->r0z));
+    S.zzd = (uint32_t)(2 * ring_of(A->r0z)) | (uint32_t)(B ? 2 * ring_of(B->r0z) : 0) << 8;
     S.o11A = A->out11;
     S.o1A = A->out1;
-    S.nosA = (uint8_t)A->nos;
-    S.zB = B ? (int16_t)(2 * ring_of(B->r0z)) : 0;
+    S.nosA = A->nos;
     S.o11B = B ? B->out11 : -1;
     S.o1B = B ? B->out1 : -1;
-    S.nosB = B ? (uint8_t)B->nos : 1;
+    S.nosB = B ? B->nos : 1;
     slots.push_back(S);
   }
   for (const auto &kv : pair) slots.push_back(kv.second);

@@ -25,10 +25,11 @@ struct nb_ray {
 // its upward ray A (r0 -> r1) and downward ray B (r1 -> r0), or for d = 0 two direct planes.
 // Slots are ordered by d, so the lanes of a warp make about equally many plane crossings.
 struct nb_slot {
-  int16_t zA, zB;      // voxel plane of ring r0 (2 r0) and of ring r1 (direct: of each plane)
+  uint32_t zzd;        // plane of ring r0 (2 r0) | plane of ring r1 << 8 | d << 16 (direct: the
+                       // two planes)
   int16_t o11A, o11B;  // span-11 sinogram of each ray, -1: no such ray
   int16_t o1A, o1B;    // span-1 sinogram (a reduced range's own numbers in nb_rings)
-  uint8_t d, nosA, nosB, pad;
+  int16_t nosA, nosB;  // span-1 planes in the ray's span-11 sinogram
 };
 #define NB_NSLOT 2048  // slot table capacity: 32 for the direct planes, 2010 pairs, padding
 

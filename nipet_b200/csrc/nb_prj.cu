@@ -191,12 +191,20 @@ extern "C" int nb_sens_col128(nb_geom *g, float *sens128, const float *an, const
 
 extern "C" int nb_fprj(nb_geom *g, float *sino, const float *im, const int32_t *subs, int nprj,
                        int span, int att, void *stream) {
+  NB_RANGE("nb_fprj");
   int st = check_common(g, nprj, subs, span);
   if (st) return st;
   NB_REQUIRE(sino && im, "nb_fprj: NULL sino or image");
-  st = nb_im_to_col128(g->d_scratch128, im, 1, stream);
-  if (st) return st;
-  return nb_fprj_col128(g, sino, g->d_scratch128, subs, nprj, span, att, stream);
+  NB_REQUIRE(att == 0 || att == 1, "att must be 0 or 1");
+  // the kernel reads the reference layout's columns as they are (their planes in pairs, two
+  // wavefronts a read for one): a conversion pass would take 30 us whatever the LORs, against
+  // 1% of the walk of a subset
+  nbw::WalkArgs a = nb_walk_args(g, subs, nprj, span, 1, 1);
+  a.att = att;
+  a.img = im;
+  a.natural = 1;
+  a.sino = sino;
+  return nb_walk_launch(g, a, nbw::MODE_FWD, 1, 0, (cudaStream_t)stream);
 }
 
 extern "C" int nb_bprj(nb_geom *g, float *im, const float *sino, const int32_t *subs, int nprj,

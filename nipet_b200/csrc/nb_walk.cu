@@ -26,9 +26,22 @@ int launch(nb_geom *g, const nbw::WalkArgs &a, cudaStream_t s) {
   return NB_OK;
 }
 
-template <int MODE> int launch_default(nb_geom *g, const nbw::WalkArgs &a, int bs, cudaStream_t s) {
-  if (bs == 4) return launch<4, 2, 32, 1024, MODE, 1>(g, a, s);
-  if (bs == 2) return launch<2, 2, 24, 512, MODE, 2>(g, a, s);
+// Kernel shapes <BS, images per thread of the running sums, steps per chunk, threads, mode,
+// blocks per SM>.  One image: two blocks of 512 threads at 64 registers (256 threads at 128: 4%
+// slower forward, 13% in the fused mode; 32-step chunks 14% and 6%).  Two and four images need
+// the registers: 16 warps of 128 registers an SM beat 32 of 64, which spill (us per image and
+// 4894 LORs, dense image; fused sub-iteration / forward / back):
+//   two images    24 steps, 2 x 512 threads  1593 / 741 / 693
+//                 24 steps, 2 x 256 threads  1383 / 693 / 644
+//                 32 steps, 2 x 256 threads  1471 / 641 / 633
+//                 64 steps, 1 x 512 threads  1361 / 651 / 716
+//   four images   32 steps, 1 x 1024 threads 1727 / 942 / 735
+//                 32 steps, 1 x 512 threads  1346 / 687 / 651
+//                 24 steps, 1 x 384 threads  1475 / 763 / 681
+//                 32 steps, 1 x 256 threads  1469 / 751 / 693
+template <int MODE> int launch_prj(nb_geom *g, const nbw::WalkArgs &a, int bs, cudaStream_t s) {
+  if (bs == 4) return launch<4, 4, 32, 512, MODE, 1>(g, a, s);
+  if (bs == 2) return launch<2, 2, 32, 256, MODE, 2>(g, a, s);
   return launch<1, 1, 64, 512, MODE, 2>(g, a, s);
 }
 
@@ -36,15 +49,19 @@ template <int MODE> int launch_default(nb_geom *g, const nbw::WalkArgs &a, int b
 
 int nb_walk_launch(nb_geom *g, const nbw::WalkArgs &a, int mode, int bs, int tile,
                    cudaStream_t s) {
-  if (mode == nbw::MODE_FWD) return launch_default<nbw::MODE_FWD>(g, a, bs, s);
-  if (mode == nbw::MODE_BWD) return launch_default<nbw::MODE_BWD>(g, a, bs, s);
+  if (mode == nbw::MODE_FWD) return launch_prj<nbw::MODE_FWD>(g, a, bs, s);
+  if (mode == nbw::MODE_BWD) return launch_prj<nbw::MODE_BWD>(g, a, bs, s);
+  // the fused mode's tile picks among the best shapes (batch.autotune); one image has one
   constexpr int M = nbw::MODE_OSEM;
-  if (tile == 0) return launch_default<M>(g, a, bs, s);
   if (bs == 4)
-    return tile == 1 ? launch<4, 2, 16, 1024, M, 1>(g, a, s) : launch<4, 4, 32, 512, M, 1>(g, a, s);
+    return tile == 0   ? launch<4, 4, 32, 512, M, 1>(g, a, s)
+           : tile == 1 ? launch<4, 4, 24, 384, M, 1>(g, a, s)
+                       : launch<4, 4, 32, 256, M, 1>(g, a, s);
   if (bs == 2)
-    return tile == 1 ? launch<2, 2, 16, 512, M, 2>(g, a, s) : launch<2, 2, 32, 1024, M, 1>(g, a, s);
-  return tile == 1 ? launch<1, 1, 32, 512, M, 2>(g, a, s) : launch<1, 1, 64, 1024, M, 1>(g, a, s);
+    return tile == 0   ? launch<2, 2, 64, 512, M, 1>(g, a, s)
+           : tile == 1 ? launch<2, 2, 24, 256, M, 2>(g, a, s)
+                       : launch<2, 2, 32, 256, M, 2>(g, a, s);
+  return launch<1, 1, 64, 512, M, 2>(g, a, s);
 }
 
 nbw::WalkArgs nb_walk_args(const nb_geom *g, const int32_t *subs, int nprj, int span, int nrep,

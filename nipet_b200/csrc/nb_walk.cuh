@@ -37,16 +37,18 @@
 // wave 9% of the SMs' time idle at 4894 LORs).
 //
 // Measured (B200, 1965 MHz; per call, against the step-by-step walk it replaces): attenuation
-// factors of all LORs at span 11 28.0 -> 4.0 ms (chunks without any value are skipped), a
-// 4894-LOR emission projection 2.16 -> 0.36 ms, a 5003-LOR span-1 back projection 2.58 ->
-// 0.84 ms, a drop-in OSEM iteration 64.5 -> 23.2 ms, 9 images batched 341 -> 215 ms.  Against
+// factors of all LORs at span 11 28.0 -> 3.4 ms (chunks without any value are skipped), a
+// 4894-LOR emission projection 2.16 -> 0.30 ms, a 5003-LOR span-1 back projection 2.57 ->
+// 0.84 ms, a drop-in OSEM iteration 64.4 -> 22.9 ms, 9 images batched 341 -> 172 ms.  Against
 // the FP64 oracle the error halves (forward 1.2e-7 -> 5e-8, back 1.5e-7 -> 6e-8 relative L2).
-// What bounds it: the shared-memory (LSU) pipe at 79 .. 81% of its wavefronts, half of them the
-// crossings' (a warp of 32 pairs spans up to 8 ring differences, whose lanes share banks: 3.1
-// wavefronts per 8-byte read where 2 would do); per LOR and image ~100k warp instructions, the
-// crossings 30%, running sums 21%, each chunk's set-up of the pairs 21% (64-step chunks in
-// place of 32 took 30% off).  Aligning differences to half-warps saved 20% of the crossings'
-// wavefronts and lost more to 20% more sets (0.77 -> 0.85 ms).
+// What bounds it: the shared-memory (LSU) pipe at 79 .. 81% of its wavefronts for one image,
+// half of them the crossings' (a warp of 32 pairs spans up to 8 ring differences, whose lanes
+// share banks: 3.1 wavefronts per 8-byte read where 2 would do); of the time the crossings take
+// a third, the running sums a fifth, each chunk's set-up of the pairs a seventh, the rest loads,
+// bounds and the LOR's start and end.  Aligning differences to half-warps saved 20% of the
+// crossings' wavefronts and lost more to 20% more sets (0.77 -> 0.85 ms); warps that own steps
+// instead (no tables: one shared reduction per crossing and ray) took 1.5 to 2 times as long
+// for one image and as long for four.
 #pragma once
 #include "nb_axial.cuh"
 #include "nb_internal.cuh"
@@ -74,6 +76,7 @@ struct WalkArgs {
   int att;                    // forward: 0 emission, 1 attenuation factors
   int in_by_lor;              // backward: row of a LOR is its LOR index, not its subset position
   const float *img;           // [ngroups][NCOL][128][BS]
+  int natural;                // forward, BS 1: img is the reference's [NCOL][127] instead
   float *bimg;                // same layout, accumulated
   float *sino;                // forward output [nrep][nprj][nout]
   const float *sino_in;       // backward input [nrep][nprj][nout] (or [naw][nout] if in_by_lor)
@@ -100,9 +103,9 @@ template <int BS, int CH, int NSEG> struct WSmem {
   static constexpr size_t run_off = align128(oc_off + 4ull * (CH + NSEG) * BS);      // [2][128][BS]
   static constexpr size_t rec_off = align128(run_off + 1024ull * BS);
   static constexpr size_t cs_off = align128(rec_off + NB_REC_MAX);          // [2][2][stride]
-  static constexpr size_t rat_off = align128(cs_off + 16ull * NB_STEP_STRIDE);
-  static constexpr size_t max_off = align128(rat_off + 837ull * 4 * BS);   // [3][NSEG][BS]
-  static constexpr size_t misc_off = align128(max_off + 12ull * NSEG * BS);
+  static constexpr size_t max_off = align128(cs_off + 16ull * NB_STEP_STRIDE);  // [3][NSEG][BS]
+  static constexpr size_t obl_off = align128(max_off + 12ull * NSEG * BS);      // [64]
+  static constexpr size_t misc_off = obl_off + 256;
   static constexpr size_t total = misc_off + 128;
   static_assert(total <= 227 * 1024, "too much shared memory");
 };
@@ -171,7 +174,7 @@ static __device__ __forceinline__ void lds_tab(uint32_t addr, int *D, int *X) {
 
 // byte offset of a plane in a row whose planes are `unit` bytes wide (even planes first)
 static __device__ __forceinline__ int plane_off(int P, int unit) {
-  return ((P >> 1) + ((P & 1) << 6)) * unit;
+  return P * (unit / 2) + (P & 1) * (127 * unit / 2);
 }
 static __device__ __forceinline__ float oblique_s(int d, float atn) {
   if (d == 0) return 1.f;
@@ -184,22 +187,25 @@ static __device__ __forceinline__ float oblique_s(int d, float atn) {
 template <int BS>
 static __device__ __noinline__ void slow_ray(const float *gimg, const int32_t *col,
                                              const float *st, float tp, int s0, int s1, int z,
-                                             int dir, const uint2 *ent, int cnt, float *acc) {
+                                             int dir, const uint2 *ent, int cnt, bool natural,
+                                             float *acc) {
+  // (plane 127 reads as zero: the padding slot, or no voxel in the natural order)
+  auto vox = [&](const float *c, int z, int k) {
+    return !natural ? c[nb_zi(z) * BS + k] : (z < NB_IMZ ? c[z] : 0.f);
+  };
   for (int s = s0; s < s1; s++) {
     const float tn = st[s], lt = __fsub_rn(tn, tp);
-    const float *c = gimg + (size_t)col[s] * NB_COLW * BS;
+    const float *c = gimg + (size_t)col[s] * (natural ? NB_IMZ : NB_COLW * BS);
     tp = tn;
-    const float *p0 = c + nb_zi(z) * BS;
     if (cnt > 0 && (int)ent->x == s) {
       const float f = (float)(int)ent->y * (1.f / (1 << QBITS));
-      z += dir;
-      const float *p1 = c + nb_zi(z) * BS;
       for (int k = 0; k < BS; k++)
-        acc[k] = fmaf(f * lt, p0[k], fmaf((1.f - f) * lt, p1[k], acc[k]));
+        acc[k] = fmaf(f * lt, vox(c, z, k), fmaf((1.f - f) * lt, vox(c, z + dir, k), acc[k]));
+      z += dir;
       ent++;
       cnt--;
     } else {
-      for (int k = 0; k < BS; k++) acc[k] = fmaf(lt, p0[k], acc[k]);
+      for (int k = 0; k < BS; k++) acc[k] = fmaf(lt, vox(c, z, k), acc[k]);
     }
   }
 }
@@ -208,12 +214,13 @@ template <int BS, int VB, int CH, int NT, int MODE, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
   constexpr int NSEG = NT * VB / (64 * BS);   // step segments of a chunk, one per 64 threads
   constexpr int SEGL = CH / NSEG;
-  constexpr int SPT = NB_NSLOT / NT;          // slots (ray pairs) per thread
+  constexpr int SPT = (NB_NSLOT + NT - 1) / NT;          // slots (ray pairs) per thread
   constexpr int W = NT / 32;
   constexpr int UNIT = BS == 1 ? 8 : 16;      // bytes per plane of a table row
   constexpr int LOGR = BS == 1 ? 10 : (BS == 2 ? 11 : 12);   // table row bytes
   constexpr int LOGG = LOGR - 1;                             // accumulator row bytes
   static_assert(CH % 8 == 0 && CH % NSEG == 0 && SEGL >= 1, "chunk shape");
+  static_assert(NSEG * BS % 4 == 0, "the bounds are read 16 bytes at a time");
   using L = WSmem<BS, CH, NSEG>;
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char *tab = smem;
@@ -224,7 +231,7 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
   int *soc = reinterpret_cast<int *>(smem + L::oc_off);              // prefixes of voxel 63
   int *srun = reinterpret_cast<int *>(smem + L::run_off);
   unsigned char *rec = smem + L::rec_off;
-  float *rat = reinterpret_cast<float *>(smem + L::rat_off);
+  float *sobl = reinterpret_cast<float *>(smem + L::obl_off);        // oblique length factors
   unsigned char *misc = smem + L::misc_off;
   uint64_t *bar = reinterpret_cast<uint64_t *>(misc);
   uint64_t *bar2 = reinterpret_cast<uint64_t *>(misc + 8);
@@ -306,6 +313,26 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
     if (tid == 0) nb_clc_request(clc, bar2);
 
     auto slot_of = [&](int j) { return ((j & 1) ? (j + 1) * W - 1 - warp : j * W + warp) * 32 + lane; };
+    // lengths of this thread's steps in the chunk at s0 (0 past the LOR's end, where the reads
+    // find other data of the block)
+    auto step_lengths = [&](int s0, float *lt) {
+      float t[SEGL];
+      const int f0 = s0 + seg * SEGL;
+      if (SEGL % 4 == 0) {
+#pragma unroll
+        for (int j = 0; j < SEGL; j += 4) ldv<4>(sst + f0 + j, t + j);
+      } else {
+#pragma unroll
+        for (int j = 0; j < SEGL; j++) t[j] = sst[f0 + j];
+      }
+      float tp = f0 ? sst[f0 - 1] : h.x;
+#pragma unroll
+      for (int j = 0; j < SEGL; j++) {
+        lt[j] = f0 + j < n ? __fsub_rn(t[j], tp) : 0.f;
+        tp = t[j];
+      }
+    };
+
     // this thread's slots: start planes of the two rays (8 bits each) and ring difference;
     // the few rays whose start plane rounds away from their group's are listed in the record
     uint32_t zzd[SPT];
@@ -315,18 +342,17 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
       const int sl = slot_of(j);
       zzd[j] = 0u;
       if (sl >= a.nslots) continue;
-      const nb_slot S = a.slots[sl];
-      const int m = rec[NB_REC_M + S.d];
-      int zA = S.zA + m - 1, zB = S.zB - m + 1;
+      const uint32_t zz = __ldg(&a.slots[sl].zzd);
+      // the upward ray starts m - 1 planes above its ring's, the downward one as many below
+      zzd[j] = zz - (uint32_t)(rec[NB_REC_M + (zz >> 16)] - 1) * 255u;
       for (int x = 0; x < nirr; x++) {
         const char4 e = reinterpret_cast<const char4 *>(rec + NB_REC_IRR)[x];
-        if (e.x == S.d && 2 * (int)e.y == S.zA) {
-          zA += e.z ? 0 : e.w;
-          zB += e.z ? e.w : 0;
-        }
+        if (e.x == (int)(zz >> 16) && 2 * (int)e.y == (int)(zz & 255u))
+          zzd[j] += (uint32_t)(e.z ? 256 * (int)e.w : (int)e.w);
       }
-      zzd[j] = (uint32_t)zA | (uint32_t)zB << 8 | (uint32_t)S.d << 16;
     }
+    if (tid < 64) sobl[tid] = oblique_s(tid, h.y);
+    if (MODE == MODE_BWD) __syncthreads();           // (the forward pass has later barriers)
 
     float FA[SPT][BS], FB[SPT][BS];           // forward: line integrals
 #pragma unroll
@@ -337,14 +363,27 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
     // ------------------------------------------------------------------ forward
     if (MODE != MODE_BWD) {
       float E[SEGL][VB], O[SEGL][VB];         // this thread's values: planes 2 s, 2 s + 1
+      const bool natural = MODE == MODE_FWD && BS == 1 && a.natural != 0;
       auto prefetch = [&](int c) {
+        int col[SEGL];
+        const int f0 = c * CH + seg * SEGL;
+        if (SEGL % 4 == 0) {
+#pragma unroll
+          for (int j = 0; j < SEGL; j += 4) ldi<4>(scol + f0 + j, col + j);
+        } else {
+#pragma unroll
+          for (int j = 0; j < SEGL; j++) col[j] = scol[f0 + j];
+        }
 #pragma unroll
         for (int j = 0; j < SEGL; j++) {
-          const int step = c * CH + seg * SEGL + j;
-          if (step < n) {
-            const float *x = gimg + ((size_t)scol[step] * NB_COLW + s) * BS + iv;
+          if (f0 + j < n) {
+            const float *x = gimg + (size_t)col[j] * (natural ? NB_IMZ : NB_COLW * BS) +
+                             (natural ? 2 * s : s * BS + iv);
             ldg_v<VB>(x, E[j]);
-            ldg_v<VB>(x + 64 * BS, O[j]);
+            if (natural && s == 63)
+              O[j][0] = 0.f;
+            else
+              ldg_v<VB>(x + (natural ? 1 : 64 * BS), O[j]);
           } else {
 #pragma unroll
             for (int v = 0; v < VB; v++) E[j][v] = O[j][v] = 0.f;
@@ -358,14 +397,10 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
         // of |value| of any plane
         float lt[SEGL];
         {
+          step_lengths(s0, lt);
           float m[VB];
 #pragma unroll
           for (int v = 0; v < VB; v++) m[v] = 0.f;
-#pragma unroll
-          for (int j = 0; j < SEGL; j++) {
-            const int step = s0 + seg * SEGL + j;
-            lt[j] = step < n ? __fsub_rn(sst[step], step ? sst[step - 1] : h.x) : 0.f;
-          }
 #pragma unroll
           for (int v = 0; v < VB; v++) {
             float me = 0.f, mo = 0.f;
@@ -382,12 +417,15 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
         unsigned any = 0u;
         bool slow = false;
         const float t0 = s0 ? sst[s0 - 1] : h.x;
-        float scale[BS], inv[BS];
+        float scale[BS], inv[BS], bnd[NSEG * BS];
+#pragma unroll
+        for (int x = 0; x < NSEG * BS; x += 4)
+          ldv<4>(reinterpret_cast<const float *>(smax) + mrot * NSEG * BS + x, bnd + x);
 #pragma unroll
         for (int k = 0; k < BS; k++) {
           float bound = 0.f;
 #pragma unroll
-          for (int x = 0; x < NSEG; x++) bound += __uint_as_float(smax[(mrot * NSEG + x) * BS + k]);
+          for (int x = 0; x < NSEG; x++) bound += bnd[x * BS + k];
           const unsigned bb = __float_as_uint(bound);
           any |= bb;
           // bound < 2^e: scale 2^(30 - e); non-finite, above 2^100 or below 2^-60: step by step
@@ -406,16 +444,18 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
         if (!slow) {
           // fixed-point running integrals: within the segment, then the segments before it
           int cE[SEGL][VB], cO[SEGL][VB], tE[VB], tO[VB];
+          float sv[VB];
 #pragma unroll
-          for (int v = 0; v < VB; v++) tE[v] = tO[v] = 0;
+          for (int v = 0; v < VB; v++) {
+            tE[v] = tO[v] = 0;
+            sv[v] = scale[v];
+            if (VB < BS && iv) sv[v] = scale[(VB + v) % BS];
+          }
 #pragma unroll
           for (int j = 0; j < SEGL; j++) {
 #pragma unroll
             for (int v = 0; v < VB; v++) {
-              float sc = scale[0];
-#pragma unroll
-              for (int k = 1; k < BS; k++) sc = (iv + v == k) ? scale[k] : sc;
-              const float w = lt[j] * sc;
+              const float w = lt[j] * sv[v];
               cE[j][v] = tE[v];
               cO[j][v] = tO[v];
               tE[v] += __float2int_rn(E[j][v] * w);
@@ -427,21 +467,29 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
           sti<VB>(sseg + (seg * 128 + s) * BS + iv, tE);
           sti<VB>(sseg + (seg * 128 + 64 + s) * BS + iv, tO);
           __syncthreads();
-          int bE[VB], bO[VB], bP[VB];
+          int bE[VB], bO[VB];
 #pragma unroll
-          for (int v = 0; v < VB; v++) bE[v] = bO[v] = bP[v] = 0;
+          for (int v = 0; v < VB; v++) bE[v] = bO[v] = 0;
           for (int x = 0; x < seg; x++) {
             int u[VB], w[VB];
             ldi<VB>(sseg + (x * 128 + s) * BS + iv, u);
             ldi<VB>(sseg + (x * 128 + 64 + s) * BS + iv, w);
 #pragma unroll
             for (int v = 0; v < VB; v++) bE[v] += u[v], bO[v] += w[v];
-            if (s == 32) {
+          }
+          // the thread of plane 64 gets plane 63's prefixes through shared memory (its neighbour
+          // is another warp's); the thread of plane 0 has no plane below and its D[0] no reader
+          const bool fix = s == 32;
+          int bP[VB];
+#pragma unroll
+          for (int v = 0; v < VB; v++) bP[v] = 0;
+          if (fix)
+            for (int x = 0; x < seg; x++) {
+              int u[VB];
               ldi<VB>(sseg + (x * 128 + 64 + 31) * BS + iv, u);
 #pragma unroll
               for (int v = 0; v < VB; v++) bP[v] += u[v];
             }
-          }
           if (seg == NSEG - 1) {              // the chunk's whole integral per plane
             int u[VB], w[VB];
 #pragma unroll
@@ -461,10 +509,7 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
               const int ce = (j < SEGL ? cE[j < SEGL ? j : 0][v] : tE[v]) + bE[v];
               const int co = (j < SEGL ? cO[j < SEGL ? j : 0][v] : tO[v]) + bO[v];
               int cp = __shfl_up_sync(0xffffffffu, co, 1);      // plane 2 s - 1
-              if (lane == 0) {
-                const int o = (seg * (SEGL + 1) + j) * BS + iv + v;
-                cp = s ? bP[v] + soc[o] : ce;
-              }
+              if (fix) cp = bP[v] + soc[(seg * (SEGL + 1) + j) * BS + iv + v];
               De[v] = cp - ce;
               Do[v] = ce - co;
               ne[v] -= De[v];
@@ -500,8 +545,8 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
           const int zA = (zz & 255) + ka, zB = ((zz >> 8) & 255) - ka;
           if (slow) {
             const uint2 *ent = reinterpret_cast<const uint2 *>(rec + NB_REC_ENT) + e0;
-            slow_ray<BS>(gimg, scol, sst, t0, s0, s1, zA, 1, ent, cnt, FA[j]);
-            slow_ray<BS>(gimg, scol, sst, t0, s0, s1, zB, -1, ent, cnt, FB[j]);
+            slow_ray<BS>(gimg, scol, sst, t0, s0, s1, zA, 1, ent, cnt, natural, FA[j]);
+            slow_ray<BS>(gimg, scol, sst, t0, s0, s1, zB, -1, ent, cnt, natural, FB[j]);
             continue;
           }
           const int endA = zA + cnt, endB = zB - cnt;
@@ -509,8 +554,9 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
           // cursors of the next crossing and the one after (their plane offsets in a row);
           // two crossings on, both have moved by one unit
           const uint32_t base = tab_u - ((uint32_t)s0 << LOGR);
-          uint32_t cA0 = base + plane_off(zA + 1, UNIT), cA1 = base + plane_off(zA + 2, UNIT);
-          uint32_t cB0 = base + plane_off(zB, UNIT), cB1 = base + plane_off(zB - 1, UNIT);
+          uint32_t cA0 = base + plane_off(zA + 1, UNIT), cB0 = base + plane_off(zB, UNIT);
+          uint32_t cA1 = cA0 + 64 * UNIT - ((zA + 1) & 1) * (127 * UNIT);
+          uint32_t cB1 = cB0 + 63 * UNIT - (zB & 1) * (127 * UNIT);
           // sums of D and of dD * fraction (64 bits: 2^30 by 2^31, up to ~100 of them)
           int iA[BS], iB[BS];
           long long xA[BS], xB[BS];
@@ -578,8 +624,10 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
       for (int j = 0; j < SPT; j++) {
         const int sl = slot_of(j);
         if (sl >= a.nslots) continue;
-        const nb_slot S = a.slots[sl];
-        const float so = oblique_s(S.d, h.y);
+        const nb_slot *S = a.slots + sl;
+        const float so = sobl[zzd[j] >> 16];
+        int oA = 0, oB = 0;
+        if (!span11) oA = S->o1A, oB = S->o1B;
 #pragma unroll
         for (int k = 0; k < BS; k++) {
           float vA = FA[j][k] * so, vB = FB[j][k] * so;
@@ -587,8 +635,8 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
             vA = expf(-vA);
             vB = expf(-vB);
             if (span11) {
-              vA = vA / (float)S.nosA;
-              vB = vB / (float)S.nosB;
+              vA = vA / (float)S->nosA;
+              vB = vB / (float)S->nosB;
             }
           }
           if (span11) {
@@ -598,12 +646,12 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
             const int rep = g * BS + k;
             if (rep < a.nrep) {
               float *row = a.sino + ((size_t)rep * a.nprj + p) * a.nout;
-              if (S.o1A >= 0) row[S.o1A] = vA;
-              if (S.o1B >= 0) row[S.o1B] = vB;
+              if (oA >= 0) row[oA] = vA;
+              if (oB >= 0) row[oB] = vB;
             }
           } else {
-            FA[j][k] = S.o1A >= 0 ? ratio(vA, S.o1A, k) : 0.f;
-            FB[j][k] = S.o1B >= 0 ? ratio(vB, S.o1B, k) : 0.f;
+            FA[j][k] = oA >= 0 ? ratio(vA, oA, k) : 0.f;
+            FB[j][k] = oB >= 0 ? ratio(vB, oB, k) : 0.f;
           }
         }
       }
@@ -621,7 +669,11 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
             const int rep = g * BS + k;
             if (rep < a.nrep) a.sino[((size_t)rep * a.nprj + p) * a.nout + o] = v;
           } else {
-            rat[x] = ratio(v, o, k);
+            // back to the bin's rays (a ray is in one bin; its integral is not read again)
+            v = ratio(v, o, k);
+#pragma unroll
+            for (int r = 0; r < 8; r++)
+              if (lst[r] >= 0) vals[lst[r] * BS + k] = v;
           }
         }
         if (MODE == MODE_OSEM) __syncthreads();
@@ -643,9 +695,9 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
           for (int k = 0; k < BS; k++) FA[j][k] = FB[j][k] = 0.f;
           continue;
         }
-        const nb_slot S = a.slots[sl];
-        const float so = oblique_s(S.d, h.y);
-        const int oA = span11 ? S.o11A : S.o1A, oB = span11 ? S.o11B : S.o1B;
+        const short2 o2 = __ldg(reinterpret_cast<const short2 *>(span11 ? &a.slots[sl].o11A : &a.slots[sl].o1A));
+        const float so = sobl[zzd[j] >> 16];
+        const int oA = o2.x, oB = o2.y;
 #pragma unroll
         for (int k = 0; k < BS; k++) {
           if (MODE == MODE_BWD) {
@@ -655,8 +707,8 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
             FA[j][k] = oA >= 0 && rep < a.nrep ? row[oA] : 0.f;
             FB[j][k] = oB >= 0 && rep < a.nrep ? row[oB] : 0.f;
           } else if (span11) {
-            FA[j][k] = oA >= 0 ? rat[oA * BS + k] : 0.f;
-            FB[j][k] = oB >= 0 ? rat[oB * BS + k] : 0.f;
+            FA[j][k] = oA >= 0 ? vals[(2 * sl) * BS + k] : 0.f;
+            FB[j][k] = oB >= 0 ? vals[(2 * sl + 1) * BS + k] : 0.f;
           }
           FA[j][k] *= so;
           FB[j][k] *= so;
@@ -669,10 +721,11 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
         const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(mm[k]));
         if (lane == 0 && m) atomicMax(&smaxb[par * BS + k], m);
       }
-      if (MODE == MODE_OSEM)
-        for (int i = tid; i < (CH + 1) * 128 * BS; i += NT) gacc[i] = 0;
       for (int i = tid; i < 128 * BS; i += NT) srun[i] = 0;
       __syncthreads();
+      if (MODE == MODE_OSEM)                  // (the ratios have been read; a barrier follows)
+        for (int i = tid; i < (CH + 1) * 32 * BS; i += NT)
+          reinterpret_cast<int4 *>(gacc)[i] = make_int4(0, 0, 0, 0);
       float inv[BS];
       int VA[SPT][BS], VB_[SPT][BS];          // the rays' values, integers
       unsigned any = 0u;
@@ -711,6 +764,7 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
           if (vB) reds_add_s32(run_u + (nb_zi(zB) * BS + k) * 4, vB);
         }
       }
+      if (MODE == MODE_OSEM) __syncthreads();
       float *gb = a.bimg + (size_t)g * NB_IMG_COL128 * BS;
       for (int c = 0; c < nchb; c++) {
         const int s0 = c * CH, s1 = min(n, s0 + CH);
@@ -725,8 +779,9 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
           const int zA = (zz & 255) + ka, zB = ((zz >> 8) & 255) - ka;
           uint32_t ep = rec_u + NB_REC_ENT + e0 * 8;
           const uint32_t base = g_u - ((uint32_t)s0 << LOGG);
-          uint32_t cA0 = base + plane_off(zA + 1, 4), cA1 = base + plane_off(zA + 2, 4);
-          uint32_t cB0 = base + plane_off(zB, 4), cB1 = base + plane_off(zB - 1, 4);
+          uint32_t cA0 = base + plane_off(zA + 1, 4), cB0 = base + plane_off(zB, 4);
+          uint32_t cA1 = cA0 + 256 - ((zA + 1) & 1) * 508;
+          uint32_t cB1 = cB0 + 252 - (zB & 1) * 508;
           // upward flow over a plane boundary is positive; image k of a row is k * 512 bytes on.
           // q = floor(f V) = high word of f 2^26 by V 2^6
           auto cross = [&](int f, uint32_t rA, uint32_t rB) {
@@ -764,15 +819,21 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
         if (last && tid == 0) next_job(job);
         // flows -> running sums: this thread's planes z = 2 s and 2 s + 1, SEGL steps
         int rE[SEGL][VB], rO[SEGL][VB], cy[2][VB];
+        int *g0 = gacc + (seg * SEGL * BS + iv) * 128 + s;
 #pragma unroll
         for (int v = 0; v < VB; v++) {
-          int tE = 0, tO = 0;
+          int tE = 0, tO = 0, lp[SEGL];
+          if (s == 31)                        // its neighbour above is another warp's
+#pragma unroll
+            for (int j = 0; j < SEGL; j++) lp[j] = g0[(j * BS + v) * 128 + 1];
+          if (s == 63)                        // nothing crosses the top of plane 127
+#pragma unroll
+            for (int j = 0; j < SEGL; j++) lp[j] = 0;
 #pragma unroll
           for (int j = 0; j < SEGL; j++) {
-            const int *row = gacc + (seg * SEGL + j) * 128 * BS + (iv + v) * 128;
-            const int ge = row[s], go = row[64 + s];
+            const int ge = g0[(j * BS + v) * 128], go = g0[(j * BS + v) * 128 + 64];
             int gn = __shfl_down_sync(0xffffffffu, ge, 1);
-            if (lane == 31) gn = s == 31 ? row[32] : 0;
+            if (lane == 31) gn = lp[j];
             tE += ge - go;
             tO += go - gn;
             rE[j][v] = tE;
@@ -781,11 +842,12 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
           sseg[(seg * 128 + s) * BS + iv + v] = tE;
           sseg[(seg * 128 + 64 + s) * BS + iv + v] = tO;
           if (seg == 0) {                     // the row that spills into the next chunk
-            const int *row = gacc + CH * 128 * BS + (iv + v) * 128;
-            cy[0][v] = row[s];
-            cy[1][v] = row[64 + s];
+            cy[0][v] = g0[(CH * BS + v) * 128];
+            cy[1][v] = g0[(CH * BS + v) * 128 + 64];
           }
         }
+        float lt[SEGL];
+        step_lengths(s0, lt);
         __syncthreads();
         const int *run0 = srun + (c & 1) * 128 * BS;
         int *run1 = srun + ((c & 1) ^ 1) * 128 * BS;
@@ -809,31 +871,35 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
           sti<VB>(run1 + s * BS + iv, u);
           sti<VB>(run1 + (64 + s) * BS + iv, w);
         }
+        float ie[VB], io[VB];                 // plane 127 is padding: nothing goes back to it
+#pragma unroll
+        for (int v = 0; v < VB; v++) {
+          ie[v] = inv[v];
+          if (VB < BS && iv) ie[v] = inv[(VB + v) % BS];
+          io[v] = s == 63 ? 0.f : ie[v];
+        }
+        float *o0 = stage + (seg * SEGL * 128 + s) * BS + iv;
 #pragma unroll
         for (int j = 0; j < SEGL; j++) {
-          const int row = seg * SEGL + j, step = s0 + row;
-          const float lt = step < n ? __fsub_rn(sst[step], step ? sst[step - 1] : h.x) : 0.f;
           int oe[VB], oo[VB];
 #pragma unroll
           for (int v = 0; v < VB; v++) {
-            float ic = inv[0];
-#pragma unroll
-            for (int k = 1; k < BS; k++) ic = (iv + v == k) ? inv[k] : ic;
-            const float w = lt * ic;
-            oe[v] = __float_as_int((float)(bE[v] + rE[j][v]) * w);
-            // plane 127 is padding: nothing is written back to it
-            oo[v] = s == 63 ? 0 : __float_as_int((float)(bO[v] + rO[j][v]) * w);
-            int *gr = gacc + row * 128 * BS + (iv + v) * 128;
-            gr[s] = row == 0 && !last ? cy[0][v] : 0;
-            gr[64 + s] = row == 0 && !last ? cy[1][v] : 0;
-            if (row == 0) {
-              gr[CH * 128 * BS + s] = 0;
-              gr[CH * 128 * BS + 64 + s] = 0;
-            }
+            oe[v] = __float_as_int((float)(bE[v] + rE[j][v]) * (lt[j] * ie[v]));
+            oo[v] = __float_as_int((float)(bO[v] + rO[j][v]) * (lt[j] * io[v]));
+            g0[(j * BS + v) * 128] = 0;
+            g0[(j * BS + v) * 128 + 64] = 0;
           }
-          int *so = reinterpret_cast<int *>(stage) + (row * 128 + s) * BS + iv;
-          sti<VB>(so, oe);
-          sti<VB>(so + 64 * BS, oo);
+          sti<VB>(reinterpret_cast<int *>(o0) + j * 128 * BS, oe);
+          sti<VB>(reinterpret_cast<int *>(o0) + j * 128 * BS + 64 * BS, oo);
+        }
+        if (seg == 0) {
+#pragma unroll
+          for (int v = 0; v < VB; v++) {
+            g0[v * 128] = last ? 0 : cy[0][v];
+            g0[v * 128 + 64] = last ? 0 : cy[1][v];
+            g0[(CH * BS + v) * 128] = 0;
+            g0[(CH * BS + v) * 128 + 64] = 0;
+          }
         }
         nb_fence_proxy_async_smem();
         __syncthreads();
