@@ -168,3 +168,24 @@ def test_hist_trim_releases_the_replicate_scratch(params, stream, cuda_device):
     assert free1 - free0 >= 72557856 * 8 * 4 * 0.9   # the span-11 scratch of 4 replicates
     b = mmr_lmproc.hist_stream(stream, params['txLUT'], params['axLUT'], Cnt, nrep=4, seed=3)
     assert torch.equal(a['psino'], b['psino']) and torch.equal(a['ssr'], b['ssr'])
+
+
+@pytest.mark.parametrize('n', [1, 3, 4, 1023, 4 * 1184 * 256 * 2 + 5])
+@pytest.mark.parametrize('off', [0, 1, 4])
+def test_unpack_sizes_and_alignments(cuda_device, n, off):
+    """Prompts, delayeds and totals of a packed sinogram at any length and start."""
+    import ctypes as C
+    from nipet_b200 import _lib
+    from nipet_b200.device import dev_ptr, stream_ptr
+    g = torch.Generator(device=cuda_device).manual_seed(n + off)
+    w = torch.randint(-2 ** 31, 2 ** 31, (n + off,), generator=g, device=cuda_device).to(torch.int32)
+    out = [torch.full((n + off + 1,), 7, device=cuda_device, dtype=torch.int16) for _ in range(2)]
+    ps, ds = C.c_ulonglong(), C.c_ulonglong()
+    _lib.check(_lib.load().nb_hist_unpack(dev_ptr(w[off:]), n, dev_ptr(out[0][off:]),
+                                          dev_ptr(out[1][off:]), C.byref(ps), C.byref(ds),
+                                          stream_ptr(cuda_device)))
+    x = w[off:].to(torch.int64) & 0xffffffff
+    for got, want, total in ((out[0], x & 0xffff, ps), (out[1], x >> 16, ds)):
+        assert torch.equal(got[off:-1].to(torch.int64) & 0xffff, want)
+        assert int(got[-1]) == 7 and (off == 0 or int(got[off - 1]) == 7)
+        assert total.value == int(want.sum())
