@@ -24,9 +24,10 @@ import numpy as np
 import torch
 
 from . import _lib, geometry, phantoms
-from .device import dev_ptr, device_of, get_geometry, resolve_device, stream_ptr
+from .device import (dev_ptr, device_of, get_geometry, resolve_device, stream_ptr,
+                     to_device)
 from .geometry import get_subsets14
-from .petprj import COL128, from_col128, to_col128
+from .petprj import COL128, _writeback, from_col128, to_col128
 
 __all__ = ['get_subsets14', 'subset_table', 'synthetic_scan', 'Recon', 'norm_sinogram_gpu',
            'osemone', 'image_affine', 'RecOut', 'ISOTOPES']
@@ -403,8 +404,8 @@ def osemone(datain, mumaps, hst, scanner_params, recmod=3, itr=4, fwhm=0., psf=N
         asng = _gapfree(attnsino, txLUT, Cnt, dev, torch.float32)
     else:
         muh, muo = mumaps
-        as_dev = lambda m: torch.as_tensor(np.asarray(m, np.float32) if not isinstance(  # noqa: E731
-            m, torch.Tensor) else m).to(dev, torch.float32)
+        as_dev = lambda m: (m.to(dev, torch.float32) if isinstance(m, torch.Tensor) else  # noqa: E731
+                            to_device(np.asarray(m, np.float32), np.float32, dev))
         mus = geo.convert2dev(as_dev(muo) + as_dev(muh), Cnt)
         asng = attenuation_sino(mus, scanner_params, dev, span)
     # randoms
@@ -441,7 +442,9 @@ def osemone(datain, mumaps, hst, scanner_params, recmod=3, itr=4, fwhm=0., psf=N
             rec.set_scatter(_gapfree(ssn, txLUT, Cnt, dev, torch.float32))
     rec.geom.check()
     dcycrr, qf, qf_loc = decay_quant_factors(hst, Cnt, ncmp, decay_ref_time)
-    im = geo.convert2e7(rec.image(img) * np.float32(dcycrr * qf * qf_loc), Cnt).cpu().numpy()
+    d_im = geo.convert2e7(rec.image(img) * np.float32(dcycrr * qf * qf_loc), Cnt)
+    im = np.empty(tuple(d_im.shape), np.float32)
+    _writeback(im, d_im)
     opth = outpath if outpath is not None else os.path.join(datain.get('corepath', ''),
                                                             'reconstructed')
     if fout is None:
