@@ -102,6 +102,11 @@ static __device__ __forceinline__ void nb_bulk_g2s(void *dst_smem, const void *s
       : "memory");
 }
 
+// global -> L2 prefetch (16-byte aligned, bytes a multiple of 16)
+static __device__ __forceinline__ void nb_bulk_prefetch_l2(const void *src_gmem, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src_gmem), "r"(bytes) : "memory");
+}
+
 // shared -> global bulk reduction (element-wise fp32 add performed at L2)
 static __device__ __forceinline__ void nb_bulk_reduce_add_f32(float *dst_gmem,
                                                               const float *src_smem,

@@ -27,18 +27,20 @@ int launch(nb_geom *g, const nbw::WalkArgs &a, cudaStream_t s) {
 }
 
 // Kernel shapes <BS, images per thread of the running sums, steps per chunk, threads, mode,
-// blocks per SM>.  One image: two blocks of 512 threads at 64 registers (256 threads at 128: 4%
-// slower forward, 13% in the fused mode; 32-step chunks 14% and 6%).  Two and four images need
-// the registers: 16 warps of 128 registers an SM beat 32 of 64, which spill (us per image and
-// 4894 LORs, dense image; fused sub-iteration / forward / back):
-//   two images    24 steps, 2 x 512 threads  1593 / 741 / 693
-//                 24 steps, 2 x 256 threads  1383 / 693 / 644
-//                 32 steps, 2 x 256 threads  1471 / 641 / 633
-//                 64 steps, 1 x 512 threads  1361 / 651 / 716
-//   four images   32 steps, 1 x 1024 threads 1727 / 942 / 735
-//                 32 steps, 1 x 512 threads  1346 / 687 / 651
-//                 24 steps, 1 x 384 threads  1475 / 763 / 681
-//                 32 steps, 1 x 256 threads  1469 / 751 / 693
+// blocks per SM>.  One image: two blocks of 512 threads at 64 registers.  Two and four images
+// need the registers: 16 warps of 128 registers an SM beat 32 of 64, which spill (us per image
+// and 4894 LORs, dense image: fused sub-iteration / forward / back):
+//   one image     64 steps, 2 x 512 threads  1486 / 701 / 764
+//                 64 steps, 2 x 256 threads  1653 / 754 / 825
+//                 32 steps, 2 x 512 threads  1681 / 797 / 803
+//   two images    32 steps, 2 x 256 threads  1257 / 643 / 628
+//                 24 steps, 2 x 256 threads  1342 / 698 / 644
+//                 64 steps, 1 x 512 threads  1361 / 661 / 720
+//                 24 steps, 2 x 384 threads  1406 / 685 / 675
+//   four images   32 steps, 1 x 512 threads  1283 / 690 / 649
+//                 24 steps, 1 x 384 threads  1414 / 780 / 681
+//                 32 steps, 1 x 256 threads  1460 / 754 / 694
+//                 32 steps, 1 x 1024 threads 1727 / 942 / 735
 template <int MODE> int launch_prj(nb_geom *g, const nbw::WalkArgs &a, int bs, cudaStream_t s) {
   if (bs == 4) return launch<4, 4, 32, 512, MODE, 1>(g, a, s);
   if (bs == 2) return launch<2, 2, 32, 256, MODE, 2>(g, a, s);
@@ -58,9 +60,9 @@ int nb_walk_launch(nb_geom *g, const nbw::WalkArgs &a, int mode, int bs, int til
            : tile == 1 ? launch<4, 4, 24, 384, M, 1>(g, a, s)
                        : launch<4, 4, 32, 256, M, 1>(g, a, s);
   if (bs == 2)
-    return tile == 0   ? launch<2, 2, 64, 512, M, 1>(g, a, s)
+    return tile == 0   ? launch<2, 2, 32, 256, M, 2>(g, a, s)
            : tile == 1 ? launch<2, 2, 24, 256, M, 2>(g, a, s)
-                       : launch<2, 2, 32, 256, M, 2>(g, a, s);
+                       : launch<2, 2, 64, 512, M, 1>(g, a, s);
   return launch<1, 1, 64, 512, M, 2>(g, a, s);
 }
 

@@ -39,7 +39,7 @@
 // Measured (B200, 1965 MHz; per call, against the step-by-step walk it replaces): attenuation
 // factors of all LORs at span 11 28.0 -> 3.4 ms (chunks without any value are skipped), a
 // 4894-LOR emission projection 2.16 -> 0.30 ms, a 5003-LOR span-1 back projection 2.57 ->
-// 0.84 ms, a drop-in OSEM iteration 64.4 -> 22.9 ms, 9 images batched 341 -> 172 ms.  Against
+// 0.84 ms, a drop-in OSEM iteration 64.4 -> 20.9 ms, 9 images batched 341 -> 163 ms.  Against
 // the FP64 oracle the error halves (forward 1.2e-7 -> 5e-8, back 1.5e-7 -> 6e-8 relative L2).
 // What bounds it: the shared-memory (LSU) pipe at 79 .. 81% of its wavefronts for one image,
 // half of them the crossings' (a warp of 32 pairs spans up to 8 ring differences, whose lanes
@@ -288,7 +288,27 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
       nb_set_error(a.err, NB_DEVERR_MBAR_TIMEOUT);
     }
     *snext = q;
-    if (q >= 0) issue(q, (job + 1) & 1);
+    if (q >= 0) {
+      issue(q, (job + 1) & 1);
+      if (MODE != MODE_FWD) {                // the next job's rows, into L2 (two images: 1%)
+        const int p = q / a.ngroups, g = q - p * a.ngroups;
+        int lor = a.subs ? a.subs[p] : p;
+        lor = lor < 0 || lor >= a.naw ? 0 : lor;
+        auto row = [](const void *x, size_t bytes) {
+          const uintptr_t a0 = ((uintptr_t)x + 15) & ~(uintptr_t)15, a1 = ((uintptr_t)x + bytes) & ~(uintptr_t)15;
+          if (a1 > a0) nb_bulk_prefetch_l2((const void *)a0, (uint32_t)(a1 - a0));
+        };
+        for (int k = 0; k < BS; k++) {
+          const int rep = g * BS + k;
+          if (rep >= a.nrep) break;
+          if (MODE == MODE_BWD)
+            row(a.sino_in + ((size_t)rep * a.nprj + (a.in_by_lor ? lor : p)) * a.nout, 4 * (size_t)a.nout);
+          else
+            row(a.psng + ((size_t)rep * a.naw + lor) * a.nout, 2 * (size_t)a.nout);
+        }
+        if (MODE == MODE_OSEM) row(a.rs + (size_t)lor * a.nout, 4 * (size_t)a.nout);
+      }
+    }
   };
   if (tid == 0) issue(blockIdx.x, 0);
 
@@ -364,7 +384,7 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
     if (MODE != MODE_BWD) {
       float E[SEGL][VB], O[SEGL][VB];         // this thread's values: planes 2 s, 2 s + 1
       const bool natural = MODE == MODE_FWD && BS == 1 && a.natural != 0;
-      auto prefetch = [&](int c) {
+      auto load = [&](int c) {
         int col[SEGL];
         const int f0 = c * CH + seg * SEGL;
         if (SEGL % 4 == 0) {
@@ -390,9 +410,11 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
           }
         }
       };
-      if (nch) prefetch(0);
       for (int c = 0; c < nch; c++) {
         const int s0 = c * CH, s1 = min(n, s0 + CH);
+        // (holding the next chunk's values through the walk instead hid their latency but
+        // spilled: 1604 against 1487 us for one image's fused subset, 1471 against 1267 for two)
+        load(c);
         // bound of the chunk's integrals per image: over its segments, the largest integral
         // of |value| of any plane
         float lt[SEGL];
@@ -437,10 +459,7 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
         // cleared two chunks before its next use: its last readers are one barrier back
         if (tid < NSEG * BS) smax[((mrot + 2) % 3) * NSEG * BS + tid] = 0u;
         mrot = (mrot + 1) % 3;
-        if (any == 0u) {                      // nothing but zeros
-          if (c + 1 < nch) prefetch(c + 1);
-          continue;
-        }
+        if (any == 0u) continue;              // nothing but zeros
         if (!slow) {
           // fixed-point running integrals: within the segment, then the segments before it
           int cE[SEGL][VB], cO[SEGL][VB], tE[VB], tO[VB];
@@ -532,7 +551,6 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
           }
           __syncthreads();
         }
-        if (c + 1 < nch) prefetch(c + 1);
 
         const unsigned char *kend = rec + NB_REC_KEND;
         const int krow0 = c * (CH / 8) - 1, krow1 = (s1 - 1) >> 3;
