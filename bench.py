@@ -304,7 +304,7 @@ def run_osem(args, ws, rank, dev):
         'gpu_launches': launches_per_step,
         'roofline': {'bound': 'hbm', 'achieved': achieved, 'peak': peak, 'unit': 'GB/s',
                      'frac': achieved / peak, 'traffic': tr,
-                     'kernel': 'k_project<OSEM> fused sub-iteration (nb_osem_subset)',
+                     'kernel': 'k_walk fused sub-iteration (nb_osem_subset)',
                      'peak_kind': peak_kind,
                      'bytes_per_launch_avg': float(np.mean(byt)),
                      'launch_ms_avg': float(np.mean(dur)) * 1e3},
@@ -368,7 +368,7 @@ def run_batch(args, ws, rank, dev):
         for _ in range(4):
             br.iteration(use_graph=True)
 
-    # per-launch algorithmic bytes of k_osem_batch (subset i): 8 B per forward voxel read and
+    # per-launch algorithmic bytes of the fused k_walk launch (subset i): 8 B per forward voxel read and
     # back-projection update per image, the images' prompt rows (2 B) and one (r+s)/(an)
     # and a*n row per image group (4 B each)
     _, per_lor = br.geom.count_reads(per_lor=True)
@@ -409,12 +409,11 @@ def run_batch(args, ws, rank, dev):
     launches_per_step = br.launches // args.steps
     t_step = _max_over_ranks(float(np.mean(times)), ws, dev)
     value = ws * nrep / t_step
-    # roofline of the dominant kernel, k_osem_batch (one graph replay = 14 of its launches +
-    # 14 image updates, ~1% of the replay).  Its binding resource is the shared-memory
-    # pipe: every Siddon voxel read/update is served from image columns staged in shared
-    # memory, each staged column serving ~35 rays.  achieved = shared-memory wavefronts of
-    # one launch (ncu count of the 8-image capture of this kernel shape -- 2 groups of 4 --
-    # scaled by the number of 4-image groups, since every group walks every LOR) over the
+    # roofline of the dominant kernel, k_walk (one graph replay = 14 of its launches + 14
+    # image updates, ~2% of the replay).  Its binding resource is the shared-memory pipe: a
+    # ray looks its plane crossings up in (adds them into) tables of running plane integrals
+    # there.  achieved = shared-memory wavefronts of one launch (ncu count of the 8-image
+    # capture of the same batch width, scaled by the image slots walked) over the
     # launch's live CUDA-event time; peak = one wavefront per cycle per SM at the sampled
     # clock.  Beside it: real DRAM traffic (ncu dram bytes, scaled the same way) against the
     # measured HBM bandwidth, and the algorithmic bytes (4 B per voxel read/update as if
@@ -424,17 +423,17 @@ def run_batch(args, ws, rank, dev):
     achieved_alg = bytes_iter / t_it / 1e9
     peak, peak_kind = _peaks()
     # the 8-image capture walks 8 image slots; a narrower tail launch is scaled the same
-    # way, per image slot (its per-image shared traffic is that of width 4 within a few %)
-    gscale = slots / 8.0 if br.bs == 4 else None
-    tr8 = _traffic('osem_batch_8img')
-    wf8 = _traffic('osem_batch_8img_smem_wavefronts')
+    # way, per image slot
+    gscale = slots / 8.0 if br.bs in (2, 4) else None
+    tr8 = _traffic(f'osem_batch_8img_w{br.bs}')
+    wf8 = _traffic(f'osem_batch_8img_w{br.bs}_smem_wavefronts')
     traffic = None if (tr8 is None or gscale is None) else tr8 * gscale
     nsm = torch.cuda.get_device_properties(dev).multi_processor_count
     mhz = clocks['sm_mhz'] if clocks and clocks.get('sm_mhz') else 1965.0
     smem_peak = nsm * mhz * 1e6
     tail = (f' + {br.parts[1].n} at width {br.parts[1].bs} in a second launch'
             if len(br.parts) > 1 else '')
-    kernel = (f'k_osem_batch (nb_osem_batch_subset, {br.bs} images per walk, tile {br.tile}, '
+    kernel = (f'k_walk fused mode (nb_osem_batch_subset, {br.bs} images per walk, tile {br.tile}, '
               f'{br.parts[0].ngroups} image groups per launch{tail}; a launch here is one '
               'sub-iteration)')
     if wf8 and gscale is not None:
@@ -453,13 +452,13 @@ def run_batch(args, ws, rank, dev):
                    'achieved': None if traffic is None else traffic / t_launch / 1e9,
                    'frac': None if traffic is None else traffic / t_launch / 1e9 / peak,
                    'source': 'ncu dram__bytes_read.sum + dram__bytes_write.sum per launch '
-                             '(8-image capture x groups / 2) over the live launch time'}
+                             '(8-image capture x image slots / 8) over the live launch time'}
     roof['algorithmic'] = {'unit': 'GB/s', 'bytes_per_launch': bytes_iter / len(br.subs),
                            'achieved': achieved_alg, 'frac_of_hbm_peak': achieved_alg / peak,
                            'note': '4 B per Siddon voxel read and per back-projection '
                                    'update, per image, as if every one came from HBM, + '
-                                   'sinogram rows; above 1 because staged columns are '
-                                   'reused from shared memory'}
+                                   'sinogram rows; above 1 because a ray looks '
+                                   'up its plane crossings instead of visiting voxels'}
 
     # e2e through the public batch API: pinned host prompts -> device, reconstruction,
     # voxel-wise mean/std images back to the host.  The device run's buffers go back to
@@ -601,8 +600,8 @@ def run_diff(args, ws, rank, dev):
     drs = [_traffic(k) for k in ('diff_fwd8', 'diff_bwd8', 'att_fprj')]
     algorithmic = {'unit': 'GB/s', 'achieved': alg, 'frac_of_hbm_peak': alg / peak,
                    'note': '4 B per Siddon voxel read and update, per image, as if every one '
-                           'came from HBM; above 1 because staged columns are reused from '
-                           'shared memory'}
+                           'came from HBM; above 1 because a ray looks up its plane '
+                           'crossings instead of visiting voxels'}
     if all(wfs):
         nsm = torch.cuda.get_device_properties(dev).multi_processor_count
         mhz = clocks['sm_mhz'] if clocks and clocks.get('sm_mhz') else 1965.0
@@ -613,9 +612,9 @@ def run_diff(args, ws, rank, dev):
                 'peak_kind': f'1 shared-memory wavefront/cycle/SM x {nsm} SMs x {mhz:.0f} MHz '
                              '(median sampled clock)',
                 'traffic': dstep,
-                'kernel': 'k_osem_batch forward + backward modes (nb_fprj_batch / '
-                          'nb_bprj_batch, 4 images per walk) + 2 attenuation projections '
-                          '(k_project), whole step',
+                'kernel': 'k_walk forward and backward modes (nb_fprj_batch / '
+                          'nb_bprj_batch, 4 images per walk) + 2 attenuation projections, '
+                          'whole step',
                 'wavefronts_per_step': wstep,
                 'hbm': ({'unit': 'GB/s', 'peak': peak, 'peak_kind': peak_kind,
                          'achieved': dstep / t_step / 1e9,
@@ -624,8 +623,7 @@ def run_diff(args, ws, rank, dev):
     else:
         roof = {'bound': 'hbm', 'achieved': alg, 'peak': peak, 'unit': 'GB/s',
                 'frac': alg / peak, 'traffic': None, 'peak_kind': peak_kind,
-                'kernel': 'k_osem_batch forward + backward modes + attenuation k_project, '
-                          'whole step', 'note': 'algorithmic bytes: no capture in '
+                'kernel': 'k_walk forward and backward modes + attenuation, whole step', 'note': 'algorithmic bytes: no capture in '
                                                 'profiles/traffic.json'}
     res = {'ms_per_step': t_step * 1e3, 'value': ws * nimg / t_step,
            'e2e': {'value': ws * nimg / te, 'unit': 'images/s',
@@ -677,7 +675,7 @@ def run_dynamic(args, ws, rank, dev):
                 ev.append((e0, e1))
         return dyn.nll_gradients()
 
-    # per-launch algorithmic bytes of k_osem_batch at span 1 (as in the batch workload:
+    # per-launch algorithmic bytes of the fused k_walk launch at span 1 (as in the batch workload:
     # 8 B per voxel read/update per frame, prompt rows and one (r+s)/(an), a*n row per group)
     _, per_lor = br.geom.count_reads(per_lor=True)
     ngroups = sum(p.ngroups for p in br.parts)
@@ -712,15 +710,15 @@ def run_dynamic(args, ws, rank, dev):
     algorithmic = {'unit': 'GB/s', 'achieved': achieved, 'frac_of_hbm_peak': achieved / peak,
                    'bytes_per_launch_avg': bytes_iter / len(br.subs),
                    'note': '4 B per Siddon voxel read and update per frame, as if every one '
-                           'came from HBM, + sinogram rows; above 1 because staged columns '
-                           'are reused from shared memory'}
-    # bound: the shared-memory pipe; wavefronts of one span-1 launch for one group of 4
-    # frames (ncu count of the same kernel shape on subset 0, `profile_cases.py diffdyn`),
-    # scaled by the launch's groups (every group walks every LOR of the subset; the 14
-    # subsets have the same number of LORs)
-    wf4 = _traffic('dyn_span1_4frames_smem_wavefronts')
-    dr4 = _traffic('dyn_span1_4frames')
-    if wf4 and br.bs == 4 and br.tile == 0:   # the captured shape
+                           'came from HBM, + sinogram rows; above 1 because a ray looks up '
+                           'its plane crossings instead of visiting voxels'}
+    # bound: the shared-memory pipe; wavefronts of one span-1 launch for 4 frames at the
+    # same batch width (ncu count on subset 0, `profile_cases.py diffdyn`), scaled by the
+    # launch's frame slots (the 14 subsets have the same number of LORs)
+    wf4 = _traffic(f'dyn_span1_4frames_w{br.bs}_smem_wavefronts')
+    dr4 = _traffic(f'dyn_span1_4frames_w{br.bs}')
+    ngroups = ngroups * br.bs / 4.0   # in fours of frames, as captured
+    if wf4 and br.tile == 0:          # the captured shape
         nsm = torch.cuda.get_device_properties(dev).multi_processor_count
         mhz = clocks['sm_mhz'] if clocks and clocks.get('sm_mhz') else 1965.0
         wl = wf4 * ngroups
@@ -729,8 +727,8 @@ def run_dynamic(args, ws, rank, dev):
                 'peak_kind': f'1 shared-memory wavefront/cycle/SM x {nsm} SMs x {mhz:.0f} MHz '
                              '(median sampled clock)',
                 'traffic': dr4 * ngroups if dr4 else None,
-                'kernel': f'k_osem_batch span 1 (nb_osem_batch_subset, {br.bs} frames per '
-                          f'walk, tile {br.tile}, {ngroups} frame groups per launch)',
+                'kernel': f'k_walk fused mode, span 1 (nb_osem_batch_subset, {br.bs} frames per '
+                          f'walk, tile {br.tile})',
                 'wavefronts_per_launch': wl, 'launch_ms_avg': launch_s * 1e3,
                 'hbm': ({'unit': 'GB/s', 'peak': peak, 'peak_kind': peak_kind,
                          'achieved': dr4 * ngroups / launch_s / 1e9,
@@ -739,7 +737,7 @@ def run_dynamic(args, ws, rank, dev):
     else:
         roof = {'bound': 'hbm', 'achieved': achieved, 'peak': peak, 'unit': 'GB/s',
                 'frac': achieved / peak, 'traffic': None, 'peak_kind': peak_kind,
-                'kernel': f'k_osem_batch span 1 (nb_osem_batch_subset, {br.bs} frames per '
+                'kernel': f'k_walk fused mode, span 1 (nb_osem_batch_subset, {br.bs} frames per '
                           f'walk, tile {br.tile})',
                 'bytes_per_launch_avg': bytes_iter / len(br.subs),
                 'launch_ms_avg': launch_s * 1e3,
@@ -1021,14 +1019,14 @@ def run_chain(args, ws, rank, dev):
     te = _max_over_ranks(float(np.mean(et)), ws, dev)
     # bound of the fused sub-iteration: the shared-memory pipe, with the wavefronts of one
     # subset launch from the one-kernel capture of the same kernel on a subset of the same
-    # size (profiles/k_project_subset_ncu_full.md); the 14 subsets have equal LOR counts
+    # size (counts in profiles/traffic.json); the 14 subsets have equal LOR counts
     wf = _traffic('osem_subiteration_smem_wavefronts')
     tr = _traffic('osem_subiteration')
     algorithmic = {'unit': 'GB/s', 'achieved': achieved, 'frac_of_hbm_peak': achieved / peak,
                    'bytes_per_launch_avg': float(np.mean(byt)),
                    'note': '4 B per Siddon voxel read and update as if every one came from '
-                           'HBM, + sinogram rows; above 1 because staged columns are reused '
-                           'from shared memory'}
+                           'HBM, + sinogram rows; above 1 because a ray looks up its plane '
+                           'crossings instead of visiting voxels'}
     if wf:
         nsm = torch.cuda.get_device_properties(dev).multi_processor_count
         mhz = clocks['sm_mhz'] if clocks and clocks.get('sm_mhz') else 1965.0
@@ -1037,7 +1035,7 @@ def run_chain(args, ws, rank, dev):
                 'unit': 'wavefronts/s', 'frac': wf / la / (nsm * mhz * 1e6),
                 'peak_kind': f'1 shared-memory wavefront/cycle/SM x {nsm} SMs x {mhz:.0f} MHz '
                              '(median sampled clock)',
-                'traffic': tr, 'kernel': 'k_project<OSEM> fused sub-iteration inside osemone',
+                'traffic': tr, 'kernel': 'k_walk fused sub-iteration inside osemone',
                 'wavefronts_per_launch': wf, 'launch_ms_avg': la * 1e3,
                 'hbm': ({'unit': 'GB/s', 'peak': peak, 'peak_kind': peak_kind,
                          'achieved': tr / la / 1e9, 'frac': tr / la / 1e9 / peak}
@@ -1046,7 +1044,7 @@ def run_chain(args, ws, rank, dev):
     else:
         roof = {'bound': 'hbm', 'achieved': achieved, 'peak': peak, 'unit': 'GB/s',
                 'frac': achieved / peak, 'traffic': tr,
-                'kernel': 'k_project<OSEM> fused sub-iteration inside osemone',
+                'kernel': 'k_walk fused sub-iteration inside osemone',
                 'peak_kind': peak_kind, 'bytes_per_launch_avg': float(np.mean(byt)),
                 'launch_ms_avg': float(np.mean(dur)) * 1e3}
     res = {'ms_per_step': t_step * 1e3, 'value': ws / t_step,

@@ -3,7 +3,7 @@
 All images share the scanner geometry, attenuation x normalisation (a*n) and hence the
 per-subset sensitivity images; each has its own prompts and a randoms level
 (`rscale[b]` times a common (r+s)/(an) sinogram).  One sub-iteration of all images is one
-persistent kernel launch (`nb_osem_batch_subset`) -- two when the images left over by the
+fused kernel launch (`nb_osem_batch_subset`) -- two when the images left over by the
 batch width go through a narrower launch of their own (`split_parts`) -- and a full
 iteration (14 sub-iterations) can be captured once as a CUDA graph and replayed.  The
 batch width `bs` (images sharing one walk of the Siddon geometry) and the kernel's tile

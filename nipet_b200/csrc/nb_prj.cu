@@ -270,7 +270,7 @@ extern "C" int nb_bprj(nb_geom *g, float *im, const float *sino, const int32_t *
 // RNG_END, prjf.cu:209-320, prjb.cu:190-308): images are the range's axial slab
 // [320][320][nvz], sinograms [nprj][nsino] numbered by the range's Michelogram.  The slab
 // is expanded into the handle's col128 scratch with zeros elsewhere (as the reference's
-// imExpand) and the persistent projector walks only the range's rays.
+// imExpand) and the projector walks only the range's rays.
 static int check_rings(nb_geom *g, const nb_rings *rr) {
   NB_REQUIRE(rr != nullptr, "NULL ring-range handle");
   NB_REQUIRE(rr->device == g->device, "ring-range handle and geometry on different devices");

@@ -1,16 +1,16 @@
 """Benchmark infrastructure beside bench.py: small, self-contained GPU cases for profiling the hot kernels with Nsight Compute.
 
-    python profile_cases.py projectors   # k_project: back, forward, fused OSEM
+    python profile_cases.py projectors   # k_walk, one image: back, forward, fused OSEM
     python profile_cases.py hist         # k_hist on a 20M-word stream
     python profile_cases.py hist200      # k_hist on the 2e8-word, 600 s stream
     python profile_cases.py hist200boot  # the same with 4 Poisson replicates
 
 `projectors` builds the geometry, a phantom image (col128 layout), subset 3 of 14 and random
 prompt / (r+s)/(an) / a*n sinograms (~0.8 GB on the device), then launches the back projection
-(sensitivity), forward projection and fused OSEM sub-iteration six times each, so the k_project
+(sensitivity), forward projection and fused OSEM sub-iteration six times each, so the k_walk
 launches 15, 16, 17 are one warm launch of each mode:
 
-    ncu --set full --clock-control none -k regex:k_project -s 15 -c 3 -o prof \\
+    ncu --set full --clock-control none -k regex:^k_walk -s 15 -c 3 -o prof \\
         python profile_cases.py projectors
 
 `hist` histograms a synthetic 20M-word span-11 stream three times (capture -k regex:k_hist -s 2);
@@ -23,13 +23,13 @@ k_slab_add).
 `sct` runs the scatter model twice (capture -k regex:k_sct_psct -s 1 -c 1).
 
 `batch` runs one batched OSEM sub-iteration (subset 0) for 8 images with batch widths 4 and
-2, twice each (capture -k regex:k_osem_batch -s 2 -c 2 for the second launch of each width:
+2, twice each (capture -k regex:^k_walk -c 4 for two launches of each width:
 launches 0, 1 are width 4, 2, 3 width 2 -- use -s 1 -c 1 and -s 3 -c 1).
 
 `diffdyn` launches the projector kernels of the differentiable-projector and dynamic-frame
 workloads twice each: batched forward and back projection of 8 images (span 11, all LORs),
 the attenuation projection, and a span-1 batched OSEM sub-iteration of 4 frames (capture
--k regex:"k_osem_batch|k_project" -c 8).
+-k regex:^k_walk -c 10).
 """
 from __future__ import annotations
 
@@ -51,7 +51,8 @@ def projectors(device='cuda:0'):
     g = get_geometry(p['txLUT'], p['axLUT'], dev)
     lib = _lib.load()
     st = stream_ptr(dev)
-    img = petprj.to_col128(torch.from_numpy(phantoms.brain_phantom(0)).to(dev)).reshape(-1)
+    # positive everywhere, as an OSEM iterate (chunks of zeros would be skipped)
+    img = petprj.to_col128(torch.from_numpy(phantoms.brain_phantom(0)).to(dev) + 0.01).reshape(-1)
     subs = torch.from_numpy(geometry.get_subsets14(3, p)[0]).to(dev)
     gen = torch.Generator(device=dev).manual_seed(0)
     an = torch.rand((68516, 837), device=dev, generator=gen) + 0.5
@@ -137,11 +138,10 @@ def sct(device='cuda:0'):
 def diffdyn(device='cuda:0'):
     """The projector launches of the differentiable-projector and dynamic-frame workloads,
     two of each, in this order: the batched forward projection of 8 images (width 4, span
-    11, all 68516 LORs; k_osem_batch forward mode), their batched back projection
-    (backward mode), the attenuation projection of the mu-map (k_project forward), and one
-    span-1 batched OSEM sub-iteration of 4 frames (width 4, subset 0).  About 5 GB on the
-    device.  Capture all eight with
-    -k regex:"k_osem_batch|k_project" -c 8 and a few metrics."""
+    11, all 68516 LORs; k_walk forward mode), their batched back projection
+    (backward mode), the attenuation projection of the mu-map (one image), and one
+    span-1 batched OSEM sub-iteration of 4 frames at widths 4 and 2 (subset 0).  About 5 GB on
+    the device.  Capture all ten with -k regex:^k_walk -c 10 and a few metrics."""
     from nipet_b200 import batch as B
     from nipet_b200 import diffprj, geometry, phantoms
     dev = torch.device(device)
@@ -149,7 +149,7 @@ def diffdyn(device='cuda:0'):
     gen = torch.Generator(device=dev).manual_seed(1)
     prj = diffprj.MMRProjector(p, mu=torch.from_numpy(phantoms.water_mumap()), span=11,
                                device=dev)
-    x = torch.rand((8, 320, 320, 127), device=dev, generator=gen)
+    x = torch.stack([torch.from_numpy(phantoms.random_ellipsoids(i)).to(dev) for i in range(8)])
     for _ in range(2):
         s = prj.project(x)
     for _ in range(2):
@@ -166,13 +166,15 @@ def diffdyn(device='cuda:0'):
                       dtype=torch.int16).view(torch.uint16)
     an = torch.rand((68516, 4084), device=dev, generator=gen) + 0.5
     rs = torch.full((68516, 4084), 0.01, device=dev)
-    br = B.BatchRecon(p, y, rs, an, device=dev, span=1, bs=4)
-    br.sens128.fill_(1.0)
-    br.init_images()
-    for _ in range(2):
-        br.subiteration(0)
-    torch.cuda.synchronize(dev)
-    br.geom.check()
+    for bs in (4, 2):
+        br = B.BatchRecon(p, y, rs, an, device=dev, span=1, bs=bs)
+        br.sens128.fill_(1.0)
+        br.init_images()
+        for _ in range(2):
+            br.subiteration(0)
+        torch.cuda.synchronize(dev)
+        br.geom.check()
+        del br
     print('diffdyn ok')
 
 
