@@ -69,7 +69,7 @@ class MMRProjector:
         self.nsng = None if nsng is None else to_device(nsng, np.float32, dev)
         if self.nsng is not None and tuple(self.nsng.shape) != (NAW, self.nsn):
             raise ValueError(f'nsng must have shape {(NAW, self.nsn)}')
-        self.launches = 0  # kernels launched (layout conversion + projector per image)
+        self.launches = 0  # kernels launched (projector, and layout conversions where made)
 
     # -- the raw projection pair (no weights) ---------------------------------------------
     def _subs_ptr(self):
@@ -102,7 +102,7 @@ class MMRProjector:
         for b in range(B):
             _lib.check(self.lib.nb_fprj(self.geom.handle, dev_ptr(out[b]), dev_ptr(x[b]),
                                         self._subs_ptr(), self.nprj, self.span, att, st))
-            self.launches += 2
+            self.launches += 1
         return out
 
     def backproject(self, s: torch.Tensor) -> torch.Tensor:
