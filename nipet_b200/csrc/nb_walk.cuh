@@ -22,10 +22,11 @@
 // streamed into shared memory with the LOR (24 KB, one bulk copy).
 //
 // Exactness.  Running integrals are int32 fixed point, one power-of-two scale per chunk of
-// CH steps and image (2^30 over a bound of the planes' integrals of |value|), so the
-// differences cancel exactly: a ray through empty planes is exactly zero whatever its
-// neighbours hold, and integer sums do not depend on the order.  The fraction terms are
-// float32 and need no cancellation.  In the back projection a ray's value is rounded once,
+// CH steps and image (2^29 over a bound of the planes' integrals of |value|, so that the
+// difference of two planes of opposite sign fits as well), so the differences cancel exactly: a
+// ray through empty planes is exactly zero whatever its neighbours hold, and integer sums do not
+// depend on the order.  A ray's own sum, with the fraction terms, is 64 bits wide: it collects
+// from one plane after another and can exceed what any of them holds.  In the back projection a ray's value is rounded once,
 // to 2^-22 of the LOR's largest, its two parts of a crossing sum to it exactly, and at most
 // 242 rays meet in a plane, so no sum leaves int32.  A chunk that holds a non-finite (or a
 // denormal-small) value is walked step by step in float32 instead, which keeps the value in
@@ -175,6 +176,13 @@ static __device__ __forceinline__ void lds_tab(uint32_t addr, int *D, int *X) {
 // byte offset of a plane in a row whose planes are `unit` bytes wide (even planes first)
 static __device__ __forceinline__ int plane_off(int P, int unit) {
   return P * (unit / 2) + (P & 1) * (127 * unit / 2);
+}
+// u + x / 2^QBITS as float32: the words one by one (exactly 0 for 0; a small negative sum is off
+// by 2^-18 at the most)
+static __device__ __forceinline__ float quanta(int u, long long x) {
+  x += (long long)u * (1 << QBITS);
+  return fmaf((float)(int)(x >> 32), (float)(1 << (32 - QBITS)),
+              (float)(uint32_t)x * (1.f / (1 << QBITS)));
 }
 static __device__ __forceinline__ float oblique_s(int d, float atn) {
   if (d == 0) return 1.f;
@@ -450,11 +458,11 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
           for (int x = 0; x < NSEG; x++) bound += bnd[x * BS + k];
           const unsigned bb = __float_as_uint(bound);
           any |= bb;
-          // bound < 2^e: scale 2^(30 - e); non-finite, above 2^100 or below 2^-60: step by step
+          // bound < 2^e: scale 2^(29 - e); non-finite, above 2^100 or below 2^-60: step by step
           const int e = (int)(bb >> 23) - 126;
           slow |= bb >= 0x71800000u || (bb != 0u && bb < 0x21800000u);
-          scale[k] = bb ? __uint_as_float((uint32_t)(min(max(30 - e, -126), 127) + 127) << 23) : 0.f;
-          inv[k] = __uint_as_float((uint32_t)(min(max(e - 30, -126), 127) + 127) << 23);
+          scale[k] = bb ? __uint_as_float((uint32_t)(min(max(29 - e, -126), 127) + 127) << 23) : 0.f;
+          inv[k] = __uint_as_float((uint32_t)(min(max(e - 29, -126), 127) + 127) << 23);
         }
         // cleared two chunks before its next use: its last readers are one barrier back
         if (tid < NSEG * BS) smax[((mrot + 2) % 3) * NSEG * BS + tid] = 0u;
@@ -575,36 +583,36 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
           uint32_t cA0 = base + plane_off(zA + 1, UNIT), cB0 = base + plane_off(zB, UNIT);
           uint32_t cA1 = cA0 + 64 * UNIT - ((zA + 1) & 1) * (127 * UNIT);
           uint32_t cB1 = cB0 + 63 * UNIT - (zB & 1) * (127 * UNIT);
-          // sums of D and of dD * fraction (64 bits: 2^30 by 2^31, up to ~100 of them)
-          int iA[BS], iB[BS];
+          // sums of D + dD * fraction in 2^-QBITS quanta, 64 bits: a ray that changes planes can
+          // collect more than any plane holds, up to SEGL times 2^29.  Two crossings' D fit 32
+          // (the plane between them cancels but for what the ray collects in it: 3 x 2^29)
           long long xA[BS], xB[BS];
+          int dA[BS], dB[BS];
 #pragma unroll
-          for (int k = 0; k < BS; k++) {
-            iA[k] = iB[k] = 0;
-            xA[k] = xB[k] = 0;
-          }
+          for (int k = 0; k < BS; k++) xA[k] = xB[k] = 0;
           auto cross = [&](int f, uint32_t rA, uint32_t rB) {
-            int D[BS], X[BS];
-            lds_tab<BS>(rA, D, X);
+            int X[BS];
+            lds_tab<BS>(rA, dA, X);
 #pragma unroll
-            for (int k = 0; k < BS; k++) {
-              iA[k] += D[k];
-              xA[k] += (long long)X[k] * f;
-            }
-            lds_tab<BS>(rB, D, X);
+            for (int k = 0; k < BS; k++) xA[k] += (long long)X[k] * f;
+            lds_tab<BS>(rB, dB, X);
 #pragma unroll
-            for (int k = 0; k < BS; k++) {
-              iB[k] += D[k];
-              xB[k] += (long long)X[k] * f;
-            }
+            for (int k = 0; k < BS; k++) xB[k] += (long long)X[k] * f;
           };
           for (; cnt >= 2; cnt -= 2) {
-            int i0, i1, f0, f1;
+            int i0, i1, f0, f1, eA[BS], eB[BS];
             lds_ent(ep, i0, f0);
             lds_ent(ep + 8, i1, f1);
             ep += 16;
             cross(f0, cA0 + (i0 << LOGR), cB0 + (i0 << LOGR));
+#pragma unroll
+            for (int k = 0; k < BS; k++) eA[k] = dA[k], eB[k] = dB[k];
             cross(f1, cA1 + (i1 << LOGR), cB1 + (i1 << LOGR));
+#pragma unroll
+            for (int k = 0; k < BS; k++) {
+              xA[k] += (long long)(eA[k] + dA[k]) * (1 << QBITS);
+              xB[k] += (long long)(eB[k] + dB[k]) * (1 << QBITS);
+            }
             cA0 += UNIT;
             cA1 += UNIT;
             cB0 -= UNIT;
@@ -614,6 +622,11 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
             int i0, f0;
             lds_ent(ep, i0, f0);
             cross(f0, cA0 + (i0 << LOGR), cB0 + (i0 << LOGR));
+#pragma unroll
+            for (int k = 0; k < BS; k++) {
+              xA[k] += (long long)dA[k] * (1 << QBITS);
+              xB[k] += (long long)dB[k] * (1 << QBITS);
+            }
           }
           // the down-going ray leaves C[P] for C[P-1]: its differences count negative
           int u[BS], w[BS];
@@ -621,8 +634,8 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
           ldi<BS>(srun + nb_zi(endB) * BS, w);
 #pragma unroll
           for (int k = 0; k < BS; k++) {
-            FA[j][k] = fmaf((float)(u[k] + iA[k] + (int)(xA[k] >> QBITS)), inv[k], FA[j][k]);
-            FB[j][k] = fmaf((float)(w[k] - iB[k] - (int)(xB[k] >> QBITS)), inv[k], FB[j][k]);
+            FA[j][k] = fmaf(quanta(u[k], xA[k]), inv[k], FA[j][k]);
+            FB[j][k] = fmaf(quanta(w[k], -xB[k]), inv[k], FB[j][k]);
           }
         }
       }
