@@ -187,10 +187,7 @@ int nb_osem_subset_psf(nb_geom *g, float *img128, float *bimg128, const float *s
  *   psng       dev [nrep][68516][nsinos] uint16 prompts; rs dev [68516][nsinos] float
  *              (r+s)/(an) from nb_osem_rs; rscale dev [nrep] per-image randoms factor
  *   bs         1, 2 or 4; span 11 (837 sinograms) or 1 (4084)
- *   tile       kernel shape: 0 = 1024 threads x 4 rays each, 64/bs columns of the LOR
- *              staged per shared-memory chunk; 1 = the same threads, 32/bs columns per
- *              chunk; 2 = 512 threads x 8 rays, 64/bs columns.  Results agree to rounding;
- *              batch.autotune picks (bs, tile) by timing them.
+ *   tile       0, 1 or 2: accepted and without effect, since each width has one kernel shape
  * nb_to_batch / nb_from_batch convert nrep reference-layout images [nrep][320][320][127]
  * to and from that layout; nb_fill_batch sets every voxel of the nrep images in that layout
  * to `value` (the OSEM start image) without a reference-layout source, zeroing the padding

@@ -6,9 +6,8 @@ per-subset sensitivity images; each has its own prompts and a randoms level
 fused kernel launch (`nb_osem_batch_subset`) -- two when the images left over by the
 batch width go through a narrower launch of their own (`split_parts`) -- and a full
 iteration (14 sub-iterations) can be captured once as a CUDA graph and replayed.  The
-batch width `bs` (images sharing one walk of the Siddon geometry) and the kernel's tile
-shape (columns of the LOR staged per shared-memory chunk, rays per thread) are chosen by
-`autotune`, which times the candidates on the device and caches the choice per device.
+batch width `bs` (images sharing one walk of the Siddon geometry) is chosen by `autotune`,
+which times the candidates on the device and caches the choice per device.
 """
 from __future__ import annotations
 
@@ -218,14 +217,15 @@ def _cache_file():
     return os.path.join(d, 'autotune.json')
 
 
+# accepted by `nb_osem_batch_subset`; every width has one kernel shape
 TILES = (0, 1, 2)
 
 
 def autotune(rec: BatchRecon, candidates=None, repeats: int = 2):
-    """Pick the batch width (images per Siddon walk) and tile shape (see
-    `nb_osem_batch_subset`) with the best images/s for this device, span and batch size,
-    timing `repeats` sub-iterations per candidate after one warm-up.  Returns (bs, tile);
-    results are cached in memory and in `~/.cache/nipet_b200/autotune.json`."""
+    """Pick the batch width (images per Siddon walk) with the best images/s for this device,
+    span and batch size, timing `repeats` sub-iterations per candidate (bs, tile) after one
+    warm-up.  Returns (bs, tile); results are cached in memory and in
+    `~/.cache/nipet_b200/autotune.json`."""
     name = torch.cuda.get_device_name(rec.device)
     # (the kernel's name: choices stored for another kernel say nothing about this one)
     key = f'{name}|k_walk|span{rec.span}|n{rec.nrep}'
@@ -244,8 +244,7 @@ def autotune(rec: BatchRecon, candidates=None, repeats: int = 2):
     if candidates is None:
         widths = [1, 2, 4]
         widths = [w for w in widths if w <= max(1, rec.nrep) or w == 1]
-        # one image per walk has one kernel shape
-        candidates = [(w, t) for w in widths for t in (TILES if w > 1 else TILES[:1])]
+        candidates = [(w, 0) for w in widths]
     best, best_t = candidates[0], float('inf')
     rec.sens128.fill_(1.0)
     for bs, tile in candidates:

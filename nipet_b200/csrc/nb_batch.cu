@@ -142,6 +142,7 @@ extern "C" int nb_osem_batch_subset(nb_geom *g, float *img, float *bimg, const f
   NB_REQUIRE(nrep > 0 && nrep <= NB_MAXREP, "nb_osem_batch_subset: nrep out of range");
   NB_REQUIRE(span == 11 || span == 1, "nb_osem_batch_subset: span must be 1 or 11");
   NB_REQUIRE(bs == 1 || bs == 2 || bs == 4, "nb_osem_batch_subset: bs must be 1, 2 or 4");
+  // (each width has one kernel shape: the tile is checked and has no effect)
   NB_REQUIRE(tile >= 0 && tile <= 2, "nb_osem_batch_subset: tile must be 0, 1 or 2");
   NB_REQUIRE(nprj > 0, "nb_osem_batch_subset: empty subset");
   NB_CUDA(cudaSetDevice(g->device));
@@ -153,7 +154,7 @@ extern "C" int nb_osem_batch_subset(nb_geom *g, float *img, float *bimg, const f
   a.psng = psng;
   a.rs = rs;
   a.rscale = rscale;
-  const int st = nb_walk_launch(g, a, nbw::MODE_OSEM, bs, tile, s);
+  const int st = nb_walk_launch(g, a, nbw::MODE_OSEM, bs, s);
   if (st) return st;
   const dim3 ugrid(g->nsm * 4, ngroups < 16 ? ngroups : 16);
   if (bs == 4)
@@ -200,7 +201,7 @@ extern "C" int nb_osem_subset_span1(nb_geom *g, float *img128, float *bimg128,
     a.bimg = bimg128;
     a.psng = psng;
     a.rs = rs;
-    st = nb_walk_launch(g, a, nbw::MODE_OSEM, 1, 0, s);
+    st = nb_walk_launch(g, a, nbw::MODE_OSEM, 1, s);
     if (!st && krnl) st = nb_psf_col128(rm, bimg128, krnl, tmp, stream);
     if (!st) {
       k_update_batch<1><<<dim3(g->nsm * 4, 1), 256, 0, s>>>(img128, krnl ? rm : bimg128,
@@ -225,7 +226,7 @@ extern "C" int nb_fprj_batch(nb_geom *g, float *sino, const float *img, int nrep
   nbw::WalkArgs a = nb_walk_args(g, subs, nprj, span, nrep, bs);
   a.img = img;
   a.sino = sino;
-  return nb_walk_launch(g, a, nbw::MODE_FWD, bs, 0, (cudaStream_t)stream);
+  return nb_walk_launch(g, a, nbw::MODE_FWD, bs, (cudaStream_t)stream);
 }
 
 extern "C" int nb_bprj_batch(nb_geom *g, float *bimg, const float *sino, int nrep, int bs,
@@ -241,5 +242,5 @@ extern "C" int nb_bprj_batch(nb_geom *g, float *bimg, const float *sino, int nre
   nbw::WalkArgs a = nb_walk_args(g, subs, nprj, span, nrep, bs);
   a.bimg = bimg;
   a.sino_in = sino;
-  return nb_walk_launch(g, a, nbw::MODE_BWD, bs, 0, (cudaStream_t)stream);
+  return nb_walk_launch(g, a, nbw::MODE_BWD, bs, (cudaStream_t)stream);
 }

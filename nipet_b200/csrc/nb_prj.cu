@@ -207,7 +207,7 @@ extern "C" int nb_fprj_col128(nb_geom *g, float *sino, const float *im128, const
   a.att = att;
   a.img = im128;
   a.sino = sino;
-  return nb_walk_launch(g, a, nbw::MODE_FWD, 1, 0, (cudaStream_t)stream);
+  return nb_walk_launch(g, a, nbw::MODE_FWD, 1, (cudaStream_t)stream);
 }
 
 extern "C" int nb_bprj_col128(nb_geom *g, float *im128, const float *sino, const int32_t *subs,
@@ -219,7 +219,7 @@ extern "C" int nb_bprj_col128(nb_geom *g, float *im128, const float *sino, const
   nbw::WalkArgs a = nb_walk_args(g, subs, nprj, span, 1, 1);
   a.bimg = im128;
   a.sino_in = sino;
-  return nb_walk_launch(g, a, nbw::MODE_BWD, 1, 0, (cudaStream_t)stream);
+  return nb_walk_launch(g, a, nbw::MODE_BWD, 1, (cudaStream_t)stream);
 }
 
 extern "C" int nb_sens_col128(nb_geom *g, float *sens128, const float *an, const int32_t *subs,
@@ -233,7 +233,7 @@ extern "C" int nb_sens_col128(nb_geom *g, float *sens128, const float *an, const
   a.bimg = sens128;
   a.sino_in = an;
   a.in_by_lor = 1;
-  return nb_walk_launch(g, a, nbw::MODE_BWD, 1, 0, (cudaStream_t)stream);
+  return nb_walk_launch(g, a, nbw::MODE_BWD, 1, (cudaStream_t)stream);
 }
 
 extern "C" int nb_fprj(nb_geom *g, float *sino, const float *im, const int32_t *subs, int nprj,
@@ -251,7 +251,7 @@ extern "C" int nb_fprj(nb_geom *g, float *sino, const float *im, const int32_t *
   a.img = im;
   a.natural = 1;
   a.sino = sino;
-  return nb_walk_launch(g, a, nbw::MODE_FWD, 1, 0, (cudaStream_t)stream);
+  return nb_walk_launch(g, a, nbw::MODE_FWD, 1, (cudaStream_t)stream);
 }
 
 extern "C" int nb_bprj(nb_geom *g, float *im, const float *sino, const int32_t *subs, int nprj,
@@ -299,7 +299,7 @@ extern "C" int nb_fprj_rings(nb_geom *g, const nb_rings *rr, float *sino, const 
   a.att = att;
   a.img = g->d_scratch128;
   a.sino = sino;
-  return nb_walk_launch(g, a, nbw::MODE_FWD, 1, 0, s);
+  return nb_walk_launch(g, a, nbw::MODE_FWD, 1, s);
 }
 
 extern "C" int nb_bprj_rings(nb_geom *g, const nb_rings *rr, float *im, const float *sino,
@@ -318,7 +318,7 @@ extern "C" int nb_bprj_rings(nb_geom *g, const nb_rings *rr, float *im, const fl
   a.nout = rr->nrays;
   a.bimg = g->d_scratch128;
   a.sino_in = sino;
-  st = nb_walk_launch(g, a, nbw::MODE_BWD, 1, 0, s);
+  st = nb_walk_launch(g, a, nbw::MODE_BWD, 1, s);
   if (st) return st;
   k_col128_to_slab<<<(NB_NCOL * 32 + 255) / 256, 256, 0, s>>>(im, g->d_scratch128, rr->nvz,
                                                                rr->vz0);
@@ -350,7 +350,7 @@ extern "C" int nb_osem_subset(nb_geom *g, float *img128, float *bimg128, const f
   a.bimg = bimg128;
   a.psng = psng;
   a.rs = rs;
-  st = nb_walk_launch(g, a, nbw::MODE_OSEM, 1, 0, s);
+  st = nb_walk_launch(g, a, nbw::MODE_OSEM, 1, s);
   if (st) return st;
   const size_t n4 = NB_IMG_COL128 / 4;
   k_osem_update<<<g->nsm * 8, 256, 0, s>>>((float4 *)img128, (float4 *)bimg128,
@@ -385,7 +385,7 @@ extern "C" int nb_osem_subset_psf(nb_geom *g, float *img128, float *bimg128,
   a.bimg = bimg128;
   a.psng = psng;
   a.rs = rs;
-  st = nb_walk_launch(g, a, nbw::MODE_OSEM, 1, 0, s);
+  st = nb_walk_launch(g, a, nbw::MODE_OSEM, 1, s);
   if (st) return st;
   st = nb_psf_col128(rm, bimg128, krnl, tmp, stream);  // rm: the convolved back projection
   if (st) return st;

@@ -5,12 +5,12 @@
 
 namespace {
 
-template <int BS, int VB, int CH, int NT, int MODE, int MINB>
+template <int BS, int CH, int NT, int MODE, int MINB>
 int launch(nb_geom *g, const nbw::WalkArgs &a, cudaStream_t s) {
-  constexpr int NSEG = NT * VB / (64 * BS);
+  constexpr int NSEG = NT / 64;
   constexpr size_t smem = nbw::WSmem<BS, CH, NSEG>::total;
   static_assert(smem * MINB + 1024 * MINB <= 228 * 1024, "too much shared memory per SM");
-  auto *k = nbw::k_walk<BS, VB, CH, NT, MODE, MINB>;
+  auto *k = nbw::k_walk<BS, CH, NT, MODE, MINB>;
   // the shared-memory opt-in is set once per device and kernel shape; host threads may
   // launch concurrently, so the flags are atomics (setting the attribute twice is harmless)
   static std::atomic<bool> set[64];
@@ -26,10 +26,10 @@ int launch(nb_geom *g, const nbw::WalkArgs &a, cudaStream_t s) {
   return NB_OK;
 }
 
-// Kernel shapes <BS, images per thread of the running sums, steps per chunk, threads, mode,
-// blocks per SM>.  One image: two blocks of 512 threads at 64 registers.  Two and four images
-// need the registers: 16 warps of 128 registers an SM beat 32 of 64, which spill (us per image
-// and 4894 LORs, dense image: fused sub-iteration / forward / back):
+// Kernel shapes <BS, steps per chunk, threads, mode, blocks per SM>, one per width.  One image:
+// two blocks of 512 threads at 64 registers.  Two and four images need the registers: 16 warps
+// of 128 registers an SM beat 32 of 64, which spill (us per image and 4894 LORs, dense image:
+// fused sub-iteration / forward / back):
 //   one image     64 steps, 2 x 512 threads  1486 / 701 / 764
 //                 64 steps, 2 x 256 threads  1653 / 754 / 825
 //                 32 steps, 2 x 512 threads  1681 / 797 / 803
@@ -41,29 +41,21 @@ int launch(nb_geom *g, const nbw::WalkArgs &a, cudaStream_t s) {
 //                 24 steps, 1 x 384 threads  1414 / 780 / 681
 //                 32 steps, 1 x 256 threads  1460 / 754 / 694
 //                 32 steps, 1 x 1024 threads 1727 / 942 / 735
+// The order holds for fused sub-iterations of 600 LORs and of 2 to 8 images, at both spans; at 33
+// LORs the two-image shape of 512 threads is the faster one (300 against 349 us), but no subset
+// is that small.
 template <int MODE> int launch_prj(nb_geom *g, const nbw::WalkArgs &a, int bs, cudaStream_t s) {
-  if (bs == 4) return launch<4, 4, 32, 512, MODE, 1>(g, a, s);
-  if (bs == 2) return launch<2, 2, 32, 256, MODE, 2>(g, a, s);
-  return launch<1, 1, 64, 512, MODE, 2>(g, a, s);
+  if (bs == 4) return launch<4, 32, 512, MODE, 1>(g, a, s);
+  if (bs == 2) return launch<2, 32, 256, MODE, 2>(g, a, s);
+  return launch<1, 64, 512, MODE, 2>(g, a, s);
 }
 
 }  // namespace
 
-int nb_walk_launch(nb_geom *g, const nbw::WalkArgs &a, int mode, int bs, int tile,
-                   cudaStream_t s) {
+int nb_walk_launch(nb_geom *g, const nbw::WalkArgs &a, int mode, int bs, cudaStream_t s) {
   if (mode == nbw::MODE_FWD) return launch_prj<nbw::MODE_FWD>(g, a, bs, s);
   if (mode == nbw::MODE_BWD) return launch_prj<nbw::MODE_BWD>(g, a, bs, s);
-  // the fused mode's tile picks among the best shapes (batch.autotune); one image has one
-  constexpr int M = nbw::MODE_OSEM;
-  if (bs == 4)
-    return tile == 0   ? launch<4, 4, 32, 512, M, 1>(g, a, s)
-           : tile == 1 ? launch<4, 4, 24, 384, M, 1>(g, a, s)
-                       : launch<4, 4, 32, 256, M, 1>(g, a, s);
-  if (bs == 2)
-    return tile == 0   ? launch<2, 2, 32, 256, M, 2>(g, a, s)
-           : tile == 1 ? launch<2, 2, 24, 256, M, 2>(g, a, s)
-                       : launch<2, 2, 64, 512, M, 1>(g, a, s);
-  return launch<1, 1, 64, 512, M, 2>(g, a, s);
+  return launch_prj<nbw::MODE_OSEM>(g, a, bs, s);
 }
 
 nbw::WalkArgs nb_walk_args(const nb_geom *g, const int32_t *subs, int nprj, int span, int nrep,

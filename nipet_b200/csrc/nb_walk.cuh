@@ -218,9 +218,9 @@ static __device__ __noinline__ void slow_ray(const float *gimg, const int32_t *c
   }
 }
 
-template <int BS, int VB, int CH, int NT, int MODE, int MINB>
+template <int BS, int CH, int NT, int MODE, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
-  constexpr int NSEG = NT * VB / (64 * BS);   // step segments of a chunk, one per 64 threads
+  constexpr int NSEG = NT / 64;               // step segments of a chunk, one per 64 threads
   constexpr int SEGL = CH / NSEG;
   constexpr int SPT = (NB_NSLOT + NT - 1) / NT;          // slots (ray pairs) per thread
   constexpr int W = NT / 32;
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int s = tid & 63;                     // scan: this thread's planes 2 s and 2 s + 1
-  const int seg = (tid >> 6) % NSEG, iv = ((tid >> 6) / NSEG) * VB;
+  const int seg = tid >> 6;                   // ... in this segment
   const uint32_t tab_u = nb_smem_u32(tab), rec_u = nb_smem_u32(rec);
   const bool span11 = a.span == 11;
 
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
 
     // ------------------------------------------------------------------ forward
     if (MODE != MODE_BWD) {
-      float E[SEGL][VB], O[SEGL][VB];         // this thread's values: planes 2 s, 2 s + 1
+      float E[SEGL][BS], O[SEGL][BS];         // this thread's values: planes 2 s, 2 s + 1
       const bool natural = MODE == MODE_FWD && BS == 1 && a.natural != 0;
       auto load = [&](int c) {
         int col[SEGL];
@@ -406,15 +406,15 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
         for (int j = 0; j < SEGL; j++) {
           if (f0 + j < n) {
             const float *x = gimg + (size_t)col[j] * (natural ? NB_IMZ : NB_COLW * BS) +
-                             (natural ? 2 * s : s * BS + iv);
-            ldg_v<VB>(x, E[j]);
+                             (natural ? 2 * s : s * BS);
+            ldg_v<BS>(x, E[j]);
             if (natural && s == 63)
               O[j][0] = 0.f;
             else
-              ldg_v<VB>(x + (natural ? 1 : 64 * BS), O[j]);
+              ldg_v<BS>(x + (natural ? 1 : 64 * BS), O[j]);
           } else {
 #pragma unroll
-            for (int v = 0; v < VB; v++) E[j][v] = O[j][v] = 0.f;
+            for (int v = 0; v < BS; v++) E[j][v] = O[j][v] = 0.f;
           }
         }
       };
@@ -428,11 +428,11 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
         float lt[SEGL];
         {
           step_lengths(s0, lt);
-          float m[VB];
+          float m[BS];
 #pragma unroll
-          for (int v = 0; v < VB; v++) m[v] = 0.f;
+          for (int v = 0; v < BS; v++) m[v] = 0.f;
 #pragma unroll
-          for (int v = 0; v < VB; v++) {
+          for (int v = 0; v < BS; v++) {
             float me = 0.f, mo = 0.f;
 #pragma unroll
             for (int j = 0; j < SEGL; j++) {
@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
               mo = fmaf(lt[j], fabsf(O[j][v]), mo);
             }
             const unsigned u = __reduce_max_sync(0xffffffffu, max(__float_as_uint(me), __float_as_uint(mo)));
-            if (lane == 0 && u) atomicMax(&smax[(mrot * NSEG + seg) * BS + iv + v], u);
+            if (lane == 0 && u) atomicMax(&smax[(mrot * NSEG + seg) * BS + v], u);
           }
         }
         __syncthreads();
@@ -470,73 +470,72 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
         if (any == 0u) continue;              // nothing but zeros
         if (!slow) {
           // fixed-point running integrals: within the segment, then the segments before it
-          int cE[SEGL][VB], cO[SEGL][VB], tE[VB], tO[VB];
-          float sv[VB];
+          int cE[SEGL][BS], cO[SEGL][BS], tE[BS], tO[BS];
+          float sv[BS];
 #pragma unroll
-          for (int v = 0; v < VB; v++) {
+          for (int v = 0; v < BS; v++) {
             tE[v] = tO[v] = 0;
             sv[v] = scale[v];
-            if (VB < BS && iv) sv[v] = scale[(VB + v) % BS];
           }
 #pragma unroll
           for (int j = 0; j < SEGL; j++) {
 #pragma unroll
-            for (int v = 0; v < VB; v++) {
+            for (int v = 0; v < BS; v++) {
               const float w = lt[j] * sv[v];
               cE[j][v] = tE[v];
               cO[j][v] = tO[v];
               tE[v] += __float2int_rn(E[j][v] * w);
               tO[v] += __float2int_rn(O[j][v] * w);
             }
-            if (s == 31) sti<VB>(soc + (seg * (SEGL + 1) + j) * BS + iv, cO[j]);
+            if (s == 31) sti<BS>(soc + (seg * (SEGL + 1) + j) * BS, cO[j]);
           }
-          if (s == 31) sti<VB>(soc + (seg * (SEGL + 1) + SEGL) * BS + iv, tO);
-          sti<VB>(sseg + (seg * 128 + s) * BS + iv, tE);
-          sti<VB>(sseg + (seg * 128 + 64 + s) * BS + iv, tO);
+          if (s == 31) sti<BS>(soc + (seg * (SEGL + 1) + SEGL) * BS, tO);
+          sti<BS>(sseg + (seg * 128 + s) * BS, tE);
+          sti<BS>(sseg + (seg * 128 + 64 + s) * BS, tO);
           __syncthreads();
-          int bE[VB], bO[VB];
+          int bE[BS], bO[BS];
 #pragma unroll
-          for (int v = 0; v < VB; v++) bE[v] = bO[v] = 0;
+          for (int v = 0; v < BS; v++) bE[v] = bO[v] = 0;
           for (int x = 0; x < seg; x++) {
-            int u[VB], w[VB];
-            ldi<VB>(sseg + (x * 128 + s) * BS + iv, u);
-            ldi<VB>(sseg + (x * 128 + 64 + s) * BS + iv, w);
+            int u[BS], w[BS];
+            ldi<BS>(sseg + (x * 128 + s) * BS, u);
+            ldi<BS>(sseg + (x * 128 + 64 + s) * BS, w);
 #pragma unroll
-            for (int v = 0; v < VB; v++) bE[v] += u[v], bO[v] += w[v];
+            for (int v = 0; v < BS; v++) bE[v] += u[v], bO[v] += w[v];
           }
           // the thread of plane 64 gets plane 63's prefixes through shared memory (its neighbour
           // is another warp's); the thread of plane 0 has no plane below and its D[0] no reader
           const bool fix = s == 32;
-          int bP[VB];
+          int bP[BS];
 #pragma unroll
-          for (int v = 0; v < VB; v++) bP[v] = 0;
+          for (int v = 0; v < BS; v++) bP[v] = 0;
           if (fix)
             for (int x = 0; x < seg; x++) {
-              int u[VB];
-              ldi<VB>(sseg + (x * 128 + 64 + 31) * BS + iv, u);
+              int u[BS];
+              ldi<BS>(sseg + (x * 128 + 64 + 31) * BS, u);
 #pragma unroll
-              for (int v = 0; v < VB; v++) bP[v] += u[v];
+              for (int v = 0; v < BS; v++) bP[v] += u[v];
             }
           if (seg == NSEG - 1) {              // the chunk's whole integral per plane
-            int u[VB], w[VB];
+            int u[BS], w[BS];
 #pragma unroll
-            for (int v = 0; v < VB; v++) u[v] = tE[v] + bE[v], w[v] = tO[v] + bO[v];
-            sti<VB>(srun + s * BS + iv, u);
-            sti<VB>(srun + (64 + s) * BS + iv, w);
+            for (int v = 0; v < BS; v++) u[v] = tE[v] + bE[v], w[v] = tO[v] + bO[v];
+            sti<BS>(srun + s * BS, u);
+            sti<BS>(srun + (64 + s) * BS, w);
           }
           // D at the start of each step and its change over the step
-          int De[VB], Do[VB];
+          int De[BS], Do[BS];
 #pragma unroll
           for (int j = SEGL; j >= 0; j--) {
-            int ne[VB], no[VB];               // D at the end of step j
+            int ne[BS], no[BS];               // D at the end of step j
 #pragma unroll
-            for (int v = 0; v < VB; v++) {
+            for (int v = 0; v < BS; v++) {
               ne[v] = De[v];
               no[v] = Do[v];
               const int ce = (j < SEGL ? cE[j < SEGL ? j : 0][v] : tE[v]) + bE[v];
               const int co = (j < SEGL ? cO[j < SEGL ? j : 0][v] : tO[v]) + bO[v];
               int cp = __shfl_up_sync(0xffffffffu, co, 1);      // plane 2 s - 1
-              if (fix) cp = bP[v] + soc[(seg * (SEGL + 1) + j) * BS + iv + v];
+              if (fix) cp = bP[v] + soc[(seg * (SEGL + 1) + j) * BS + v];
               De[v] = cp - ce;
               Do[v] = ce - co;
               ne[v] -= De[v];
@@ -547,14 +546,14 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
             if (BS == 1) {
               *reinterpret_cast<int2 *>(r) = make_int2(De[0], ne[0]);
               *reinterpret_cast<int2 *>(r + 64 * UNIT) = make_int2(Do[0], no[0]);
-            } else if (BS == 2 && VB == 2) {
-              *reinterpret_cast<int4 *>(r) = make_int4(De[0], De[VB - 1], ne[0], ne[VB - 1]);
-              *reinterpret_cast<int4 *>(r + 64 * UNIT) = make_int4(Do[0], Do[VB - 1], no[0], no[VB - 1]);
+            } else if (BS == 2) {
+              *reinterpret_cast<int4 *>(r) = make_int4(De[0], De[BS - 1], ne[0], ne[BS - 1]);
+              *reinterpret_cast<int4 *>(r + 64 * UNIT) = make_int4(Do[0], Do[BS - 1], no[0], no[BS - 1]);
             } else {
-              sti<VB>(reinterpret_cast<int *>(r) + iv, De);
-              sti<VB>(reinterpret_cast<int *>(r + 64 * UNIT) + iv, Do);
-              sti<VB>(reinterpret_cast<int *>(r + 2048) + iv, ne);
-              sti<VB>(reinterpret_cast<int *>(r + 2048 + 64 * UNIT) + iv, no);
+              sti<BS>(reinterpret_cast<int *>(r), De);
+              sti<BS>(reinterpret_cast<int *>(r + 64 * UNIT), Do);
+              sti<BS>(reinterpret_cast<int *>(r + 2048), ne);
+              sti<BS>(reinterpret_cast<int *>(r + 2048 + 64 * UNIT), no);
             }
           }
           __syncthreads();
@@ -849,10 +848,10 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
         const bool last = c == nch - 1;
         if (last && tid == 0) next_job(job);
         // flows -> running sums: this thread's planes z = 2 s and 2 s + 1, SEGL steps
-        int rE[SEGL][VB], rO[SEGL][VB], cy[2][VB];
-        int *g0 = gacc + (seg * SEGL * BS + iv) * 128 + s;
+        int rE[SEGL][BS], rO[SEGL][BS], cy[2][BS];
+        int *g0 = gacc + seg * SEGL * BS * 128 + s;
 #pragma unroll
-        for (int v = 0; v < VB; v++) {
+        for (int v = 0; v < BS; v++) {
           int tE = 0, tO = 0, lp[SEGL];
           if (s == 31)                        // its neighbour above is another warp's
 #pragma unroll
@@ -870,8 +869,8 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
             rE[j][v] = tE;
             rO[j][v] = tO;
           }
-          sseg[(seg * 128 + s) * BS + iv + v] = tE;
-          sseg[(seg * 128 + 64 + s) * BS + iv + v] = tO;
+          sseg[(seg * 128 + s) * BS + v] = tE;
+          sseg[(seg * 128 + 64 + s) * BS + v] = tO;
           if (seg == 0) {                     // the row that spills into the next chunk
             cy[0][v] = g0[(CH * BS + v) * 128];
             cy[1][v] = g0[(CH * BS + v) * 128 + 64];
@@ -882,50 +881,49 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
         __syncthreads();
         const int *run0 = srun + (c & 1) * 128 * BS;
         int *run1 = srun + ((c & 1) ^ 1) * 128 * BS;
-        int bE[VB], bO[VB];
-        ldi<VB>(run0 + s * BS + iv, bE);
-        ldi<VB>(run0 + (64 + s) * BS + iv, bO);
+        int bE[BS], bO[BS];
+        ldi<BS>(run0 + s * BS, bE);
+        ldi<BS>(run0 + (64 + s) * BS, bO);
         for (int x = 0; x < seg; x++) {
-          int u[VB], w[VB];
-          ldi<VB>(sseg + (x * 128 + s) * BS + iv, u);
-          ldi<VB>(sseg + (x * 128 + 64 + s) * BS + iv, w);
+          int u[BS], w[BS];
+          ldi<BS>(sseg + (x * 128 + s) * BS, u);
+          ldi<BS>(sseg + (x * 128 + 64 + s) * BS, w);
 #pragma unroll
-          for (int v = 0; v < VB; v++) bE[v] += u[v], bO[v] += w[v];
+          for (int v = 0; v < BS; v++) bE[v] += u[v], bO[v] += w[v];
         }
         if (seg == NSEG - 1) {
-          int u[VB], w[VB];
+          int u[BS], w[BS];
 #pragma unroll
-          for (int v = 0; v < VB; v++) {
+          for (int v = 0; v < BS; v++) {
             u[v] = bE[v] + rE[SEGL - 1][v];
             w[v] = bO[v] + rO[SEGL - 1][v];
           }
-          sti<VB>(run1 + s * BS + iv, u);
-          sti<VB>(run1 + (64 + s) * BS + iv, w);
+          sti<BS>(run1 + s * BS, u);
+          sti<BS>(run1 + (64 + s) * BS, w);
         }
-        float ie[VB], io[VB];                 // plane 127 is padding: nothing goes back to it
+        float ie[BS], io[BS];                 // plane 127 is padding: nothing goes back to it
 #pragma unroll
-        for (int v = 0; v < VB; v++) {
+        for (int v = 0; v < BS; v++) {
           ie[v] = inv[v];
-          if (VB < BS && iv) ie[v] = inv[(VB + v) % BS];
           io[v] = s == 63 ? 0.f : ie[v];
         }
-        float *o0 = stage + (seg * SEGL * 128 + s) * BS + iv;
+        float *o0 = stage + (seg * SEGL * 128 + s) * BS;
 #pragma unroll
         for (int j = 0; j < SEGL; j++) {
-          int oe[VB], oo[VB];
+          int oe[BS], oo[BS];
 #pragma unroll
-          for (int v = 0; v < VB; v++) {
+          for (int v = 0; v < BS; v++) {
             oe[v] = __float_as_int((float)(bE[v] + rE[j][v]) * (lt[j] * ie[v]));
             oo[v] = __float_as_int((float)(bO[v] + rO[j][v]) * (lt[j] * io[v]));
             g0[(j * BS + v) * 128] = 0;
             g0[(j * BS + v) * 128 + 64] = 0;
           }
-          sti<VB>(reinterpret_cast<int *>(o0) + j * 128 * BS, oe);
-          sti<VB>(reinterpret_cast<int *>(o0) + j * 128 * BS + 64 * BS, oo);
+          sti<BS>(reinterpret_cast<int *>(o0) + j * 128 * BS, oe);
+          sti<BS>(reinterpret_cast<int *>(o0) + j * 128 * BS + 64 * BS, oo);
         }
         if (seg == 0) {
 #pragma unroll
-          for (int v = 0; v < VB; v++) {
+          for (int v = 0; v < BS; v++) {
             g0[v * 128] = last ? 0 : cy[0][v];
             g0[v * 128 + 64] = last ? 0 : cy[1][v];
             g0[(CH * BS + v) * 128] = 0;
@@ -952,8 +950,7 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
 }  // namespace nbw
 
 // nb_walk.cu: the geometry's arguments for `nrep` images, `bs` to a walk; and the launch of one
-// mode (tile: kernel shape of the fused sub-iteration, 0 .. 2)
+// mode
 nbw::WalkArgs nb_walk_args(const nb_geom *g, const int32_t *subs, int nprj, int span, int nrep,
                            int bs);
-int nb_walk_launch(nb_geom *g, const nbw::WalkArgs &a, int mode, int bs, int tile,
-                   cudaStream_t s);
+int nb_walk_launch(nb_geom *g, const nbw::WalkArgs &a, int mode, int bs, cudaStream_t s);

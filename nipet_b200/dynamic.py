@@ -89,8 +89,8 @@ class DynamicRecon:
     """Batched span-1 OSEM of all frames of a `dynamic_scan`, then per-frame Poisson
     log-likelihood gradients through `diffprj.MMRProjector`.
 
-    bs (frames per walk of the geometry: 1, 2 or 4) and the kernel tile are picked
-    by the batch autotuner when None."""
+    bs (frames per walk of the geometry: 1, 2 or 4) is picked by the batch autotuner when
+    None; every tile (0, 1, 2) names the same kernel shape."""
 
     def __init__(self, params: dict, scan: dict, device=None, bs: int | None = None,
                  nsub: int = 14, tile: int | None = None):

@@ -59,6 +59,8 @@ def test_batch_cuda_graph_replay(params, scan, replicates, cuda_device):
 
 @pytest.mark.parametrize('bs,tile', [(4, 1), (4, 2), (2, 1), (2, 2), (1, 1), (1, 2)])
 def test_tile_shapes_agree(params, scan, replicates, cuda_device, bs, tile):
+    """Every accepted tile gives the default's images (a width has one kernel shape; the fused
+    kernel's own edges are checked in test_gpu_walk.py)."""
     an = scan['asng'] * scan['nsng']
     rs = torch.where(an.abs() < 1e-6, torch.zeros_like(an), scan['rsng'] / an)
     out = []

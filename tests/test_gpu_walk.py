@@ -9,7 +9,8 @@ import numpy as np
 import pytest
 import torch
 
-from nipet_b200 import diffprj, geometry, petprj
+from nipet_b200 import _lib, diffprj, geometry, petprj
+from nipet_b200.device import dev_ptr, get_geometry, stream_ptr
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -162,3 +163,44 @@ def test_walk_ray_outruns_planes(env, lines, nimg, kind):
             want = env['orc'].fprj(im, subs, span=1)
             size = env['orc'].fprj(np.abs(im), subs, span=1)
             assert (np.abs(g - want) <= 1e-5 * size + 1e-6 * size.max()).all()
+
+
+@pytest.mark.parametrize('span', [11, 1])
+@pytest.mark.parametrize('bs,nimg', [(1, 1), (1, 2), (2, 1), (2, 3), (4, 3), (4, 5)])
+def test_walk_fused_edges(env, span, bs, nimg):
+    """One fused sub-iteration over the edge LORs, images not a multiple of the width and count
+    levels decades apart, against the oracle's projections.  Bar: two projections' 1e-6 each and
+    the float32 ratio and update, 4e-6 relative L2."""
+    p, orc, subs = env['p'], env['orc'], env['subs']
+    nsn = 4084 if span == 1 else 837
+    dev = torch.device('cuda')
+    g, lib, st = get_geometry(p['txLUT'], p['axLUT'], dev), _lib.load(), stream_ptr(dev)
+    r = np.random.default_rng(10 * bs + nimg)
+    ims = np.stack([_image(3 * bs + i) + np.float32(1e-3) for i in range(nimg)])
+    ims *= (10.0 ** (-np.arange(nimg)))[:, None, None, None].astype(np.float32)
+    y = np.zeros((nimg, 68516, nsn), np.uint16)
+    y[:, subs] = r.poisson(3.0, (nimg, subs.size, nsn))
+    rs = np.zeros((68516, nsn), np.float32)
+    rs[subs] = r.uniform(0.1, 2.0, (subs.size, nsn))
+    rs[subs[2]] = 0
+    rscale = r.uniform(0.5, 2.0, nimg).astype(np.float32)
+    groups = -(-nimg // bs)
+    d = lambda a: torch.from_numpy(a).to(dev)  # noqa: E731
+    x, d_y, d_rs, d_sc, d_subs = d(ims), d(y), d(rs), d(rscale), d(subs)
+    sens = torch.full((320 * 320 * 128,), 2.0, device=dev)
+    msk = torch.ones(320 * 320 * 128, device=dev, dtype=torch.uint8)
+    xb = torch.empty(groups * bs * 320 * 320 * 128, device=dev)
+    bb = torch.empty_like(xb)
+    _lib.check(lib.nb_to_batch(dev_ptr(xb), dev_ptr(x), nimg, bs, st))
+    _lib.check(lib.nb_osem_batch_subset(g.handle, dev_ptr(xb), dev_ptr(bb.zero_()), dev_ptr(sens),
+                                        dev_ptr(msk), dev_ptr(d_y), dev_ptr(d_rs), dev_ptr(d_sc),
+                                        nimg, bs, 0, span, dev_ptr(d_subs), subs.size, st))
+    out = torch.empty_like(x)
+    _lib.check(lib.nb_from_batch(dev_ptr(out), dev_ptr(xb), nimg, bs, st))
+    g.check()
+    for i in range(nimg):
+        e = orc.fprj(ims[i], subs, span=span) + rscale[i] * rs[subs].astype(np.float64)
+        q = np.where(np.abs(e) < 1e-6, 0.0, y[i, subs] / np.where(e == 0, 1, e))
+        want = ims[i] * orc.bprj(q.astype(np.float32), subs, span=span) / 2.0
+        got = out[i].cpu().numpy().astype(np.float64)
+        assert np.linalg.norm(got - want) <= 4e-6 * np.linalg.norm(want)
