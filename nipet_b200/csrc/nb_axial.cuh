@@ -67,6 +67,15 @@ static __device__ __forceinline__ void nb_axial_setup(const nb_ray &R, float atn
   }
 }
 
+// An mMR ring pair (r0, r0 + d) as a ray (kind: 0 direct, 1 +RD, 2 -RD)
+static __device__ __forceinline__ nb_ray nb_ring_pair(int r0, int d, int kind) {
+  nb_ray R;
+  R.r0z = __fmul_rn((float)(r0 - NB_NRINGS / 2), NB_RING);
+  R.r1z = __fmul_rn((float)(r0 + d - NB_NRINGS / 2), NB_RING);
+  R.kind = (int8_t)kind;
+  return R;
+}
+
 // The first plane boundary (0 .. 127) an oblique ray of ring pair R reaches on its way up from
 // the LOR's entry point tp.
 static __device__ __forceinline__ int nb_first_plane(const nb_ray &R, float atn, float tp) {

@@ -102,6 +102,16 @@ static __device__ __forceinline__ void nb_bulk_g2s(void *dst_smem, const void *s
       : "memory");
 }
 
+// global -> shared copies of B = 4, 8 or 16 bytes a thread (aligned to B), and the wait for this
+// thread's
+template <int B> static __device__ __forceinline__ void nb_cp_async(void *dst_smem, const void *src_gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(nb_smem_u32(dst_smem)), "l"(src_gmem), "n"(B)
+               : "memory");
+}
+static __device__ __forceinline__ void nb_cp_async_wait() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 // global -> L2 prefetch (16-byte aligned, bytes a multiple of 16)
 static __device__ __forceinline__ void nb_bulk_prefetch_l2(const void *src_gmem, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src_gmem), "r"(bytes) : "memory");

@@ -235,14 +235,6 @@ __global__ void k_check_walk(const float4 *__restrict__ hdr, const float *__rest
 // One block of 64 threads per LOR, thread d for difference d.  FILL = false counts: sizes[lor]
 // in 16-byte units; FILL = true writes the records.  err: a schedule or list over capacity.
 // ---------------------------------------------------------------------------------------
-static __device__ __forceinline__ nb_ray ring_pair(int r0, int d, int kind) {
-  nb_ray R;
-  R.r0z = __fmul_rn((float)(r0 - NB_NRINGS / 2), NB_RING);
-  R.r1z = __fmul_rn((float)(r0 + d - NB_NRINGS / 2), NB_RING);
-  R.kind = (int8_t)kind;
-  return R;
-}
-
 template <bool FILL>
 __global__ void k_sched(const float4 *__restrict__ hdr, const float *__restrict__ st,
                         uint32_t *__restrict__ sizes, const uint32_t *__restrict__ rec_off,
@@ -260,7 +252,7 @@ __global__ void k_sched(const float4 *__restrict__ hdr, const float *__restrict_
     // the first boundary (relative to 2 r0) that most rays of the difference have
     int lo = 1 << 20, clo = 0, rlo = 0, rhi = 0;
     for (int r0 = 0; r0 + d < NB_NRINGS; r0++) {
-      const int k = nb_first_plane(ring_pair(r0, d, 1), h.y, h.x) - 2 * r0;
+      const int k = nb_first_plane(nb_ring_pair(r0, d, 1), h.y, h.x) - 2 * r0;
       if (k < lo) {
         rhi = rlo;
         lo = k;
@@ -273,11 +265,11 @@ __global__ void k_sched(const float4 *__restrict__ hdr, const float *__restrict_
     }
     const bool up = 2 * clo < NB_NRINGS - d;   // the other value is in the majority
     rc = up ? rhi : rlo;
-    m = nb_first_plane(ring_pair(rc, d, 1), h.y, h.x) - 2 * rc;
+    m = nb_first_plane(nb_ring_pair(rc, d, 1), h.y, h.x) - 2 * rc;
   }
   nb_axial A;
   A.tzc = A.dtz = 0.f;
-  if (live) nb_axial_setup(ring_pair(rc, d, 1), h.y, h.x, h.z, A);
+  if (live) nb_axial_setup(nb_ring_pair(rc, d, 1), h.y, h.x, h.z, A);
   auto walk = [&](bool fill, int base) {
     int k = 0;
     float tp = h.x, tzc = A.tzc;
@@ -323,11 +315,11 @@ __global__ void k_sched(const float4 *__restrict__ hdr, const float *__restrict_
   if (live)
     for (int r0 = 0; r0 + d < NB_NRINGS; r0++) {
       nb_axial U, D;
-      nb_axial_setup(ring_pair(r0, d, 1), h.y, h.x, h.z, U);
-      nb_axial_setup(ring_pair(r0, d, 2), h.y, h.x, h.z, D);
+      nb_axial_setup(nb_ring_pair(r0, d, 1), h.y, h.x, h.z, U);
+      nb_axial_setup(nb_ring_pair(r0, d, 2), h.y, h.x, h.z, D);
       // start planes at the group's own first crossing: one that is reached earlier (later)
       // than the group's has moved the ray one plane on (back) by then
-      const int k = nb_first_plane(ring_pair(r0, d, 1), h.y, h.x) - 2 * r0 - m;
+      const int k = nb_first_plane(nb_ring_pair(r0, d, 1), h.y, h.x) - 2 * r0 - m;
       const int bu = U.w - k - (2 * r0 + m - 1), bd = D.w + k - (2 * (r0 + d) - m + 1);
       for (int dir = 0; dir < 2; dir++) {
         const int b = dir ? bd : bu;

@@ -26,11 +26,17 @@
 // difference of two planes of opposite sign fits as well), so the differences cancel exactly: a
 // ray through empty planes is exactly zero whatever its neighbours hold, and integer sums do not
 // depend on the order.  A ray's own sum, with the fraction terms, is 64 bits wide: it collects
-// from one plane after another and can exceed what any of them holds.  In the back projection a ray's value is rounded once,
-// to 2^-22 of the LOR's largest, its two parts of a crossing sum to it exactly, and at most
-// 242 rays meet in a plane, so no sum leaves int32.  A chunk that holds a non-finite (or a
-// denormal-small) value is walked step by step in float32 instead, which keeps the value in
-// the rays that meet it.
+// from one plane after another and can exceed what any of them holds.
+//   The scale is set by the chunk's hottest plane, so a ray through values decades below it is a
+// sum of few quanta.  At the end of a LOR, rays below 2^20 quanta per chunk whose planes hold weak
+// values, and any below 1.5 x 2^16, are walked again step by step in float32, as the reference
+// walks every ray (walk_weak); so are all rays of an image whose chunk has no scale (a value that
+// is not finite, or above 2^100).  The fused mode leaves out those whose ratio does not need them:
+// nothing counted, or randoms above 2^20 quanta.  Every bin is then good to 1e-5 of its value, but
+// for slivers of a step (a fraction is good to 2^-25 of the step).
+//   In the back projection a ray's value is rounded once, to 2^-22 of the LOR's largest, its two
+// parts of a crossing sum to it exactly, and at most 242 rays meet in a plane, so no sum leaves
+// int32.
 //
 // Jobs.  One block per (LOR, image group); a finished block takes over a block that has not
 // started (cluster launch control), so LORs of 10 to 404 steps even out over the SMs and the
@@ -59,6 +65,11 @@ namespace nbw {
 constexpr uint32_t WAIT_POLLS = 1u << 20;
 enum { MODE_FWD = 0, MODE_BWD = 1, MODE_OSEM = 2 };
 constexpr int FXBITS = 23;    // back projection: |V| <= 2^23 (see the file comment)
+// A ray's sum is good to float32's precision from so many quanta per chunk on: a ray through
+// weak values, whose every voxel is rounded; and any other, which may clip a voxel or two
+constexpr float WEAK_QUANTA = 1048576.f, CLIP_QUANTA = 98304.f;   // 2^20, 1.5 * 2^16
+// A value is weak below 2^15 quanta for a step of 1/16 cm
+constexpr float WEAK_VALUE = 524288.f;
 constexpr int QBITS = NB_REC_QBITS;  // crossing fractions are int32 with this many fraction bits
 
 struct WalkArgs {
@@ -107,7 +118,12 @@ template <int BS, int CH, int NSEG> struct WSmem {
   static constexpr size_t max_off = align128(cs_off + 16ull * NB_STEP_STRIDE);  // [3][NSEG][BS]
   static constexpr size_t obl_off = align128(max_off + 12ull * NSEG * BS);      // [64]
   static constexpr size_t misc_off = obl_off + 256;
-  static constexpr size_t total = misc_off + 128;
+  static constexpr size_t total = misc_off + 256;
+  // walk_weak: the rays' integrals [4096][BS], the list of rays, then columns of the image
+  static constexpr size_t list_off = 4096ull * 4 * BS;
+  static constexpr size_t col_off = list_off + 4096 * 2;
+  static constexpr int ncol = (int)((region - col_off) / (512 * BS)) & ~7;
+  static_assert(region >= col_off + 16 * 512 * BS, "room for some columns");
   static_assert(total <= 227 * 1024, "too much shared memory");
 };
 
@@ -190,36 +206,201 @@ static __device__ __forceinline__ float oblique_s(int d, float atn) {
   return __fsqrt_rn(__fmaf_rn(az_atn, az_atn, 1.0f));
 }
 
-// One ray over steps [s0, s1) of a chunk, step by step in float32 (chunks whose values have
-// no fixed-point scale).  `ent` points at the ray's crossings of the chunk.
-template <int BS>
-static __device__ __noinline__ void slow_ray(const float *gimg, const int32_t *col,
-                                             const float *st, float tp, int s0, int s1, int z,
-                                             int dir, const uint2 *ent, int cnt, bool natural,
-                                             float *acc) {
-  // (plane 127 reads as zero: the padding slot, or no voxel in the natural order)
-  auto vox = [&](const float *c, int z, int k) {
-    return !natural ? c[nb_zi(z) * BS + k] : (z < NB_IMZ ? c[z] : 0.f);
-  };
-  for (int s = s0; s < s1; s++) {
-    const float tn = st[s], lt = __fsub_rn(tn, tp);
-    const float *c = gimg + (size_t)col[s] * (natural ? NB_IMZ : NB_COLW * BS);
-    tp = tn;
-    if (cnt > 0 && (int)ent->x == s) {
-      const float f = (float)(int)ent->y * (1.f / (1 << QBITS));
-      for (int k = 0; k < BS; k++)
-        acc[k] = fmaf(f * lt, vox(c, z, k), fmaf((1.f - f) * lt, vox(c, z + dir, k), acc[k]));
-      z += dir;
-      ent++;
-      cnt--;
-    } else {
-      for (int k = 0; k < BS; k++) acc[k] = fmaf(lt, vox(c, z, k), acc[k]);
+// does [lo, hi] hold a plane of the mask (words: planes 0, 2 .. 62; 64 .. 126; 1 .. 63; 65 .. 127)
+static __device__ __forceinline__ bool mask_meets(const unsigned *mask, int lo, int hi) {
+  bool hit = false;
+#pragma unroll
+  for (int par = 0; par < 2; par++) {
+    const uint2 m2 = *reinterpret_cast<const uint2 *>(mask + 2 * par);
+    const unsigned long long m = (unsigned long long)m2.y << 32 | m2.x;
+    const int a = (lo + 1 - par) >> 1, b = (hi - par) >> 1;   // b = -1: no odd plane below 1
+    hit |= b >= a && (m >> a & (~0ull >> (63 - (b - a)))) != 0ull;
+  }
+  return hit;
+}
+
+// Walks the rays of a LOR whose fixed-point sums (vals, [4096][BS]) are too few quanta to be good
+// to float32's precision again: step by step in float32, as the reference does, from columns
+// staged in shared memory (40 KB at a time).  All threads; false if there was none to walk.
+template <int BS, int NT, int MODE, class L>
+static __device__ __noinline__ bool walk_weak(const WalkArgs &a, unsigned char *smem, int par,
+                                              int g, int lor, int n, const float4 h) {
+  static_assert(NT % (128 * BS) == 0, "a thread stays with its plane and image");
+  const int32_t *scol = reinterpret_cast<const int32_t *>(
+      smem + L::cs_off + (size_t)par * 8 * NB_STEP_STRIDE);
+  const float *sst = reinterpret_cast<const float *>(scol) + NB_STEP_STRIDE;
+  const unsigned char *rec = smem + L::rec_off;
+  float *vals = reinterpret_cast<float *>(smem);
+  uint16_t *list = reinterpret_cast<uint16_t *>(smem + L::list_off);
+  float *cols = reinterpret_cast<float *>(smem + L::col_off);
+  unsigned char *misc = smem + L::misc_off;
+  int *scount = reinterpret_cast<int *>(misc + 40);
+  const float *sthr = reinterpret_cast<const float *>(misc + 96);
+  const int *sweak = reinterpret_cast<const int *>(misc + 112);
+  unsigned *smask = reinterpret_cast<unsigned *>(misc + 176);   // [BS][4] planes of weak values
+  const int tid = threadIdx.x;
+  const bool natural = MODE == MODE_FWD && BS == 1 && a.natural != 0;
+  const size_t stride = natural ? NB_IMZ : NB_COLW * BS;
+  const float *gimg = a.img + (size_t)g * NB_IMG_COL128 * BS;
+  if (tid == 0) *scount = 0;
+  if (tid < 4 * BS) smask[tid] = 0u;
+  // this thread's rays tid + i NT whose sums are weak in an image (bit k * R + i)
+  constexpr int R = 4096 / NT;
+  static_assert(R * BS <= 64, "a bit for each ray and image");
+  unsigned long long cand = 0ull;
+  bool flagged = false;
+#pragma unroll
+  for (int k = 0; k < BS; k++) {
+    const float clip = sthr[k] * CLIP_QUANTA, all = sweak[k] ? sthr[k] * WEAK_QUANTA : 0.f;
+    flagged |= sweak[k] != 0;
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+      const int ray = tid + i * NT;
+      const float f = ray < 2 * a.nslots ? fabsf(vals[ray * BS + k]) : __int_as_float(0x7f800000);
+      if (f < all || (f < clip && f > 0.f)) cand |= 1ull << (k * R + i);
     }
   }
+  if (MODE == MODE_OSEM) {
+    // where the randoms outweigh the error, or nothing was counted, the ratio does not need it
+    float rs[R];
+    int o[R];
+    unsigned long long any = cand;
+#pragma unroll
+    for (int k = 1; k < BS; k++) any |= cand >> (k * R);
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+      const int ray = tid + i * NT;
+      const nb_slot *S = a.slots + (ray >> 1);
+      const int16_t *out = a.span == 11 ? &S->o11A : &S->o1A;
+      o[i] = any >> i & 1u ? __ldg(out + (ray & 1)) : -1;
+    }
+#pragma unroll
+    for (int i = 0; i < R; i++) rs[i] = o[i] >= 0 ? __ldg(a.rs + (size_t)lor * a.nout + o[i]) : 0.f;
+#pragma unroll
+    for (int k = 0; k < BS; k++) {
+      const int rep = g * BS + k;
+      const float q = sthr[k], scale = rep < a.nrep ? a.rscale[rep] : 0.f;
+      const uint16_t *y = a.psng + ((size_t)(rep < a.nrep ? rep : 0) * a.naw + lor) * a.nout;
+#pragma unroll
+      for (int i = 0; i < R; i++)
+        if (cand >> (k * R + i) & 1u) {
+          const bool skip = o[i] < 0 || rep >= a.nrep || (q < __int_as_float(0x7f800000) &&
+                            (scale * rs[i] >= q * WEAK_QUANTA || __ldg(y + o[i]) == 0));
+          if (skip) cand &= ~(1ull << (k * R + i));
+        }
+    }
+  }
+  if (!__syncthreads_or(cand != 0ull)) return false;
+  if (flagged) {
+    const int e = tid % (128 * BS), q = e / BS, k = e % BS;
+    const int z = natural ? q : (q < 64 ? 2 * q : 2 * (q - 64) + 1);
+    const float lim = sthr[k] * WEAK_VALUE;
+    bool hit = false;
+    if (z < NB_IMZ)
+#pragma unroll 8
+      for (int s = tid / (128 * BS); s < n; s += NT / (128 * BS)) {
+        const float v = __ldg(gimg + (size_t)scol[s] * stride + e);
+        // (without a scale every value counts, NaN too)
+        hit |= v != 0.f && (fabsf(v) < lim || lim == __int_as_float(0x7f800000));
+      }
+    if (hit) atomicOr(&smask[4 * k + (z & 1) * 2 + (z >> 6)], 1u << (z >> 1 & 31));
+    __syncthreads();
+  }
+  const int last = n > 0 ? ((n - 1) >> 3) * 64 : 0;
+#pragma unroll
+  for (int i = 0; i < R; i++) {
+    const int ray = tid + i * NT;
+    bool weak = false;
+#pragma unroll
+    for (int k = 0; k < BS; k++)
+      if (cand >> (k * R + i) & 1u) {
+        const float f = fabsf(vals[ray * BS + k]);
+        if (f > 0.f && f < sthr[k] * CLIP_QUANTA) {
+          weak = true;
+        } else {
+          // the ray's planes, one more either side (its start plane may round away)
+          const uint32_t zz = a.slots[ray >> 1].zzd;
+          const int d = (int)(zz >> 16), m1 = rec[NB_REC_M + d] - 1, cnt = rec[NB_REC_KEND + last + d];
+          const int z = ray & 1 ? (int)(zz >> 8 & 255u) - m1 : (int)(zz & 255u) + m1;
+          weak |= mask_meets(smask + 4 * k, max(0, z - (ray & 1 ? cnt : 0) - 1),
+                             min(127, z + (ray & 1 ? 0 : cnt) + 1));
+        }
+      }
+    if (weak) list[atomicAdd(scount, 1)] = (uint16_t)ray;
+  }
+  __syncthreads();
+  const int count = *scount;
+  if (count == 0) return false;
+  for (int b0 = 0; b0 < count; b0 += NT) {
+    const bool live = b0 + tid < count;
+    const int ray = list[live ? b0 + tid : b0];
+    const uint32_t zz = a.slots[ray >> 1].zzd;
+    const int d = (int)(zz >> 16);
+    nb_axial A;
+    nb_axial_setup(nb_ring_pair((int)((d ? zz : zz >> (ray & 1) * 8) & 255u) / 2, d,
+                                d ? 1 + (ray & 1) : 0), h.y, h.x, h.z, A);
+    // offset of the ray's plane in a column (plane 127 reads as zero) and its change at the next
+    // crossing; in the col128 order every second crossing turns between the even and odd halves
+    int zo = (natural ? A.w : nb_zi(A.w)) * BS;
+    int dz = natural ? A.dir : (A.dir > 0 ? ((A.w & 1) ? -63 : 64) : ((A.w & 1) ? -64 : 63)) * BS;
+    const int dsum = natural ? 2 * A.dir : A.dir * BS;
+    float tp = h.x, tzc = A.tzc, acc[BS];
+#pragma unroll
+    for (int k = 0; k < BS; k++) acc[k] = 0.f;
+    for (int s0 = 0; s0 < n; s0 += L::ncol) {
+      const int m = min(L::ncol, n - s0);
+      __syncthreads();                        // the columns before have been walked
+      for (int x = tid; x < m * 128; x += NT)
+        if (!natural || (x & 127) < NB_IMZ)
+          nb_cp_async<4 * BS>(cols + x * BS, gimg + (size_t)scol[s0 + (x >> 7)] * stride + (x & 127) * BS);
+        else
+          cols[x] = 0.f;
+      nb_cp_async_wait();
+      __syncthreads();
+      if (!live) continue;
+      const float *c = cols + zo;
+      auto step = [&](int u, float tn) {
+        float v[BS];
+        ldv<BS>(c + u * 128 * BS, v);
+        const float w = __fsub_rn(fminf(tn, tzc), tp);
+#pragma unroll
+        for (int k = 0; k < BS; k++) acc[k] = fmaf(w, v[k], acc[k]);
+        if (tn > tzc) {
+          c += dz;
+          dz = dsum - dz;
+          ldv<BS>(c + u * 128 * BS, v);
+          const float w1 = __fsub_rn(tn, tzc);
+#pragma unroll
+          for (int k = 0; k < BS; k++) acc[k] = fmaf(w1, v[k], acc[k]);
+          tzc = __fadd_rn(tzc, A.dtz);
+        }
+        tp = tn;
+      };
+      int i = 0;
+      for (; i + 8 <= m; i += 8) {
+        float t[8];
+        ldv<4>(sst + s0 + i, t);
+        ldv<4>(sst + s0 + i + 4, t + 4);
+#pragma unroll
+        for (int u = 0; u < 8; u++) step(u, t[u]);
+        c += 8 * 128 * BS;
+      }
+      for (; i < m; i++) {
+        step(0, sst[s0 + i]);
+        c += 128 * BS;
+      }
+      zo = (int)(c - cols) - m * 128 * BS;
+    }
+    if (live)
+#pragma unroll
+      for (int k = 0; k < BS; k++) vals[ray * BS + k] = acc[k];
+  }
+  __syncthreads();
+  return true;
 }
 
 template <int BS, int CH, int NT, int MODE, int MINB>
-__global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
+__global__ void __launch_bounds__(NT, MINB) k_walk(const __grid_constant__ WalkArgs a) {
   constexpr int NSEG = NT / 64;               // step segments of a chunk, one per 64 threads
   constexpr int SEGL = CH / NSEG;
   constexpr int SPT = (NB_NSLOT + NT - 1) / NT;          // slots (ray pairs) per thread
@@ -248,6 +429,9 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
   int *snext = reinterpret_cast<int *>(misc + 36);
   unsigned *smax = reinterpret_cast<unsigned *>(smem + L::max_off);  // forward bounds
   unsigned *smaxb = reinterpret_cast<unsigned *>(misc + 64);         // [2][BS] backward
+  float *sthr = reinterpret_cast<float *>(misc + 96);                // [BS] sum of the quanta
+  int *sweak = reinterpret_cast<int *>(misc + 112);                  // [BS] weak values were met
+  unsigned *smin = reinterpret_cast<unsigned *>(misc + 128);         // [3][BS] least |value|
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int s = tid & 63;                     // scan: this thread's planes 2 s and 2 s + 1
@@ -260,6 +444,7 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
     nb_mbar_init(bar2, 1);
     *sflag = 0;
     for (int k = 0; k < 3 * NSEG * BS; k++) smax[k] = 0u;
+    for (int k = 0; k < 3 * BS; k++) smin[k] = ~0u;
     for (int k = 0; k < 2 * BS; k++) smaxb[k] = 0u;
     nb_fence_mbar_init();
   }
@@ -339,6 +524,8 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
     __syncthreads();
     if (*sflag) break;
     if (tid == 0) nb_clc_request(clc, bar2);
+    if (MODE != MODE_BWD && tid == 0)         // (this thread alone writes them)
+      for (int k = 0; k < BS; k++) sthr[k] = 0.f, sweak[k] = 0;
 
     auto slot_of = [&](int j) { return ((j & 1) ? (j + 1) * W - 1 - warp : j * W + warp) * 32 + lane; };
     // lengths of this thread's steps in the chunk at s0 (0 past the LOR's end, where the reads
@@ -440,13 +627,20 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
               mo = fmaf(lt[j], fabsf(O[j][v]), mo);
             }
             const unsigned u = __reduce_max_sync(0xffffffffu, max(__float_as_uint(me), __float_as_uint(mo)));
-            if (lane == 0 && u) atomicMax(&smax[(mrot * NSEG + seg) * BS + v], u);
+            if (u == 0u) continue;            // (the whole warp)
+            unsigned lo = ~0u;                // least non-zero |value|, as 2 * bits - 1
+#pragma unroll
+            for (int j = 0; j < SEGL; j++)
+              lo = min(lo, min(2u * __float_as_uint(E[j][v]) - 1u, 2u * __float_as_uint(O[j][v]) - 1u));
+            lo = __reduce_min_sync(0xffffffffu, lo);
+            if (lane == 0) {
+              atomicMax(&smax[(mrot * NSEG + seg) * BS + v], u);
+              atomicMin(&smin[mrot * BS + v], lo);
+            }
           }
         }
         __syncthreads();
         unsigned any = 0u;
-        bool slow = false;
-        const float t0 = s0 ? sst[s0 - 1] : h.x;
         float scale[BS], inv[BS], bnd[NSEG * BS];
 #pragma unroll
         for (int x = 0; x < NSEG * BS; x += 4)
@@ -458,34 +652,39 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
           for (int x = 0; x < NSEG; x++) bound += bnd[x * BS + k];
           const unsigned bb = __float_as_uint(bound);
           any |= bb;
-          // bound < 2^e: scale 2^(29 - e); non-finite, above 2^100 or below 2^-60: step by step
-          const int e = (int)(bb >> 23) - 126;
-          slow |= bb >= 0x71800000u || (bb != 0u && bb < 0x21800000u);
-          scale[k] = bb ? __uint_as_float((uint32_t)(min(max(29 - e, -126), 127) + 127) << 23) : 0.f;
-          inv[k] = __uint_as_float((uint32_t)(min(max(e - 29, -126), 127) + 127) << 23);
+          // bound < 2^e: scale 2^(29 - e), as far as float32 has it.  A bound that is not finite or
+          // above 2^100 has none: the image's rays are all walked again
+          const int x = min(155 - (int)(bb >> 23), 126);
+          const bool none = bb >= 0x71800000u;
+          scale[k] = bb && !none ? __uint_as_float((uint32_t)(127 + x) << 23) : 0.f;
+          inv[k] = bb && !none ? __uint_as_float((uint32_t)(127 - x) << 23) : 0.f;
+          if (bb != 0u && tid == 0) {
+            sthr[k] += none ? __int_as_float(0x7f800000) : inv[k];
+            if (none || smin[mrot * BS + k] < 2u * __float_as_uint(inv[k] * WEAK_VALUE) - 1u) sweak[k] = 1;
+          }
         }
         // cleared two chunks before its next use: its last readers are one barrier back
         if (tid < NSEG * BS) smax[((mrot + 2) % 3) * NSEG * BS + tid] = 0u;
+        if (tid < BS) smin[((mrot + 2) % 3) * BS + tid] = ~0u;
         mrot = (mrot + 1) % 3;
         if (any == 0u) continue;              // nothing but zeros
-        if (!slow) {
+        {
           // fixed-point running integrals: within the segment, then the segments before it
+          // (rounded with offsets spread over (-1/2, 1/2), so that the errors of equal values do
+          // not add up; 0 stays 0)
           int cE[SEGL][BS], cO[SEGL][BS], tE[BS], tO[BS];
-          float sv[BS];
 #pragma unroll
-          for (int v = 0; v < BS; v++) {
-            tE[v] = tO[v] = 0;
-            sv[v] = scale[v];
-          }
+          for (int v = 0; v < BS; v++) tE[v] = tO[v] = 0;
 #pragma unroll
           for (int j = 0; j < SEGL; j++) {
+            const float off = (float)(2 * ((5 * j + 2) % 8) - 7) / 16.f;
 #pragma unroll
             for (int v = 0; v < BS; v++) {
-              const float w = lt[j] * sv[v];
+              const float w = lt[j] * scale[v];
               cE[j][v] = tE[v];
               cO[j][v] = tO[v];
-              tE[v] += __float2int_rn(E[j][v] * w);
-              tO[v] += __float2int_rn(O[j][v] * w);
+              tE[v] += __float2int_rn(fmaf(E[j][v], w, off));
+              tO[v] += __float2int_rn(fmaf(O[j][v], w, off));
             }
             if (s == 31) sti<BS>(soc + (seg * (SEGL + 1) + j) * BS, cO[j]);
           }
@@ -568,12 +767,6 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
           int cnt = kend[krow1 * 64 + d] - ka;
           const int e0 = reinterpret_cast<const uint16_t *>(rec + NB_REC_OFF)[d] + ka;
           const int zA = (zz & 255) + ka, zB = ((zz >> 8) & 255) - ka;
-          if (slow) {
-            const uint2 *ent = reinterpret_cast<const uint2 *>(rec + NB_REC_ENT) + e0;
-            slow_ray<BS>(gimg, scol, sst, t0, s0, s1, zA, 1, ent, cnt, natural, FA[j]);
-            slow_ray<BS>(gimg, scol, sst, t0, s0, s1, zB, -1, ent, cnt, natural, FB[j]);
-            continue;
-          }
           const int endA = zA + cnt, endB = zB - cnt;
           uint32_t ep = rec_u + NB_REC_ENT + e0 * 8;
           // cursors of the next crossing and the one after (their plane offsets in a row);
@@ -638,8 +831,41 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const WalkArgs a) {
           }
         }
       }
-      __syncthreads();   // the walk is done: the table region and the record are free
-      if (MODE == MODE_FWD && tid == 0) next_job(job);
+      // rays whose sums are too few quanta to be good to float32's precision are walked again
+      bool weak = false;
+#pragma unroll
+      for (int k = 0; k < BS; k++) {
+        const float clip = sthr[k] * CLIP_QUANTA, all = sweak[k] ? sthr[k] * WEAK_QUANTA : 0.f;
+#pragma unroll
+        for (int j = 0; j < SPT; j++) {
+          const float fA = fabsf(FA[j][k]), fB = fabsf(FB[j][k]);
+          weak |= fA < all || (fA < clip && fA > 0.f) || fB < all || (fB < clip && fB > 0.f);
+        }
+      }
+      if (__syncthreads_or(weak)) {           // (the walk is done: the table region is free)
+#pragma unroll
+        for (int j = 0; j < SPT; j++) {
+          const int sl = slot_of(j);
+          if (sl >= a.nslots) continue;
+#pragma unroll
+          for (int k = 0; k < BS; k++) {
+            vals[2 * sl * BS + k] = FA[j][k];
+            vals[(2 * sl + 1) * BS + k] = FB[j][k];
+          }
+        }
+        __syncthreads();
+        if (walk_weak<BS, NT, MODE, L>(a, smem, job & 1, g, lor, n, h)) {
+#pragma unroll
+          for (int j = 0; j < SPT; j++) {
+            const int sl = slot_of(j);
+            if (sl >= a.nslots) continue;
+            ldv<BS>(vals + 2 * sl * BS, FA[j]);
+            ldv<BS>(vals + (2 * sl + 1) * BS, FB[j]);
+          }
+          __syncthreads();
+        }
+      }
+      if (MODE == MODE_FWD && tid == 0) next_job(job);   // the record is free
 
       // ratio of a bin (recon.cu:459-470): y / (Ax + rscale (r+s)/(an)), 0 where |.| < 1e-6
       auto ratio = [&](float v, int o, int k) {

@@ -165,6 +165,77 @@ def test_walk_ray_outruns_planes(env, lines, nimg, kind):
             assert (np.abs(g - want) <= 1e-5 * size + 1e-6 * size.max()).all()
 
 
+def _errors(env, im, subs, nimg, slack):
+    """Bins of nimg copies of an image against the oracle: 1e-5 of each, and `slack` besides."""
+    prj = diffprj.MMRProjector(env['p'], span=1, subs=subs)
+    got = prj.project(torch.from_numpy(np.stack([im] * nimg)).cuda()).cpu().numpy()
+    prj.check()
+    want = env['orc'].fprj(im, subs, span=1)
+    for g in got.astype(np.float64):
+        bad = np.abs(g - want) > 1e-5 * want + slack
+        assert not bad.any(), (bad.sum(), (np.abs(g - want)[bad] / want[bad]).max())
+
+
+@pytest.mark.parametrize('ratio', [1e3, 1e4, 1e5, 1e6, 1e8])
+@pytest.mark.parametrize('nimg', [1, 2, 4])
+def test_walk_weak_planes(env, nimg, ratio):
+    """Every bin of a positive image, however much hotter neighbouring planes are.  A crossing's
+    fraction of its step (0.3 cm at the most) is good to 2^-25, so rays that meet a hot plane,
+    perhaps with a sliver of a step, have that much of its value besides."""
+    im = np.random.default_rng(5).uniform(0.5, 1.5, (320, 320, 127)).astype(np.float32)
+    im[:, :, 20:60:4] *= np.float32(ratio)
+    im[:, :, 90:] /= np.float32(ratio)
+    subs = env['subs']
+    hot = env['orc'].fprj((im >= ratio / 2).astype(np.float32), subs, span=1) > 0
+    _errors(env, im, subs, nimg, hot * (0.3 * 2.0 ** -25 * im.max()))
+
+
+@pytest.mark.parametrize('ratio', [100, 300, 700, 2000, 10000])
+def test_walk_equal_weak_values(env, ratio):
+    """Equal weak values on LORs of equal steps (along the grid and its diagonals), whose rounding
+    errors would add up."""
+    s2c, crs = env['p']['txLUT']['s2c'].astype(int), env['p']['txLUT']['crs'].astype(float)
+    x, y = 0.5 * (crs[:, 0] + crs[:, 2]), 0.5 * (crs[:, 1] + crs[:, 3])
+    dx, dy = np.abs(x[s2c[:, 0]] - x[s2c[:, 1]]), np.abs(y[s2c[:, 0]] - y[s2c[:, 1]])
+    near = [np.argsort(v, kind='stable')[:200:20] for v in (dx, dy, np.abs(dx - dy))]
+    subs = np.unique(np.concatenate(near)).astype(np.int32)
+    im = np.full((320, 320, 127), 1.0 / ratio, np.float32)
+    im[:, :, 50:70] = 1.0
+    hot = env['orc'].fprj((im == 1).astype(np.float32), subs, span=1) > 0
+    for nimg in (1, 2, 4):
+        _errors(env, im, subs, nimg, hot * (0.3 * 2.0 ** -25))
+
+
+@pytest.mark.parametrize('value', [1e6, 1e9, 1e12])
+@pytest.mark.parametrize('nimg', [1, 2, 4])
+def test_walk_hot_voxel(env, nimg, value):
+    """A hot voxel leaves the rays that miss it, and those that only pass its plane, alone."""
+    im = np.random.default_rng(6).uniform(0.5, 1.5, (320, 320, 127)).astype(np.float32)
+    im[:, :, 100:] *= 1e-3
+    for vox in ((160, 150, 63), (161, 150, 20), (159, 210, 100)):
+        im[vox] = value
+    subs = env['subs']
+    hot = env['orc'].fprj((im == np.float32(value)).astype(np.float32), subs, span=1) > 0
+    _errors(env, im, subs, nimg, hot * (0.3 * 2.0 ** -25 * value))
+
+
+@pytest.mark.parametrize('nimg', [1, 2, 4])
+def test_walk_clipped_voxels(env, lines, nimg):
+    """Bins that clip a voxel or two, to 1e-5 of their own value."""
+    subs, ims = lines
+    _errors(env, ims[1], subs, nimg, 0.0)
+
+
+@pytest.mark.parametrize('value', [1e-20, 1e-33])
+@pytest.mark.parametrize('nimg', [1, 2, 4])
+def test_walk_faint_background(env, nimg, value):
+    """Values far below 2^-60 beside ordinary ones, and on their own."""
+    r = np.random.default_rng(8)
+    im = (r.uniform(0.5, 1.5, (320, 320, 127)) * value).astype(np.float32)
+    im[140:180, 140:180, 50:70] += r.uniform(0.5, 1.5, (40, 40, 20)).astype(np.float32)
+    _errors(env, im, env['subs'], nimg, 0.0)
+
+
 @pytest.mark.parametrize('span', [11, 1])
 @pytest.mark.parametrize('bs,nimg', [(1, 1), (1, 2), (2, 1), (2, 3), (4, 3), (4, 5)])
 def test_walk_fused_edges(env, span, bs, nimg):
