@@ -228,9 +228,10 @@ __global__ void k_check_walk(const float4 *__restrict__ hdr, const float *__rest
 // schedule is that ray's own walk (prjf.cu:164-190: at most one crossing a step, the crossing
 // parameter advanced by float additions).  What differs between the rays of a difference is
 // the start plane where it rounds across a plane boundary (~700 of 2.8e8 rays); those are
-// listed with their offset.  A first boundary that rounds to the next one is the same walk
-// with a segment of ~1e-6 cm moved between neighbouring planes, so only the start plane at the
-// group's own first crossing matters.
+// listed with their offset.  Where the first or last boundary of a pair rounds to the next one
+// (some pairs of one difference on 18 of the mMR's LORs), its first crossing or their spacing is another float; the
+// additions of another spacing drift by up to 1e-4 cm along the walk.  Such pairs get a schedule
+// of their own, numbered 61 .. 63.
 //
 // One block of 64 threads per LOR, thread d for difference d.  FILL = false counts: sizes[lor]
 // in 16-byte units; FILL = true writes the records.  err: a schedule or list over capacity.
@@ -240,36 +241,68 @@ __global__ void k_sched(const float4 *__restrict__ hdr, const float *__restrict_
                         uint32_t *__restrict__ sizes, const uint32_t *__restrict__ rec_off,
                         unsigned char *__restrict__ rec, int *err) {
   const int lor = blockIdx.x, d = threadIdx.x;
-  __shared__ int scnt[64], soff[64], nirr;
+  __shared__ int scnt[64], soff[64], nirr, nalt, alt_d[NB_REC_NALT], alt_r0[NB_REC_NALT];
   const float4 h = hdr[lor];
   const int n = __float_as_int(h.w);
   const float *t = st + (size_t)lor * NB_STEP_STRIDE;
   unsigned char *out = FILL ? rec + (size_t)rec_off[lor] * 16 : nullptr;
-  if (d == 0) nirr = 0;
+  if (d == 0) nirr = nalt = 0;
+  __syncthreads();
   int m = 1, rc = 0;
-  const bool live = d >= 1 && d <= NB_MAXRD && n > 0;
-  if (live) {
-    // the first boundary (relative to 2 r0) that most rays of the difference have
-    int lo = 1 << 20, clo = 0, rlo = 0, rhi = 0;
-    for (int r0 = 0; r0 + d < NB_NRINGS; r0++) {
-      const int k = nb_first_plane(nb_ring_pair(r0, d, 1), h.y, h.x) - 2 * r0;
-      if (k < lo) {
-        rhi = rlo;
-        lo = k;
-        clo = 0;
-        rlo = r0;
-      } else if (k > lo) {
-        rhi = r0;
+  bool live = d >= 1 && d <= NB_MAXRD && n > 0;
+  auto first = [&](int r0, int d) { return nb_first_plane(nb_ring_pair(r0, d, 1), h.y, h.x) - 2 * r0; };
+  auto up_ray = [&](int r0, int d, nb_axial &U) { nb_axial_setup(nb_ring_pair(r0, d, 1), h.y, h.x, h.z, U); };
+  // do the pairs r0 and r1 of difference d cross at the same floats?
+  auto same = [&](int r0, int r1, int d) {
+    nb_axial U, V;
+    up_ray(r0, d, U);
+    up_ray(r1, d, V);
+    return first(r0, d) == first(r1, d) && __float_as_int(U.tzc) == __float_as_int(V.tzc) &&
+           __float_as_int(U.dtz) == __float_as_int(V.dtz);  // (a single crossing has no spacing: NaN)
+  };
+  // the pair whose schedule pair r0 of this thread's difference follows, and its number
+  auto schedule = [&](int r0, int &id) {
+    id = d;
+    if (same(r0, rc, d)) return rc;
+    for (int x = 0; x < min(nalt, NB_REC_NALT); x++)
+      if (alt_d[x] == d && same(r0, alt_r0[x], d)) {
+        id = NB_MAXRD + 1 + x;
+        return alt_r0[x];
       }
-      clo += k == lo;
+    return -1;
+  };
+  if (live) {
+    // the pair that most agree with (Boyer and Moore's majority vote)
+    for (int r0 = 0, votes = 0; r0 + d < NB_NRINGS; r0++) {
+      if (votes == 0) rc = r0;
+      votes += same(r0, rc, d) ? 1 : -1;
     }
-    const bool up = 2 * clo < NB_NRINGS - d;   // the other value is in the majority
-    rc = up ? rhi : rlo;
-    m = nb_first_plane(nb_ring_pair(rc, d, 1), h.y, h.x) - 2 * rc;
+    // pairs that cross at other floats
+    int mine = 0, own[NB_REC_NALT];
+    for (int r0 = 0; r0 + d < NB_NRINGS; r0++) {
+      bool found = same(r0, rc, d);
+      for (int x = 0; x < mine; x++) found = found || same(r0, own[x], d);
+      if (found) continue;
+      const int i = atomicAdd(&nalt, 1);
+      if (i >= NB_REC_NALT || mine >= NB_REC_NALT) break;
+      own[mine++] = r0;
+      alt_d[i] = d;
+      alt_r0[i] = r0;
+    }
+  }
+  __syncthreads();
+  int dd = d;                                  // ring difference of this thread's schedule
+  if (d > NB_MAXRD && d - NB_MAXRD - 1 < min(nalt, NB_REC_NALT)) {
+    live = true;
+    dd = alt_d[d - NB_MAXRD - 1];
+    rc = alt_r0[d - NB_MAXRD - 1];
   }
   nb_axial A;
   A.tzc = A.dtz = 0.f;
-  if (live) nb_axial_setup(nb_ring_pair(rc, d, 1), h.y, h.x, h.z, A);
+  if (live) {
+    m = first(rc, dd);
+    up_ray(rc, dd, A);
+  }
   auto walk = [&](bool fill, int base) {
     int k = 0;
     float tp = h.x, tzc = A.tzc;
@@ -303,7 +336,7 @@ __global__ void k_sched(const float4 *__restrict__ hdr, const float *__restrict_
       tot += scnt[x];
       if (scnt[x] > 255) atomicOr(err, 1);
     }
-    if (tot > NB_REC_MAXENT) atomicOr(err, 1);
+    if (tot > NB_REC_MAXENT || nalt > NB_REC_NALT) atomicOr(err, 1);
     if (!FILL) sizes[lor] = (uint32_t)(NB_REC_ENT + ((tot + 1) & ~1) * 8) / 16;
   }
   __syncthreads();
@@ -312,23 +345,32 @@ __global__ void k_sched(const float4 *__restrict__ hdr, const float *__restrict_
   out[NB_REC_M + d] = (uint8_t)m;
   reinterpret_cast<uint16_t *>(out + NB_REC_OFF)[d] = (uint16_t)soff[d];
   if (live && (m < 1 || m > 255)) atomicOr(err, 1);
-  if (live)
+  if (d > NB_MAXRD) out[NB_REC_META + 2 + d - NB_MAXRD - 1] = (uint8_t)(live ? dd : 0);
+  auto list = [&](int r0, int what, int value) {
+    const int i = atomicAdd(&nirr, 1);
+    if (i < NB_REC_MAXIRR)
+      reinterpret_cast<uchar4 *>(out + NB_REC_IRR)[i] =
+          make_uchar4((uint8_t)d, (uint8_t)r0, (uint8_t)what, (uint8_t)(int8_t)value);
+  };
+  if (live && d <= NB_MAXRD)
     for (int r0 = 0; r0 + d < NB_NRINGS; r0++) {
       nb_axial U, D;
-      nb_axial_setup(nb_ring_pair(r0, d, 1), h.y, h.x, h.z, U);
+      up_ray(r0, d, U);
       nb_axial_setup(nb_ring_pair(r0, d, 2), h.y, h.x, h.z, D);
-      // start planes at the group's own first crossing: one that is reached earlier (later)
-      // than the group's has moved the ray one plane on (back) by then
-      const int k = nb_first_plane(nb_ring_pair(r0, d, 1), h.y, h.x) - 2 * r0 - m;
-      const int bu = U.w - k - (2 * r0 + m - 1), bd = D.w + k - (2 * (r0 + d) - m + 1);
+      int id;
+      const int rs = schedule(r0, id);
+      if (rs < 0) {
+        atomicOr(err, 1);
+        continue;
+      }
+      if (id != d) list(r0, 2, id);
+      const int ms = first(rs, d);
+      const int bu = U.w - (2 * r0 + ms - 1), bd = D.w - (2 * (r0 + d) - ms + 1);
       for (int dir = 0; dir < 2; dir++) {
         const int b = dir ? bd : bu;
         if (b == 0) continue;
         if (b < -7 || b > 7) atomicOr(err, 2);
-        const int i = atomicAdd(&nirr, 1);
-        if (i < NB_REC_MAXIRR)
-          reinterpret_cast<uchar4 *>(out + NB_REC_IRR)[i] =
-              make_uchar4((uint8_t)d, (uint8_t)r0, (uint8_t)dir, (uint8_t)(int8_t)b);
+        list(r0, dir, b);
       }
     }
   __syncthreads();

@@ -33,13 +33,15 @@ struct nb_slot {
 };
 #define NB_NSLOT 2048  // slot table capacity: 32 for the direct planes, 2010 pairs, padding
 
-// Crossing schedule of a LOR (k_sched, nb_geom.cu), 16-byte aligned:
-//   kend[52][64]  crossings of difference d up to and including the steps of 8-step row r
+// Crossing schedule of a LOR (k_sched, nb_geom.cu), 16-byte aligned.  Schedule d is that of the
+// ring pairs of difference d; 61 .. 63 are those of pairs that cross at other floats than the
+// rest of their difference.
+//   kend[52][64]  crossings of a schedule up to and including the steps of 8-step row r
 //   m[64]         first plane boundary the upward ray crosses, relative to its ring's 2 r0
-//   off[64]       first entry of difference d (uint16)
-//   meta          uint16 count of irregular rays
+//   off[64]       first entry of a schedule (uint16)
+//   meta          uint16 count of irregular rays, then the differences of schedules 61 .. 63
 //   irr[96]       {d, r0, 0 up / 1 down, start plane offset}: rays whose start plane rounds
-//                 away from their group's
+//                 away from their schedule's; {d, r0, 2, schedule}: pairs that follow another
 //   entries       {int32 step, int32 fraction of the step before the crossing (2^26 = 1)}
 #define NB_REC_KEND 0
 #define NB_REC_M 3328
@@ -47,8 +49,9 @@ struct nb_slot {
 #define NB_REC_META 3520
 #define NB_REC_IRR 3536
 #define NB_REC_MAXIRR 96
+#define NB_REC_NALT 3
 #define NB_REC_ENT 3920
-#define NB_REC_MAXENT 3392
+#define NB_REC_MAXENT 3584
 #define NB_REC_QBITS 26
 #define NB_REC_MAX (NB_REC_ENT + 8 * NB_REC_MAXENT)
 

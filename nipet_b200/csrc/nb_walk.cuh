@@ -548,8 +548,8 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const __grid_constant__ WalkA
       }
     };
 
-    // this thread's slots: start planes of the two rays (8 bits each) and ring difference;
-    // the few rays whose start plane rounds away from their group's are listed in the record
+    // this thread's slots: start planes of the two rays (8 bits each) and crossing schedule (the
+    // ring difference, but for the few pairs listed in the record)
     uint32_t zzd[SPT];
     const int nirr = *reinterpret_cast<const uint16_t *>(rec + NB_REC_META);
 #pragma unroll
@@ -558,15 +558,21 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const __grid_constant__ WalkA
       zzd[j] = 0u;
       if (sl >= a.nslots) continue;
       const uint32_t zz = __ldg(&a.slots[sl].zzd);
-      // the upward ray starts m - 1 planes above its ring's, the downward one as many below
-      zzd[j] = zz - (uint32_t)(rec[NB_REC_M + (zz >> 16)] - 1) * 255u;
+      uint32_t id = zz >> 16, off = 0u;
       for (int x = 0; x < nirr; x++) {
         const char4 e = reinterpret_cast<const char4 *>(rec + NB_REC_IRR)[x];
-        if (e.x == (int)(zz >> 16) && 2 * (int)e.y == (int)(zz & 255u))
-          zzd[j] += (uint32_t)(e.z ? 256 * (int)e.w : (int)e.w);
+        if (e.x == (int)(zz >> 16) && 2 * (int)e.y == (int)(zz & 255u)) {
+          if (e.z == 2)
+            id = (uint32_t)e.w;
+          else
+            off += (uint32_t)(e.z ? 256 * (int)e.w : (int)e.w);
+        }
       }
+      // the upward ray starts m - 1 planes above its ring's, the downward one as many below
+      zzd[j] = (zz & 0xffffu) - (uint32_t)(rec[NB_REC_M + id] - 1) * 255u + off + (id << 16);
     }
-    if (tid < 64) sobl[tid] = oblique_s(tid, h.y);
+    if (tid < 64)
+      sobl[tid] = oblique_s(tid <= NB_MAXRD ? tid : rec[NB_REC_META + 2 + tid - NB_MAXRD - 1], h.y);
     if (MODE == MODE_BWD) __syncthreads();           // (the forward pass has later barriers)
 
     float FA[SPT][BS], FB[SPT][BS];           // forward: line integrals

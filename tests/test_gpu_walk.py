@@ -236,6 +236,21 @@ def test_walk_faint_background(env, nimg, value):
     _errors(env, im, env['subs'], nimg, 0.0)
 
 
+def test_walk_pairs_with_own_crossings(env):
+    """LORs on which a first or last plane boundary of some ring pairs rounds to the next one, so
+    that they cross planes at other floats than the rest of their difference.  Bar: each ray's
+    value is rounded to 2^-22 of the largest, and a voxel's rays and its float32 sum, 2e-6."""
+    p, orc = env['p'], env['orc']
+    r = np.random.default_rng(4)
+    for lor in (11712, 13025, 14216, 17924, 32699, 35929, 45722, 53209, 64252):
+        sub = np.array([lor], np.int32)
+        si = r.exponential(1.0, (1, 4084)).astype(np.float32)
+        b = torch.zeros((320, 320, 127), device='cuda')
+        petprj.bprj(b, torch.from_numpy(si).cuda(), p['txLUT'], p['axLUT'], sub, _cnt(env, 1))
+        want = orc.bprj(si, sub, span=1)
+        assert np.abs(b.cpu().numpy() - want).max() <= 2e-6 * want.max(), lor
+
+
 @pytest.mark.parametrize('span', [11, 1])
 @pytest.mark.parametrize('bs,nimg', [(1, 1), (1, 2), (2, 1), (2, 3), (4, 3), (4, 5)])
 def test_walk_fused_edges(env, span, bs, nimg):
