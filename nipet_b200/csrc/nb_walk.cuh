@@ -36,7 +36,7 @@
 // for slivers of a step (a fraction is good to 2^-25 of the step).
 //   In the back projection a ray's value is rounded once, to 2^-22 of the LOR's largest, its two
 // parts of a crossing sum to it exactly, and at most 242 rays meet in a plane, so no sum leaves
-// int32.
+// int32.  An image with a value that is not finite goes to the voxels ray by ray in float32.
 //
 // Jobs.  One block per (LOR, image group); a finished block takes over a block that has not
 // started (cluster launch control), so LORs of 10 to 404 steps even out over the SMs and the
@@ -107,6 +107,7 @@ __host__ __device__ constexpr size_t cmax(size_t a, size_t b) { return a > b ? a
 template <int BS, int CH, int NSEG> struct WSmem {
   static constexpr size_t tab = (size_t)CH * 1024 * BS;
   static constexpr size_t gacc = (size_t)(CH + 1) * 512 * BS;
+  static_assert(gacc >= 4096ull * 4 * BS, "a LOR's ray values fit the accumulators");
   static constexpr size_t stage = (size_t)CH * 512 * BS;
   static constexpr size_t region = cmax(cmax(tab, 4096ull * 4 * BS), align128(gacc) + stage);
   static constexpr size_t stg_off = align128(gacc);
@@ -397,6 +398,46 @@ static __device__ __noinline__ bool walk_weak(const WalkArgs &a, unsigned char *
   }
   __syncthreads();
   return true;
+}
+
+// Back projection of a LOR's values (vals, [4096][BS]) for the images of `which`: step by step in
+// float32, straight into the image.  For values without a fixed-point scale, which reach the
+// voxels of their rays and no others.  All threads.
+template <int BS, int NT, class L>
+static __device__ __forceinline__ void spread_rays(const WalkArgs &a, unsigned char *smem, int par,
+                                                int g, int n, const float4 h, unsigned which) {
+  const int32_t *scol = reinterpret_cast<const int32_t *>(
+      smem + L::cs_off + (size_t)par * 8 * NB_STEP_STRIDE);
+  const float *sst = reinterpret_cast<const float *>(scol) + NB_STEP_STRIDE;
+  const float *vals = reinterpret_cast<const float *>(smem);
+  float *gb = a.bimg + (size_t)g * NB_IMG_COL128 * BS;
+  for (int ray = threadIdx.x; ray < 2 * a.nslots; ray += NT) {
+    const uint32_t zz = a.slots[ray >> 1].zzd;
+    const int d = (int)(zz >> 16);
+    nb_axial A;
+    nb_axial_setup(nb_ring_pair((int)((d ? zz : zz >> (ray & 1) * 8) & 255u) / 2, d,
+                                d ? 1 + (ray & 1) : 0), h.y, h.x, h.z, A);
+    for (int k = 0; k < BS; k++) {
+      const float v = vals[ray * BS + k];
+      if (!(which >> k & 1u) || v == 0.f) continue;
+      int z = A.w;
+      float tp = h.x, tzc = A.tzc;
+      auto add = [&](int s, float w) {        // plane 127 is padding
+        if (w != 0.f && z < NB_IMZ)
+          atomicAdd(gb + ((size_t)scol[s] * NB_COLW + nb_zi(z)) * BS + k, w * v);
+      };
+      for (int s = 0; s < n; s++) {
+        const float tn = sst[s];
+        add(s, __fsub_rn(fminf(tn, tzc), tp));
+        if (tn > tzc) {
+          z += A.dir;
+          add(s, __fsub_rn(tn, tzc));
+          tzc = __fadd_rn(tzc, A.dtz);
+        }
+        tp = tn;
+      }
+    }
+  }
 }
 
 template <int BS, int CH, int NT, int MODE, int MINB>
@@ -946,9 +987,9 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const __grid_constant__ WalkA
     if (MODE != MODE_FWD) {
       // values to spread and their fixed-point scale, per image (images of one group can
       // differ in count level by orders of magnitude)
-      float mm[BS];
+      unsigned mm[BS];                        // largest |value|, as bits (NaN above infinity)
 #pragma unroll
-      for (int k = 0; k < BS; k++) mm[k] = 0.f;
+      for (int k = 0; k < BS; k++) mm[k] = 0u;
 #pragma unroll
       for (int j = 0; j < SPT; j++) {
         const int sl = slot_of(j);
@@ -974,13 +1015,13 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const __grid_constant__ WalkA
           }
           FA[j][k] *= so;
           FB[j][k] *= so;
-          mm[k] = fmaxf(mm[k], fmaxf(fabsf(FA[j][k]), fabsf(FB[j][k])));
+          mm[k] = max(mm[k], max(__float_as_uint(fabsf(FA[j][k])), __float_as_uint(fabsf(FB[j][k]))));
         }
       }
       const int par = job & 1;
 #pragma unroll
       for (int k = 0; k < BS; k++) {
-        const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(mm[k]));
+        const unsigned m = __reduce_max_sync(0xffffffffu, mm[k]);
         if (lane == 0 && m) atomicMax(&smaxb[par * BS + k], m);
       }
       for (int i = tid; i < 128 * BS; i += NT) srun[i] = 0;
@@ -988,6 +1029,28 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const __grid_constant__ WalkA
       if (MODE == MODE_OSEM)                  // (the ratios have been read; a barrier follows)
         for (int i = tid; i < (CH + 1) * 32 * BS; i += NT)
           reinterpret_cast<int4 *>(gacc)[i] = make_int4(0, 0, 0, 0);
+      unsigned none = 0u;                     // images without a scale: a value is not finite
+#pragma unroll
+      for (int k = 0; k < BS; k++) none |= (smaxb[par * BS + k] >= 0x7f800000u ? 1u : 0u) << k;
+      if (none) {
+        // these images' rays one by one, through the accumulators' memory
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < SPT; j++) {
+          const int sl = slot_of(j);
+          if (sl >= a.nslots) continue;
+#pragma unroll
+          for (int k = 0; k < BS; k++) {
+            vals[2 * sl * BS + k] = FA[j][k];
+            vals[(2 * sl + 1) * BS + k] = FB[j][k];
+          }
+        }
+        __syncthreads();
+        spread_rays<BS, NT, L>(a, smem, job & 1, g, n, h, none);
+        __syncthreads();
+        for (int i = tid; i < (CH + 1) * 128 * BS; i += NT) gacc[i] = 0;
+        __syncthreads();
+      }
       float inv[BS];
       int VA[SPT][BS], VB_[SPT][BS];          // the rays' values, integers
       unsigned any = 0u;
@@ -996,7 +1059,7 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const __grid_constant__ WalkA
         const unsigned mb = smaxb[par * BS + k];
         float sc = 0.f;
         inv[k] = 0.f;
-        if (mb != 0u && (mb >> 23) < 255u) {
+        if (mb != 0u && mb < 0x7f800000u) {
           const int e = max((int)(mb >> 23) - 126, -96);   // max < 2^e
           sc = __uint_as_float((uint32_t)(FXBITS - e + 127) << 23);
           inv[k] = __uint_as_float((uint32_t)(e - FXBITS + 127) << 23);
@@ -1004,7 +1067,6 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const __grid_constant__ WalkA
         }
 #pragma unroll
         for (int j = 0; j < SPT; j++) {
-          // a NaN, or an infinity (scale 0), becomes 0
           VA[j][k] = __float2int_rn(FA[j][k] * sc);
           VB_[j][k] = __float2int_rn(FB[j][k] * sc);
         }

@@ -251,6 +251,51 @@ def test_walk_pairs_with_own_crossings(env):
         assert np.abs(b.cpu().numpy() - want).max() <= 2e-6 * want.max(), lor
 
 
+@pytest.mark.parametrize('bad', [np.inf, np.nan])
+@pytest.mark.parametrize('nimg', [1, 2, 4])
+def test_walk_non_finite_bin(env, nimg, bad):
+    """A value that is not finite reaches the voxels of its ray, in its image, and no others."""
+    p, orc, subs = env['p'], env['orc'], env['subs']
+    row, o = 5, _ray_bin(p, 20, 11, True)
+    prj = diffprj.MMRProjector(p, span=1, subs=subs)
+    si = np.random.default_rng(nimg).exponential(1.0, (nimg, subs.size, 4084)).astype(np.float32)
+    si[:, row, o] = 0
+    run = lambda x: prj.backproject(torch.from_numpy(x).cuda()).cpu().numpy().astype(np.float64)  # noqa: E731
+    ref = run(si)
+    hit = _line(orc, subs[row], o) > 0
+    si[nimg - 1, row, o] = bad
+    got = run(si)
+    prj.check()
+    assert hit.any() and not np.isfinite(got[-1][hit]).any()
+    for i in range(nimg):
+        keep = ~hit if i == nimg - 1 else np.ones_like(hit)
+        assert np.linalg.norm((got[i] - ref[i])[keep]) <= 1e-6 * np.linalg.norm(ref[i])
+        assert not got[i][keep & (ref[i] == 0)].any()
+
+
+def test_walk_fused_non_finite_ratio(env):
+    """The same for a ratio of the fused sub-iteration (NaN randoms of one bin)."""
+    p, orc, subs = env['p'], env['orc'], env['subs']
+    dev = torch.device('cuda')
+    g, lib, st = get_geometry(p['txLUT'], p['axLUT'], dev), _lib.load(), stream_ptr(dev)
+    row, o = 7, _ray_bin(p, 33, 20, False)
+    hit = _line(orc, subs[row], o) > 0
+    y = torch.ones((1, 68516, 4084), device=dev, dtype=torch.int16).view(torch.uint16)
+    rs = torch.ones((68516, 4084), device=dev)
+    rs[int(subs[row]), o] = float('nan')
+    d_subs, one = torch.from_numpy(subs).to(dev), torch.ones(1, device=dev)
+    n = 320 * 320 * 128
+    x, b, sens = torch.ones(n, device=dev), torch.zeros(n, device=dev), torch.ones(n, device=dev)
+    _lib.check(lib.nb_osem_batch_subset(g.handle, dev_ptr(x), dev_ptr(b), dev_ptr(sens),
+                                        dev_ptr(sens.to(torch.uint8)), dev_ptr(y), dev_ptr(rs),
+                                        dev_ptr(one), 1, 1, 0, 1, dev_ptr(d_subs), subs.size, st))
+    out = torch.empty((320, 320, 127), device=dev)
+    _lib.check(lib.nb_from_batch(dev_ptr(out), dev_ptr(x), 1, 1, st))
+    g.check()
+    out = out.cpu().numpy()
+    assert np.isnan(out[hit]).all() and np.isfinite(out[~hit]).all()
+
+
 @pytest.mark.parametrize('span', [11, 1])
 @pytest.mark.parametrize('bs,nimg', [(1, 1), (1, 2), (2, 1), (2, 3), (4, 3), (4, 5)])
 def test_walk_fused_edges(env, span, bs, nimg):
