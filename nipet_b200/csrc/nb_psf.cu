@@ -25,8 +25,10 @@ struct PsfKernel {
 // z pass: one warp per transaxial column, four consecutive planes per lane.  The column is
 // put in plane order in shared memory with a zero halo; a lane's 20 inputs are five 16-byte
 // reads instead of 17 reads per output.  A warp reads its column before it writes it, so dst
-// may be src.
+// may be src.  VEC: images that start on an 8-byte boundary move two planes at a time; others,
+// which the other two passes take as they are, one.
 constexpr int ZW = 8;  // warps per block
+template <bool VEC>
 __global__ void __launch_bounds__(ZW * 32) k_psf_z(float *dst, const float *src,
                                                    const PsfKernel K) {
   __shared__ __align__(16) float sh[ZW][NB_COLW + 2 * R];
@@ -38,8 +40,15 @@ __global__ void __launch_bounds__(ZW * 32) k_psf_z(float *dst, const float *src,
   }
   for (int col = blockIdx.x * ZW + (threadIdx.x >> 5); col < NB_NCOL; col += gridDim.x * ZW) {
     // slot of z: even z at z/2, odd z at 64 + z/2; z = 127 is the zero padding slot
-    const float2 *c = reinterpret_cast<const float2 *>(src + (size_t)col * NB_COLW);
-    const float2 ev = c[lane], od = c[32 + lane];
+    const float *c = src + (size_t)col * NB_COLW + 2 * lane;
+    float2 ev, od;
+    if (VEC) {
+      ev = *reinterpret_cast<const float2 *>(c);
+      od = *reinterpret_cast<const float2 *>(c + 64);
+    } else {
+      ev = make_float2(c[0], c[1]);
+      od = make_float2(c[64], c[65]);
+    }
     __syncwarp();
     *reinterpret_cast<float4 *>(s + R + 4 * lane) =
         make_float4(ev.x, od.x, ev.y, lane == 31 ? 0.f : od.y);
@@ -55,9 +64,17 @@ __global__ void __launch_bounds__(ZW * 32) k_psf_z(float *dst, const float *src,
       for (int j = -R; j <= R; j++) sum = __fmaf_rn(K.k[0][R - j], v[u + R + j], sum);
       o[u] = sum;
     }
-    float2 *q = reinterpret_cast<float2 *>(dst + (size_t)col * NB_COLW);
-    q[lane] = make_float2(o[0], o[2]);
-    q[32 + lane] = make_float2(o[1], lane == 31 ? 0.f : o[3]);
+    float *q = dst + (size_t)col * NB_COLW + 2 * lane;
+    if (lane == 31) o[3] = 0.f;
+    if (VEC) {
+      *reinterpret_cast<float2 *>(q) = make_float2(o[0], o[2]);
+      *reinterpret_cast<float2 *>(q + 64) = make_float2(o[1], o[3]);
+    } else {
+      q[0] = o[0];
+      q[1] = o[2];
+      q[64] = o[1];
+      q[65] = o[3];
+    }
   }
 }
 
@@ -114,7 +131,10 @@ extern "C" int nb_psf_col128(float *dst128, const float *src128, const float *kr
   NB_CUDA(cudaGetDevice(&dev));
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   // z: src -> dst (dst may be src), x: dst -> tmp, y: tmp -> dst: the reference's order
-  k_psf_z<<<nsm * 8, ZW * 32, 0, s>>>(dst128, src128, K);
+  if ((((uintptr_t)dst128 | (uintptr_t)src128) & 7) == 0)
+    k_psf_z<true><<<nsm * 8, ZW * 32, 0, s>>>(dst128, src128, K);
+  else
+    k_psf_z<false><<<nsm * 8, ZW * 32, 0, s>>>(dst128, src128, K);
   k_psf_line<1><<<NB_IMY * SEGN, NB_COLW, 0, s>>>(tmp128, dst128, K);
   k_psf_line<2><<<NB_IMX * SEGN, NB_COLW, 0, s>>>(dst128, tmp128, K);
   NB_CUDA(cudaGetLastError());

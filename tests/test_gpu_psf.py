@@ -115,3 +115,23 @@ def test_psf_passes_match_float64(params, cuda_device, alias):
     want = want[0, 0]
     assert float(((got - want).abs() / want).max()) <= 3e-6
     assert not out.reshape(-1, 128)[:, 127].any()
+
+
+@pytest.mark.parametrize('off_src,off_dst', [(1, 0), (0, 1), (1, 3), (2, 2)])
+def test_psf_of_images_at_any_float(params, cuda_device, off_src, off_dst):
+    """Images that do not start on an 8-byte boundary: the same bits, in place or not."""
+    k = np.ascontiguousarray(_kernels(params)['asym'], np.float32)
+    img = torch.from_numpy(phantoms.random_ellipsoids(4)).to(cuda_device)
+    x = petprj.to_col128(img).reshape(-1)
+    lib, st, n = _lib.load(), stream_ptr(cuda_device), x.numel()
+    buf = lambda: torch.full((n + 4,), -1.0, device=cuda_device)  # noqa: E731
+    want, tmp, src, dst = torch.empty_like(x), torch.empty_like(x), buf(), buf()
+    src[off_src:off_src + n] = x
+    run = lambda d, s: _lib.check(lib.nb_psf_col128(dev_ptr(d), dev_ptr(s), k.ctypes.data,  # noqa: E731
+                                                    dev_ptr(tmp), st))
+    run(want, x)
+    run(dst[off_dst:], src[off_src:])
+    assert torch.equal(dst[off_dst:off_dst + n], want) and torch.equal(src[off_src:off_src + n], x)
+    run(src[off_src:], src[off_src:])
+    assert torch.equal(src[off_src:off_src + n], want)
+    assert (dst[:off_dst] == -1).all() and (dst[off_dst + n:] == -1).all()
