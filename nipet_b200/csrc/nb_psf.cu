@@ -130,13 +130,20 @@ extern "C" int nb_psf_col128(float *dst128, const float *src128, const float *kr
   int dev = 0, nsm = 148;
   NB_CUDA(cudaGetDevice(&dev));
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  // z: src -> dst (dst may be src), x: dst -> tmp, y: tmp -> dst: the reference's order
-  if ((((uintptr_t)dst128 | (uintptr_t)src128) & 7) == 0)
-    k_psf_z<true><<<nsm * 8, ZW * 32, 0, s>>>(dst128, src128, K);
+  // z: src -> dst (dst may be src), x: dst -> tmp, y: tmp -> dst: the reference's order.  Images
+  // that overlap otherwise go by way of tmp and are copied at the end
+  const uintptr_t us = (uintptr_t)src128, ud = (uintptr_t)dst128;
+  const bool apart = us == ud || (us < ud ? ud - us : us - ud) >= sizeof(float) * NB_IMG_COL128;
+  float *one = apart ? dst128 : tmp128, *two = apart ? tmp128 : dst128;
+  if ((((uintptr_t)one | us) & 7) == 0)
+    k_psf_z<true><<<nsm * 8, ZW * 32, 0, s>>>(one, src128, K);
   else
-    k_psf_z<false><<<nsm * 8, ZW * 32, 0, s>>>(dst128, src128, K);
-  k_psf_line<1><<<NB_IMY * SEGN, NB_COLW, 0, s>>>(tmp128, dst128, K);
-  k_psf_line<2><<<NB_IMX * SEGN, NB_COLW, 0, s>>>(dst128, tmp128, K);
+    k_psf_z<false><<<nsm * 8, ZW * 32, 0, s>>>(one, src128, K);
+  k_psf_line<1><<<NB_IMY * SEGN, NB_COLW, 0, s>>>(two, one, K);
+  k_psf_line<2><<<NB_IMX * SEGN, NB_COLW, 0, s>>>(one, two, K);
+  if (!apart)
+    NB_CUDA(cudaMemcpyAsync(dst128, tmp128, sizeof(float) * NB_IMG_COL128,
+                            cudaMemcpyDeviceToDevice, s));
   NB_CUDA(cudaGetLastError());
   return NB_OK;
 }

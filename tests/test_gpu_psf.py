@@ -135,3 +135,18 @@ def test_psf_of_images_at_any_float(params, cuda_device, off_src, off_dst):
     run(src[off_src:], src[off_src:])
     assert torch.equal(src[off_src:off_src + n], want)
     assert (dst[:off_dst] == -1).all() and (dst[off_dst + n:] == -1).all()
+
+
+@pytest.mark.parametrize('shift', [128, -128, 3])
+def test_psf_of_overlapping_images(params, cuda_device, shift):
+    """A source and a destination that overlap in part: the same bits."""
+    k = np.ascontiguousarray(_kernels(params)['asym'], np.float32)
+    x = petprj.to_col128(torch.from_numpy(phantoms.random_ellipsoids(4)).to(cuda_device)).reshape(-1)
+    lib, st, n, a = _lib.load(), stream_ptr(cuda_device), x.numel(), abs(shift)
+    want, tmp = torch.empty_like(x), torch.empty_like(x)
+    buf = torch.zeros(n + a, device=cuda_device)
+    src, dst = (buf[:n], buf[a:]) if shift > 0 else (buf[a:], buf[:n])
+    src.copy_(x)
+    for d, s in ((want, x), (dst, src)):
+        _lib.check(lib.nb_psf_col128(dev_ptr(d), dev_ptr(s), k.ctypes.data, dev_ptr(tmp), st))
+    assert torch.equal(dst, want)
