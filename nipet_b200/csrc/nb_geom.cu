@@ -434,7 +434,8 @@ static int ring_of(float z) {
 
 // Slots of a set of rays (those of all ring pairs, or of a reduced range): the direct planes
 // two to a slot, then the pairs by ring difference and ring.  False if the rays are not ring
-// pairs of the mMR's rings with both directions, once each.
+// pairs of the mMR's rings with both directions, once each (ring fronts at (i - 32) * 0.40625 cm,
+// differences 1 .. 60).
 static bool make_slots(const std::vector<nb_ray> &rays, std::vector<nb_slot> &slots) {
   std::map<std::pair<int, int>, nb_slot> pair;  // (d, r0)
   std::map<int, const nb_ray *> direct;
@@ -543,21 +544,10 @@ extern "C" int nb_geom_create(int device, const float *crs, int ncrs, const int1
     }
     rays[r] = R;
   }
-  std::vector<nb_slot> slots;
-  if (!make_slots(rays, slots)) {
-    free(g->h_s2c);
-    free(g);
-    nb_set_error_msg("nb_geom_create: li2rng is not the mMR's ring pairs (ring fronts at "
-                     "(i - 32) * 0.40625 cm, differences 1 .. %d, each pair once)", NB_MAXRD);
-    return NB_ERR_ARG;
-  }
-  g->nslots = (int)slots.size();
-  std::vector<int16_t> bin11(NB_NSN11 * 8, -1);
+  std::vector<int16_t> ray11(NB_NSN11 * 8, -1), bin11(NB_NSN11 * 8, -1);  // by ray, by slot
   std::vector<int> cnt11(NB_NSN11, 0), cnt1(NB_NSN1, 0);
-  for (int r = 0; r < 2 * g->nslots; r++) {
-    const nb_slot &S = slots[r / 2];
-    const int o = r & 1 ? S.o11B : S.o11A, o1 = r & 1 ? S.o1B : S.o1A;
-    if (o < 0) continue;
+  for (int r = 0; r < NB_NRAYS; r++) {
+    const int o = rays[r].out11, o1 = rays[r].out1;
     if (cnt11[o] >= 8 || cnt1[o1]++) {
       free(g->h_s2c);
       free(g);
@@ -567,7 +557,17 @@ extern "C" int nb_geom_create(int device, const float *crs, int ncrs, const int1
         nb_set_error_msg("nb_geom_create: span-1 sinogram %d mapped twice", o1);
       return NB_ERR_ARG;
     }
-    bin11[o * 8 + cnt11[o]++] = (int16_t)r;
+    ray11[o * 8 + cnt11[o]++] = (int16_t)r;
+  }
+  // rays that are not the mMR's ring pairs go without slots and crossing schedules, through the
+  // step-by-step kernel (k_walk_any)
+  std::vector<nb_slot> slots;
+  if (!make_slots(rays, slots)) slots.clear();
+  g->nslots = (int)slots.size();
+  std::fill(cnt11.begin(), cnt11.end(), 0);
+  for (int r = 0; r < 2 * g->nslots; r++) {
+    const int o = r & 1 ? slots[r / 2].o11B : slots[r / 2].o11A;
+    if (o >= 0) bin11[o * 8 + cnt11[o]++] = (int16_t)r;
   }
 
   int st = NB_OK;
@@ -594,7 +594,7 @@ extern "C" int nb_geom_create(int device, const float *crs, int ncrs, const int1
   ALLOC(g->d_tt, sizeof(float) * NB_N_TT * (size_t)naw);
   ALLOC(g->d_rays, sizeof(nb_ray) * NB_NRAYS);
   ALLOC(g->d_bin11, sizeof(int16_t) * NB_NSN11 * 8);
-  ALLOC(g->d_slots, sizeof(nb_slot) * g->nslots);
+  ALLOC(g->d_slots, sizeof(nb_slot) * (g->nslots + 1));
   ALLOC(g->d_rec_off, sizeof(uint32_t) * (naw + 1));
   ALLOC(g->d_scratch128, sizeof(float) * NB_IMG_COL128);
   ALLOC(g->d_err, sizeof(int));
@@ -650,11 +650,11 @@ extern "C" int nb_geom_create(int device, const float *crs, int ncrs, const int1
       goto fail;
     }
     std::vector<uint32_t> off(naw + 1);
-    if (e == cudaSuccess) {
+    if (e == cudaSuccess && g->nslots) {
       k_sched<false><<<naw, 64>>>(g->d_hdr, g->d_st, g->d_rec_off, nullptr, nullptr, g->d_err);
       e = cudaMemcpy(off.data(), g->d_rec_off, sizeof(uint32_t) * naw, cudaMemcpyDeviceToHost);
     }
-    if (e == cudaSuccess) {
+    if (e == cudaSuccess && g->nslots) {
       uint64_t tot = 0;  // 16-byte units: 1.2e8 for the mMR
       for (int i = 0; i <= naw; i++) {
         const uint32_t sz = i < naw ? off[i] : 0;
@@ -677,18 +677,20 @@ extern "C" int nb_geom_create(int device, const float *crs, int ncrs, const int1
         e = cudaMemcpy(g->d_rec_off, off.data(), sizeof(uint32_t) * (naw + 1),
                        cudaMemcpyHostToDevice);
     }
-    if (e == cudaSuccess) {
+    if (e == cudaSuccess && g->nslots) {
       k_sched<true><<<naw, 64>>>(g->d_hdr, g->d_st, nullptr, g->d_rec_off, g->d_rec, g->d_err);
       e = cudaMemcpy(&herr, g->d_err, sizeof(int), cudaMemcpyDeviceToHost);
     }
     if (e == cudaSuccess) e = cudaMemset(g->d_err, 0, sizeof(int));
+    if (herr) g->nslots = 0;  // schedules over capacity: step by step
+    if (e == cudaSuccess && !g->nslots) {
+      cudaFree(g->d_rec);
+      g->d_rec = nullptr;
+      e = cudaMemcpy(g->d_bin11, ray11.data(), sizeof(int16_t) * NB_NSN11 * 8,
+                     cudaMemcpyHostToDevice);
+    }
     if (e != cudaSuccess) {
       st = nb_cuda_fail(e, "nb_geom_create walk check and schedules", __FILE__, __LINE__);
-      goto fail;
-    }
-    if (herr) {
-      nb_set_error_msg("nb_geom_create: crossing schedules over capacity (%d)", herr);
-      st = NB_ERR_DATA;
       goto fail;
     }
   }
@@ -776,10 +778,7 @@ extern "C" int nb_rings_create(nb_geom *g, int rs, int re, const float *li2rng,
     used[R.out1] = 1;
   }
   std::vector<nb_slot> slots;
-  if (!make_slots(sel, slots)) {
-    nb_set_error_msg("nb_rings_create: the ring pairs are not distinct pairs of both directions");
-    return NB_ERR_ARG;
-  }
+  if (!g->nslots || !make_slots(sel, slots)) slots.clear();  // step by step, as the geometry
   NB_CUDA(cudaSetDevice(g->device));
   nb_rings *rr = (nb_rings *)calloc(1, sizeof(nb_rings));
   if (!rr) return NB_ERR_NOMEM;
@@ -790,12 +789,16 @@ extern "C" int nb_rings_create(nb_geom *g, int rs, int re, const float *li2rng,
   rr->vz0 = 2 * rs;
   rr->nvz = 2 * n - 1;
   rr->nslots = (int)slots.size();
-  cudaError_t e = cudaMalloc(&rr->d_slots, sizeof(nb_slot) * slots.size());
+  cudaError_t e = cudaMalloc(&rr->d_slots, sizeof(nb_slot) * (slots.size() + 1));
   if (e == cudaSuccess)
     e = cudaMemcpy(rr->d_slots, slots.data(), sizeof(nb_slot) * slots.size(),
                    cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMalloc(&rr->d_rays, sizeof(nb_ray) * nsino);
+  if (e == cudaSuccess)
+    e = cudaMemcpy(rr->d_rays, sel.data(), sizeof(nb_ray) * nsino, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     cudaFree(rr->d_slots);
+    cudaFree(rr->d_rays);
     free(rr);
     return nb_cuda_fail(e, "nb_rings_create upload", __FILE__, __LINE__);
   }
@@ -807,6 +810,7 @@ extern "C" int nb_rings_destroy(nb_rings *rr) {
   if (!rr) return NB_OK;
   cudaSetDevice(rr->device);
   cudaFree(rr->d_slots);
+  cudaFree(rr->d_rays);
   free(rr);
   return NB_OK;
 }

@@ -68,8 +68,10 @@ struct nb_geom {
   unsigned char *d_rec;  // crossing schedules of all LORs
   uint32_t *d_rec_off;   // [naw + 1] start of a LOR's record, in 16-byte units
   nb_slot *d_slots;      // [nslots] ray pairs
-  int nslots;
-  int16_t *d_bin11;  // [837][8] rays (2 slot + direction) of each span-11 sinogram (-1 padded)
+  int nslots;        // 0: rays that are not the mMR's ring pairs, or whose crossings do not fit the
+                     // schedules; every projection runs step by step over d_rays (k_walk_any)
+  int16_t *d_bin11;  // [837][8] rays of each span-11 sinogram (-1 padded): 2 slot + direction, or
+                     // the index in d_rays without slots
   float *d_scratch128;   // one col128 image (reference-layout entry points)
   int *d_err;            // device error flag
   float *d_one;          // the constant 1.0f (randoms factor of a single-image batch)
@@ -91,7 +93,8 @@ struct nb_rings {
   int nrays;         // rays of the range = its span-1 sinograms
   int vz0, nvz;
   nb_slot *d_slots;  // [nslots] the range's ray pairs, o1A / o1B the range's sinograms
-  int nslots;
+  int nslots;        // 0: step by step over d_rays
+  nb_ray *d_rays;    // [nrays]
 };
 
 // ---- tracing: an NVTX range around a C-ABI call (header-only NVTX3: without a profiler

@@ -295,6 +295,8 @@ extern "C" int nb_fprj_rings(nb_geom *g, const nb_rings *rr, float *sino, const 
   nbw::WalkArgs a = nb_walk_args(g, subs, nprj, 1, 1, 1);
   a.slots = rr->d_slots;
   a.nslots = rr->nslots;
+  a.rays = rr->d_rays;
+  a.nrays = rr->nrays;
   a.nout = rr->nrays;
   a.att = att;
   a.img = g->d_scratch128;
@@ -315,6 +317,8 @@ extern "C" int nb_bprj_rings(nb_geom *g, const nb_rings *rr, float *im, const fl
   nbw::WalkArgs a = nb_walk_args(g, subs, nprj, 1, 1, 1);
   a.slots = rr->d_slots;
   a.nslots = rr->nslots;
+  a.rays = rr->d_rays;
+  a.nrays = rr->nrays;
   a.nout = rr->nrays;
   a.bimg = g->d_scratch128;
   a.sino_in = sino;

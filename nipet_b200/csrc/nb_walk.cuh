@@ -80,6 +80,8 @@ struct WalkArgs {
   const uint32_t *rec_off;    // [naw + 1] start of a LOR's record, in 16-byte units
   const nb_slot *slots;
   int nslots;
+  const nb_ray *rays;         // [nrays], for k_walk_any (nslots 0)
+  int nrays;
   const int16_t *bin11;       // [837][8] rays (2 * slot + direction) of each span-11 sinogram
   const int32_t *subs;
   int nprj, naw, ngroups, nrep;
