@@ -192,33 +192,73 @@ __global__ void k_expand_steps(const float *__restrict__ tt, const unsigned char
   hdr[idx] = make_float4(t[5], t[7], t[6], __int_as_float(n));
 }
 
-// Walks every ray of every LOR once at geometry creation and counts axial positions outside
-// [0, 127]: the projector indexes shared memory by the plane without clamping.  z = 127 is one
-// plane above the image; it maps to a column's zero padding slot (reads 0, back projections
-// into it are discarded).  In the mMR geometry exactly one ray step reaches it (the last step
-// of rings 59->63 on LOR 24839).  One block per LOR.
-__global__ void k_check_walk(const float4 *__restrict__ hdr, const float *__restrict__ st,
-                             const nb_ray *__restrict__ rays, int naw, int *bad) {
+// Walks every ray of every LOR once at geometry creation (one block per LOR):
+//   out[0]  axial positions outside [0, 127]: the projector indexes shared memory by the plane
+//           without clamping.  z = 127 is one plane above the image; it maps to a column's zero
+//           padding slot (reads 0, back projections into it are discarded).  In the mMR geometry
+//           exactly one ray step reaches it (the last step of rings 59->63 on LOR 24839).
+//   out[1]  the longest piece of a walk in cm, as float bits (a crossing that the reference takes
+//           a step late, when a ray passes two planes in one, has a negative piece)
+//   out[2]  the largest sum of |weight| that the rays of a LOR bring to one plane in one step, as
+//           float bits, of the LORs with such crossings; elsewhere every weight is in [0, 1] and
+//           at most 242 rays meet in a plane (121 ring differences and directions, of each of
+//           which one is in a plane, and one more enters it in the step)
+__global__ void __launch_bounds__(256) k_check_walk(const float4 *__restrict__ hdr,
+                                                    const float *__restrict__ st,
+                                                    const nb_ray *__restrict__ rays, int naw,
+                                                    unsigned *out) {
+  constexpr int CH = 64;
+  __shared__ float acc[CH][128];
   const int lor = blockIdx.x;
   if (lor >= naw) return;
   const float4 h = hdr[lor];
   const int n = __float_as_int(h.w);
-  int nbad = 0;
-  for (int ray = threadIdx.x; ray < NB_NRAYS; ray += blockDim.x) {
+  const float *t = st + (size_t)lor * NB_STEP_STRIDE;
+  // the walk of a ray; piece(step, plane, length, step's length)
+  auto walk = [&](int ray, int end, auto piece) {
     nb_axial A;
     nb_axial_setup(rays[ray], h.y, h.x, h.z, A);
     int w = A.w;
-    float tzc = A.tzc;
-    if (w < 0 || w > NB_IMZ) nbad++;
-    for (int k = 0; k < n; k++) {
-      if (st[(size_t)lor * NB_STEP_STRIDE + k] > tzc) {
+    float tzc = A.tzc, tp = h.x;
+    piece(-1, w, 0.f, 0.f);
+    for (int k = 0; k < end; k++) {
+      const float tn = t[k], lt = __fsub_rn(tn, tp);
+      if (tn > tzc) {
+        piece(k, w, __fsub_rn(tzc, tp), lt);
         w += A.dir;
+        piece(k, w, __fsub_rn(tn, tzc), lt);
         tzc = __fadd_rn(tzc, A.dtz);
-        if (w < 0 || w > NB_IMZ) nbad++;
+      } else {
+        piece(k, w, lt, lt);
       }
+      tp = tn;
     }
+  };
+  unsigned nbad = 0;
+  float longest = 0.f;
+  bool late = false;
+  for (int ray = threadIdx.x; ray < NB_NRAYS; ray += blockDim.x)
+    walk(ray, n, [&](int, int w, float len, float lt) {
+      nbad += w < 0 || w > NB_IMZ;
+      longest = fmaxf(longest, fabsf(len));
+      late |= fabsf(len) > lt;
+    });
+  if (nbad) atomicAdd(out, nbad);
+  atomicMax(out + 1, __float_as_uint(longest));
+  if (__syncthreads_or(nbad) || !__syncthreads_or(late)) return;
+  float most = 0.f;
+  for (int c = 0; c < n; c += CH) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < CH * 128; i += blockDim.x) acc[i >> 7][i & 127] = 0.f;
+    __syncthreads();
+    for (int ray = threadIdx.x; ray < NB_NRAYS; ray += blockDim.x)
+      walk(ray, min(n, c + CH), [&](int k, int w, float len, float lt) {
+        if (k >= c && lt > 0.f) atomicAdd(&acc[k - c][w], fabsf(len) / lt);
+      });
+    __syncthreads();
+    for (int i = threadIdx.x; i < CH * 128; i += blockDim.x) most = fmaxf(most, acc[i >> 7][i & 127]);
   }
-  if (nbad) atomicAdd(bad, nbad);
+  atomicMax(out + 2, __float_as_uint(most));
 }
 
 // ---------------------------------------------------------------------------------------
@@ -638,17 +678,29 @@ extern "C" int nb_geom_create(int device, const float *crs, int ncrs, const int1
       st = NB_ERR_DEVICE;
       goto fail;
     }
-    // walk check (the projector indexes shared memory by the plane), then the schedules:
-    // count, place, fill
-    cudaMemset(g->d_err, 0, sizeof(int));
-    k_check_walk<<<naw, 256>>>(g->d_hdr, g->d_st, g->d_rays, naw, g->d_err);
-    int nbad = 0;
-    cudaError_t e = cudaMemcpy(&nbad, g->d_err, sizeof(int), cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess && nbad) {
-      nb_set_error_msg("nb_geom_create: %d ray positions leave the axial FOV", nbad);
+    // walk check, then the schedules: count, place, fill
+    unsigned *d_chk = (unsigned *)d_tv, chk[3] = {0u, 0u, 0u};  // (the tables are expanded)
+    cudaError_t e = cudaMemset(d_chk, 0, sizeof(chk));
+    if (e == cudaSuccess) {
+      k_check_walk<<<naw, 256>>>(g->d_hdr, g->d_st, g->d_rays, naw, d_chk);
+      e = cudaMemcpy(chk, d_chk, sizeof(chk), cudaMemcpyDeviceToHost);
+    }
+    if (e == cudaSuccess && chk[0]) {
+      nb_set_error_msg("nb_geom_create: %u ray positions leave the axial FOV", chk[0]);
       st = NB_ERR_DATA;
       goto fail;
     }
+    float longest, most;
+    memcpy(&longest, &chk[1], sizeof(float));
+    memcpy(&most, &chk[2], sizeof(float));
+    if (e == cudaSuccess && !(longest < 64.f)) {
+      nb_set_error_msg("nb_geom_create: walk segments too long (%g cm)", (double)longest);
+      st = NB_ERR_DATA;
+      goto fail;
+    }
+    // a plane's sum of integers below 2^23 each leaves int32 above 255 of them (the mMR: 105.8 where
+    // crossings are late, 242 at the most elsewhere)
+    if (most > 255.f) g->nslots = 0;
     std::vector<uint32_t> off(naw + 1);
     if (e == cudaSuccess && g->nslots) {
       k_sched<false><<<naw, 64>>>(g->d_hdr, g->d_st, g->d_rec_off, nullptr, nullptr, g->d_err);

@@ -34,9 +34,10 @@
 // is not finite, or above 2^100).  The fused mode leaves out those whose ratio does not need them:
 // nothing counted, or randoms above 2^20 quanta.  Every bin is then good to 1e-5 of its value, but
 // for slivers of a step (a fraction is good to 2^-25 of the step).
-//   In the back projection a ray's value is rounded once, to 2^-22 of the LOR's largest, its two
-// parts of a crossing sum to it exactly, and at most 242 rays meet in a plane, so no sum leaves
-// int32.  An image with a value that is not finite goes to the voxels ray by ray in float32.
+//   In the back projection a ray's value is rounded once, by at most 2^-23 of the LOR's largest,
+// and its two parts of a crossing sum to it exactly.  The weights that meet in a plane in one step
+// sum to 255 at the most (checked when the geometry is made: a late crossing has weights outside
+// [0, 1]) and values are below 2^23, so no sum leaves int32.  An image with a value that is not finite goes to the voxels ray by ray in float32.
 //
 // Jobs.  One block per (LOR, image group); a finished block takes over a block that has not
 // started (cluster launch control), so LORs of 10 to 404 steps even out over the SMs and the

@@ -4,7 +4,7 @@ wrong, against the FP64 oracle.
 Bars: forward, a ray's fraction terms are float32 (relative 2^-24 each, up to ~35 of them and
 one conversion per chunk) and its integer part is good to 2^-29 of its chunk's integral, so
 1e-6 relative L2 per projection, 1e-5 per bin above 1e-3 of the maximum, and exact zeros where
-the oracle has zeros; backward, values are rounded to 2^-23 of the LOR's largest: 1e-6."""
+the oracle has zeros; backward, values are rounded by up to 2^-23 of the LOR's largest: 1e-6."""
 import numpy as np
 import pytest
 import torch
@@ -239,7 +239,7 @@ def test_walk_faint_background(env, nimg, value):
 def test_walk_pairs_with_own_crossings(env):
     """LORs on which a first or last plane boundary of some ring pairs rounds to the next one, so
     that they cross planes at other floats than the rest of their difference.  Bar: each ray's
-    value is rounded to 2^-22 of the largest, and a voxel's rays and its float32 sum, 2e-6."""
+    value is rounded by up to 2^-23 of the largest, and a voxel's rays and its float32 sum, 2e-6."""
     p, orc = env['p'], env['orc']
     r = np.random.default_rng(4)
     for lor in (11712, 13025, 14216, 17924, 32699, 35929, 45722, 53209, 64252):
