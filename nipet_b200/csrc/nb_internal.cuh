@@ -126,6 +126,14 @@ int nb_cuda_fail(cudaError_t e, const char *what, const char *file, int line);
     }                                                                                          \
   } while (0)
 
+// multiprocessors of the current device
+static inline int nb_sms() {
+  int dev = 0, nsm = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess)
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  return nsm;
+}
+
 // Check the device error flag of a handle after synchronising `stream` (debug/validation
 // paths only; the hot entry points do not synchronise).
 int nb_check_device_flag(nb_geom *g, cudaStream_t stream);

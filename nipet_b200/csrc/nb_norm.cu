@@ -152,7 +152,7 @@ extern "C" int nb_norm(float *sng, const float *geo, int ngeo, const float *cinf
   cp(d_nos, sn1_sn11no, NB_NSN1);
   if (st_ == NB_OK) {
     k_norm_crystal<<<(NR * NCF + 255) / 256, 256, 0, st>>>(d_tab, d_ceff, d_dtp, d_dtnp, d_bck);
-    k_norm<<<148 * 8, 256, 0, st>>>(sng, d_geo, d_cinf, d_tab, d_axe1, d_axf1, d_rno, d_s11, d_pl,
+    k_norm<<<nb_sms() * 8, 256, 0, st>>>(sng, d_geo, d_cinf, d_tab, d_axe1, d_axf1, d_rno, d_s11, d_pl,
                                     d_nos, d_aw, nout, span);
     if (cudaGetLastError() != cudaSuccess)
       st_ = nb_cuda_fail(cudaGetLastError(), "nb_norm launch", __FILE__, __LINE__);

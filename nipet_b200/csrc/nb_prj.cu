@@ -2,6 +2,8 @@
 // the sinogram gap kernels.  The projector kernel itself is in nb_walk.cuh.
 #include <math.h>
 
+#include <algorithm>
+
 #include "nb_axial.cuh"
 #include "nb_internal.cuh"
 #include "nb_walk.cuh"
@@ -176,7 +178,7 @@ extern "C" int nb_im_to_col128(float *im128, const float *im, int nimg, void *st
   NB_REQUIRE(im128 && im && nimg > 0, "nb_im_to_col128: bad arguments");
   const int ncols = NB_NCOL * nimg;
   if ((((uintptr_t)im128 | (uintptr_t)im) & 15) == 0)
-    k_to_col128<<<ncols / CV < 148 * 8 ? ncols / CV : 148 * 8, 256, 0, (cudaStream_t)stream>>>(
+    k_to_col128<<<std::min(ncols / CV, nb_sms() * 8), 256, 0, (cudaStream_t)stream>>>(
         im128, im, ncols);
   else
     k_to_col128_any<<<(ncols * 32 + 255) / 256, 256, 0, (cudaStream_t)stream>>>(im128, im, ncols);
@@ -188,7 +190,7 @@ extern "C" int nb_col128_to_im(float *im, const float *im128, int nimg, void *st
   NB_REQUIRE(im128 && im && nimg > 0, "nb_col128_to_im: bad arguments");
   const int ncols = NB_NCOL * nimg;
   if ((((uintptr_t)im128 | (uintptr_t)im) & 15) == 0)
-    k_from_col128<<<ncols / CV < 148 * 8 ? ncols / CV : 148 * 8, 256, 0, (cudaStream_t)stream>>>(
+    k_from_col128<<<std::min(ncols / CV, nb_sms() * 8), 256, 0, (cudaStream_t)stream>>>(
         im, im128, ncols);
   else
     k_from_col128_any<<<(ncols * 32 + 255) / 256, 256, 0, (cudaStream_t)stream>>>(im, im128, ncols);
@@ -462,7 +464,7 @@ extern "C" int nb_remgaps(float *sng, const float *sino, int snno, const int32_t
                           void *stream) {
   NB_RANGE("nb_remgaps");
   NB_REQUIRE(sng && sino && aw2ali && snno > 0, "nb_remgaps: bad arguments");
-  k_gaps<float, true><<<148 * 16, 256, 0, (cudaStream_t)stream>>>(sng, sino, snno, aw2ali);
+  k_gaps<float, true><<<nb_sms() * 16, 256, 0, (cudaStream_t)stream>>>(sng, sino, snno, aw2ali);
   NB_CUDA(cudaGetLastError());
   return NB_OK;
 }
@@ -470,7 +472,7 @@ extern "C" int nb_remgaps(float *sng, const float *sino, int snno, const int32_t
 extern "C" int nb_remgaps_u16(uint16_t *sng, const uint16_t *sino, int snno,
                               const int32_t *aw2ali, void *stream) {
   NB_REQUIRE(sng && sino && aw2ali && snno > 0, "nb_remgaps_u16: bad arguments");
-  k_gaps<uint16_t, true><<<148 * 16, 256, 0, (cudaStream_t)stream>>>(sng, sino, snno, aw2ali);
+  k_gaps<uint16_t, true><<<nb_sms() * 16, 256, 0, (cudaStream_t)stream>>>(sng, sino, snno, aw2ali);
   NB_CUDA(cudaGetLastError());
   return NB_OK;
 }
@@ -481,7 +483,7 @@ extern "C" int nb_putgaps(float *sino, const float *sng, int snno, const int32_t
   NB_REQUIRE(sng && sino && aw2ali && snno > 0, "nb_putgaps: bad arguments");
   NB_CUDA(cudaMemsetAsync(sino, 0, sizeof(float) * (size_t)snno * NB_NSBINANG,
                           (cudaStream_t)stream));
-  k_gaps<float, false><<<148 * 16, 256, 0, (cudaStream_t)stream>>>(sino, sng, snno, aw2ali);
+  k_gaps<float, false><<<nb_sms() * 16, 256, 0, (cudaStream_t)stream>>>(sino, sng, snno, aw2ali);
   NB_CUDA(cudaGetLastError());
   return NB_OK;
 }

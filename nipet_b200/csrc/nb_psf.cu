@@ -127,9 +127,7 @@ extern "C" int nb_psf_col128(float *dst128, const float *src128, const float *kr
   for (int a = 0; a < 3; a++)
     for (int i = 0; i < KL; i++) K.k[a][i] = krnl[a * KL + i];
   cudaStream_t s = (cudaStream_t)stream;
-  int dev = 0, nsm = 148;
-  NB_CUDA(cudaGetDevice(&dev));
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const int nsm = nb_sms();
   // z: src -> dst (dst may be src), x: dst -> tmp, y: tmp -> dst: the reference's order.  Images
   // that overlap otherwise go by way of tmp and are copied at the end
   const uintptr_t us = (uintptr_t)src128, ud = (uintptr_t)dst128;

@@ -3,8 +3,7 @@ wrong, against the FP64 oracle.
 
 Bars: forward, a ray's fraction terms are float32 (relative 2^-24 each, up to ~35 of them and
 one conversion per chunk) and its integer part is good to 2^-29 of its chunk's integral, so
-1e-6 relative L2 per projection, 1e-5 per bin above 1e-3 of the maximum, and exact zeros where
-the oracle has zeros; backward, values are rounded by up to 2^-23 of the LOR's largest: 1e-6."""
+1e-6 relative L2 per projection, 1e-5 per bin, and exact zeros where the oracle has zeros; backward, values are rounded by up to 2^-23 of the LOR's largest: 1e-6."""
 import numpy as np
 import pytest
 import torch
@@ -47,10 +46,12 @@ def _image(seed):
     return im
 
 
-def _check_fwd(got, want):
+def _check_fwd(got, want, peak):
     assert np.linalg.norm(got - want) <= 1e-6 * np.linalg.norm(want)
     big = want >= 1e-3 * want.max()
     assert (np.abs(got - want)[big] / want[big]).max() <= 1e-5
+    # every bin, with a sliver of a step besides (test_walk_weak_planes)
+    assert (np.abs(got - want) <= 1e-5 * want + 0.3 * 2.0 ** -25 * peak).all()
     assert not got[want == 0].any()
 
 
@@ -68,7 +69,7 @@ def test_walk_edges(env, span, nimg):
     back = prj.backproject(torch.from_numpy(si).cuda()).cpu().numpy().astype(np.float64)
     prj.check()
     for i in range(nimg):
-        _check_fwd(got[i], orc.fprj(ims[i], subs, span=span))
+        _check_fwd(got[i], orc.fprj(ims[i], subs, span=span), ims[i].max())
         want = orc.bprj(si[i], subs, span=span)
         assert np.linalg.norm(back[i] - want) <= 1e-6 * np.linalg.norm(want)
         assert not back[i][want == 0].any()
