@@ -223,6 +223,96 @@ static __device__ __forceinline__ bool mask_meets(const unsigned *mask, int lo, 
   return hit;
 }
 
+// A ray of the slots as the reference's axial set-up sees it
+static __device__ __forceinline__ void slot_axial(const nb_slot *slots, int ray, const float4 &h,
+                                                  nb_axial &A) {
+  const uint32_t zz = slots[ray >> 1].zzd;
+  const int d = (int)(zz >> 16);
+  nb_axial_setup(nb_ring_pair((int)((d ? zz : zz >> (ray & 1) * 8) & 255u) / 2, d,
+                              d ? 1 + (ray & 1) : 0), h.y, h.x, h.z, A);
+}
+
+// Up to NT / 8 rays of `list` step by step in float32, straight from the image: a ray in eight
+// parts, whose lanes find their start by the crossings alone.  (Staged as below they would wait
+// for five rounds of copies: 33 LORs, which take 22 us, took 30 us longer.)
+template <int BS, int NT>
+static __device__ __noinline__ void walk_few(const float *gimg, size_t stride, bool natural,
+                                             const int32_t *scol, const float *sst, int n,
+                                             const float4 h, const nb_slot *slots,
+                                             const uint16_t *list, int count, float *vals) {
+  constexpr int U = 4;                        // steps whose reads are in flight together
+  const int tid = threadIdx.x;
+  const bool live = tid / 8 < count;
+  const int ray = list[live ? tid / 8 : 0], part = ((n + 7) / 8 + U - 1) / U * U;
+  const int s0 = min(n, (tid & 7) * part), s1 = live ? min(n, s0 + part) : 0;
+  nb_axial A;
+  slot_axial(slots, ray, h, A);
+  int z = A.w;
+  float tp = h.x, tzc = A.tzc, acc[BS];
+  for (int s = 0; s < (live ? s0 : 0); s++) {
+    tp = sst[s];
+    if (tp > tzc) {
+      z += A.dir;
+      tzc = __fadd_rn(tzc, A.dtz);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < BS; k++) acc[k] = 0.f;
+  for (int s = s0; s < s1; s += U) {
+    float v0[U][BS], v1[U][BS], w0[U], w1[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      w0[u] = w1[u] = 0.f;
+#pragma unroll
+      for (int k = 0; k < BS; k++) v0[u][k] = v1[u][k] = 0.f;
+      if (s + u >= s1) continue;
+      const float tn = sst[s + u];
+      const float *c = gimg + (size_t)scol[s + u] * stride;
+      if (!natural || z < NB_IMZ) ldg_v<BS>(c + (natural ? z : nb_zi(z) * BS), v0[u]);
+      w0[u] = __fsub_rn(fminf(tn, tzc), tp);
+      if (tn > tzc) {
+        z += A.dir;
+        if (!natural || z < NB_IMZ) ldg_v<BS>(c + (natural ? z : nb_zi(z) * BS), v1[u]);
+        w1[u] = __fsub_rn(tn, tzc);
+        tzc = __fadd_rn(tzc, A.dtz);
+      }
+      tp = tn;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+#pragma unroll
+      for (int k = 0; k < BS; k++) acc[k] = fmaf(w1[u], v1[u][k], fmaf(w0[u], v0[u][k], acc[k]));
+  }
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+    for (int k = 0; k < BS; k++) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+  if (live && (tid & 7) == 0)
+#pragma unroll
+    for (int k = 0; k < BS; k++) vals[ray * BS + k] = acc[k];
+}
+
+// Fused mode: has the LOR a bin whose ratio could need more than 2^20 quanta per chunk?  Not where
+// nothing was counted, nor where the randoms outweigh them.  (Asked for the bins in order, before
+// the rays: late iterates of noisy data have weak rays on every LOR and no such bin.)
+template <int BS, int NT>
+static __device__ __noinline__ bool bins_matter(const WalkArgs &a, const float *sthr, int g, int lor) {
+  bool some = false;
+  const size_t row = (size_t)lor * a.nout;
+#pragma unroll
+  for (int k = 0; k < BS; k++) {
+    const int rep = g * BS + k;
+    if (rep >= a.nrep) break;
+    const float q = sthr[k], scale = a.rscale[rep];
+    const uint16_t *y = a.psng + (size_t)rep * a.naw * a.nout + row;
+    some |= q == __int_as_float(0x7f800000);
+#pragma unroll 4
+    for (int o = threadIdx.x; o < a.nout; o += NT)
+      some |= (__ldg(y + o) != 0) & !(scale * __ldg(a.rs + row + o) >= q * WEAK_QUANTA);
+  }
+  return some;
+}
+
 // Walks the rays of a LOR whose fixed-point sums (vals, [4096][BS]) are too few quanta to be good
 // to float32's precision again: step by step in float32, as the reference does, from columns
 // staged in shared memory (40 KB at a time).  All threads; false if there was none to walk.
@@ -335,14 +425,16 @@ static __device__ __noinline__ bool walk_weak(const WalkArgs &a, unsigned char *
   __syncthreads();
   const int count = *scount;
   if (count == 0) return false;
+  if (count <= NT / 8) {
+    walk_few<BS, NT>(gimg, stride, natural, scol, sst, n, h, a.slots, list, count, vals);
+    __syncthreads();
+    return true;
+  }
   for (int b0 = 0; b0 < count; b0 += NT) {
     const bool live = b0 + tid < count;
     const int ray = list[live ? b0 + tid : b0];
-    const uint32_t zz = a.slots[ray >> 1].zzd;
-    const int d = (int)(zz >> 16);
     nb_axial A;
-    nb_axial_setup(nb_ring_pair((int)((d ? zz : zz >> (ray & 1) * 8) & 255u) / 2, d,
-                                d ? 1 + (ray & 1) : 0), h.y, h.x, h.z, A);
+    slot_axial(a.slots, ray, h, A);
     // offset of the ray's plane in a column (plane 127 reads as zero) and its change at the next
     // crossing; in the col128 order every second crossing turns between the even and odd halves
     int zo = (natural ? A.w : nb_zi(A.w)) * BS;
@@ -415,11 +507,8 @@ static __device__ __forceinline__ void spread_rays(const WalkArgs &a, unsigned c
   const float *vals = reinterpret_cast<const float *>(smem);
   float *gb = a.bimg + (size_t)g * NB_IMG_COL128 * BS;
   for (int ray = threadIdx.x; ray < 2 * a.nslots; ray += NT) {
-    const uint32_t zz = a.slots[ray >> 1].zzd;
-    const int d = (int)(zz >> 16);
     nb_axial A;
-    nb_axial_setup(nb_ring_pair((int)((d ? zz : zz >> (ray & 1) * 8) & 255u) / 2, d,
-                                d ? 1 + (ray & 1) : 0), h.y, h.x, h.z, A);
+    slot_axial(a.slots, ray, h, A);
     for (int k = 0; k < BS; k++) {
       const float v = vals[ray * BS + k];
       if (!(which >> k & 1u) || v == 0.f) continue;
@@ -892,7 +981,9 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const __grid_constant__ WalkA
           weak |= fA < all || (fA < clip && fA > 0.f) || fB < all || (fB < clip && fB > 0.f);
         }
       }
-      if (__syncthreads_or(weak)) {           // (the walk is done: the table region is free)
+      bool again = __syncthreads_or(weak);    // (the walk is done: the table region is free)
+      if (MODE == MODE_OSEM && again) again = __syncthreads_or(bins_matter<BS, NT>(a, sthr, g, lor));
+      if (again) {
 #pragma unroll
         for (int j = 0; j < SPT; j++) {
           const int sl = slot_of(j);
