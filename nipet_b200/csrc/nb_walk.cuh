@@ -232,7 +232,7 @@ static __device__ __forceinline__ void slot_axial(const nb_slot *slots, int ray,
                               d ? 1 + (ray & 1) : 0), h.y, h.x, h.z, A);
 }
 
-// Up to NT / 8 rays of `list` step by step in float32, straight from the image: a ray in eight
+// Up to NT / 8 rays of `list` step by step in float32, straight from the image: a ray in 8 to 32
 // parts, whose lanes find their start by the crossings alone.  (Staged as below they would wait
 // for five rounds of copies: 33 LORs, which take 22 us, took 30 us longer.)
 template <int BS, int NT>
@@ -242,19 +242,31 @@ static __device__ __noinline__ void walk_few(const float *gimg, size_t stride, b
                                              const uint16_t *list, int count, float *vals) {
   constexpr int U = 4;                        // steps whose reads are in flight together
   const int tid = threadIdx.x;
-  const bool live = tid / 8 < count;
-  const int ray = list[live ? tid / 8 : 0], part = ((n + 7) / 8 + U - 1) / U * U;
-  const int s0 = min(n, (tid & 7) * part), s1 = live ? min(n, s0 + part) : 0;
+  const int lanes = count <= NT / 32 ? 32 : (count <= NT / 16 ? 16 : 8), sub = tid & (lanes - 1);
+  const bool live = tid / lanes < count;
+  const int ray = list[live ? tid / lanes : 0], part = ((n + lanes - 1) / lanes + U - 1) / U * U;
+  const int s0 = min(n, sub * part), s1 = live ? min(n, s0 + part) : 0;
   nb_axial A;
   slot_axial(slots, ray, h, A);
   int z = A.w;
   float tp = h.x, tzc = A.tzc, acc[BS];
-  for (int s = 0; s < (live ? s0 : 0); s++) {
-    tp = sst[s];
-    if (tp > tzc) {
+  if (s0 < s1 && s0 > 0) {
+    // the crossings before the last four steps (s0 is a multiple of four), then those steps one
+    // by one: a crossing put off to the next step has caught up by then
+    const float t0 = s0 > 4 ? sst[s0 - 5] : h.x;
+    for (int c = 0; c < s0 - 4 && t0 > tzc; c++) {
       z += A.dir;
       tzc = __fadd_rn(tzc, A.dtz);
     }
+    float t[4];
+    ldv<4>(sst + s0 - 4, t);
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (t[u] > tzc) {
+        z += A.dir;
+        tzc = __fadd_rn(tzc, A.dtz);
+      }
+    tp = t[3];
   }
 #pragma unroll
   for (int k = 0; k < BS; k++) acc[k] = 0.f;
@@ -283,11 +295,10 @@ static __device__ __noinline__ void walk_few(const float *gimg, size_t stride, b
 #pragma unroll
       for (int k = 0; k < BS; k++) acc[k] = fmaf(w1[u], v1[u][k], fmaf(w0[u], v0[u][k], acc[k]));
   }
-#pragma unroll
-  for (int o = 1; o < 8; o <<= 1)
+  for (int o = 1; o < lanes; o <<= 1)
 #pragma unroll
     for (int k = 0; k < BS; k++) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-  if (live && (tid & 7) == 0)
+  if (live && sub == 0)
 #pragma unroll
     for (int k = 0; k < BS; k++) vals[ray * BS + k] = acc[k];
 }
@@ -299,16 +310,37 @@ template <int BS, int NT>
 static __device__ __noinline__ bool bins_matter(const WalkArgs &a, const float *sthr, int g, int lor) {
   bool some = false;
   const size_t row = (size_t)lor * a.nout;
+  const float *rs = a.rs + row;
+  const uint16_t *y[BS];
+  float lim[BS], scale[BS];
 #pragma unroll
   for (int k = 0; k < BS; k++) {
-    const int rep = g * BS + k;
-    if (rep >= a.nrep) break;
-    const float q = sthr[k], scale = a.rscale[rep];
-    const uint16_t *y = a.psng + (size_t)rep * a.naw * a.nout + row;
-    some |= q == __int_as_float(0x7f800000);
-#pragma unroll 4
-    for (int o = threadIdx.x; o < a.nout; o += NT)
-      some |= (__ldg(y + o) != 0) & !(scale * __ldg(a.rs + row + o) >= q * WEAK_QUANTA);
+    const int rep = min(g * BS + k, a.nrep - 1);   // (a padding image repeats the last one)
+    y[k] = a.psng + (size_t)rep * a.naw * a.nout + row;
+    scale[k] = a.rscale[rep];
+    lim[k] = sthr[k] * WEAK_QUANTA;
+    some |= lim[k] == __int_as_float(0x7f800000);
+  }
+  // four bins at a time where rows allow it (span 1)
+  const bool vec = a.nout % 4 == 0 && (((uintptr_t)a.rs & 15) | ((uintptr_t)a.psng & 7)) == 0;
+  if (vec) {
+#pragma unroll 2
+    for (int o = threadIdx.x; o < a.nout / 4; o += NT) {
+      const float4 r = __ldg(reinterpret_cast<const float4 *>(rs) + o);
+#pragma unroll
+      for (int k = 0; k < BS; k++) {
+        const ushort4 c = __ldg(reinterpret_cast<const ushort4 *>(y[k]) + o);
+        some |= ((c.x != 0) & !(scale[k] * r.x >= lim[k])) | ((c.y != 0) & !(scale[k] * r.y >= lim[k])) |
+                ((c.z != 0) & !(scale[k] * r.z >= lim[k])) | ((c.w != 0) & !(scale[k] * r.w >= lim[k]));
+      }
+    }
+  } else {
+#pragma unroll 2
+    for (int o = threadIdx.x; o < a.nout; o += NT) {
+      const float r = __ldg(rs + o);
+#pragma unroll
+      for (int k = 0; k < BS; k++) some |= (__ldg(y[k] + o) != 0) & !(scale[k] * r >= lim[k]);
+    }
   }
   return some;
 }
