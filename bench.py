@@ -8,7 +8,7 @@ configurations, whose datasets are not available here):
   batch (default) batched bootstrap OSEM: R = 50 Poisson replicates of one synthetic scan
         (45 at 3e7 counts, 5 at 3e6), all reconstructed together per step: 14 sensitivity
         images + 4 iterations x 14 subsets, span-11 (837 x 252 x 344 sinograms),
-        320x320x127 float32 images, one persistent launch per sub-iteration and one CUDA
+        320x320x127 float32 images, one fused launch per sub-iteration and one CUDA
         graph per iteration.  Metric: reconstructions (replicates) per second.
   osem  one plain OSEM reconstruction per step (same scan: brain phantom, water
         attenuation, log-normal crystal efficiencies, 20% uniform randoms, 3e7 counts).

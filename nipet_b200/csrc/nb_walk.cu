@@ -41,7 +41,8 @@ int launch(nb_geom *g, const nbw::WalkArgs &a, cudaStream_t s) {
 //                 24 steps, 1 x 384 threads  1414 / 780 / 681
 //                 32 steps, 1 x 256 threads  1460 / 754 / 694
 //                 32 steps, 1 x 1024 threads 1727 / 942 / 735
-// The order holds for fused sub-iterations of 600 LORs and of 2 to 8 images, at both spans; at 33
+// (timed before weak rays were walked again; the shapes taken now: 1420 / 680 / 760, 1252 / 633 /
+// 634 and 1281 / 676 / 659).  The order holds for fused sub-iterations of 600 LORs and of 2 to 8 images, at both spans; at 33
 // LORs the two-image shape of 512 threads is the faster one (300 against 349 us), but no subset
 // is that small.
 template <int MODE> int launch_prj(nb_geom *g, const nbw::WalkArgs &a, int bs, cudaStream_t s) {

@@ -45,12 +45,14 @@
 // wave 9% of the SMs' time idle at 4894 LORs).
 //
 // Measured (B200, 1965 MHz; per call, against the step-by-step walk it replaces): attenuation
-// factors of all LORs at span 11 28.0 -> 3.4 ms (chunks without any value are skipped), a
-// 4894-LOR emission projection 2.16 -> 0.30 ms, a 5003-LOR span-1 back projection 2.57 ->
-// 0.84 ms, a drop-in OSEM iteration 64.4 -> 20.9 ms, 9 images batched 341 -> 163 ms.  Against
-// the FP64 oracle the error halves (forward 1.2e-7 -> 5e-8, back 1.5e-7 -> 6e-8 relative L2).
-// What bounds it: the shared-memory (LSU) pipe at 79 .. 81% of its wavefronts for one image,
-// half of them the crossings' (a warp of 32 pairs spans up to 8 ring differences, whose lanes
+// factors of all LORs at span 11 28.0 -> 3.3 ms (chunks without any value are skipped), a
+// 4894-LOR emission projection 2.16 -> 0.29 ms, a 5003-LOR span-1 back projection 2.57 ->
+// 0.84 ms, a drop-in OSEM iteration 64.4 -> 20.4 ms, 9 images batched 341 -> 161 ms.  Against
+// the FP64 oracle the error is less than half (forward 1.1e-7 -> 5e-8, back 1.7e-7 -> 6e-8
+// relative L2).  An image with 1e-5 around an object in place of zeros, whose weak rays (1000 on a
+// LOR through the object) are walked again, takes 1.12 ms for 4894 LORs in place of 0.68.
+// What bounds it: the shared-memory (LSU) pipe at 70 (forward) to 79% of its wavefronts for one
+// image, half of them the crossings' (a warp of 32 pairs spans up to 8 ring differences, whose lanes
 // share banks: 3.1 wavefronts per 8-byte read where 2 would do); of the time the crossings take
 // a third, the running sums a fifth, each chunk's set-up of the pairs a seventh, the rest loads,
 // bounds and the LOR's start and end.  Aligning differences to half-warps saved 20% of the

@@ -1,13 +1,12 @@
-"""The benchmarked batched shape against the FP64 oracle, at full size.
+"""The batched reconstruction against the FP64 oracle, at full size.
 
-The headline workload reconstructs bootstrap replicates of uneven count levels together:
-4 images per walk of the geometry (`k_osem_batch`, batch width 4), 4 iterations x the
+The headline workload reconstructs bootstrap replicates of uneven count levels together,
+several images per walk of the geometry (the fused mode of `k_walk`), 4 iterations x the
 reference's 14 subsets over all 68,516 LORs, span 11, 320 x 320 x 127.  Here 9 replicates
 -- 7 at 3e7 counts and 2 at 3e6 counts, in different groups, each with its own randoms
-level -- are reconstructed with the default tile (two groups of 4 and the ninth replicate
-in a second launch at width 1, as the benchmark's 50 replicates run 48 + 2), with the
-ninth in a padded third group of 4 instead, and with the shape the autotuner picks, and
-compared with the FP64 oracle's restatement of `recon.cu:318-497` run on the same inputs:
+level -- are reconstructed at width 4 (two groups of 4 and the ninth replicate in a second
+launch at width 1), with the ninth in a padded third group of 4 instead, and at the width
+the autotuner picks (the benchmark's 50 run at 2), and compared with the FP64 oracle's restatement of `recon.cu:318-497` run on the same inputs:
 
 * every image within 1e-4 relative L2 inside the mask;
 * the voxel-wise mean and standard deviation (ddof 1) over the replicates within 1e-4
