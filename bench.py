@@ -1017,10 +1017,10 @@ def run_chain(args, ws, rank, dev):
         torch.cuda.synchronize(dev)
         et.append(time.perf_counter() - t)
     te = _max_over_ranks(float(np.mean(et)), ws, dev)
-    # bound of the fused sub-iteration: the shared-memory pipe, with the wavefronts of one
-    # subset launch from the one-kernel capture of the same kernel on a subset of the same
-    # size (counts in profiles/traffic.json); the 14 subsets have equal LOR counts
-    wf = _traffic('osem_subiteration_smem_wavefronts')
+    # bound of the fused sub-iteration: the shared-memory pipe, with the mean wavefronts of the
+    # chain's own 56 launches (counts in profiles/traffic.json): its images have cold
+    # background, whose chunks of zeros a launch skips
+    wf = _traffic('chain_subiteration_smem_wavefronts')
     tr = _traffic('osem_subiteration')
     algorithmic = {'unit': 'GB/s', 'achieved': achieved, 'frac_of_hbm_peak': achieved / peak,
                    'bytes_per_launch_avg': float(np.mean(byt)),

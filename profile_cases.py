@@ -30,6 +30,10 @@ launches 0, 1 are width 4, 2, 3 width 2 -- use -s 1 -c 1 and -s 3 -c 1).
 workloads twice each: batched forward and back projection of 8 images (span 11, all LORs),
 the attenuation projection, and a span-1 batched OSEM sub-iteration of 4 frames (capture
 -k regex:^k_walk -c 10).
+
+`chain` reconstructs one frame from the 2e8-word, 600 s stream as `bench.py --workload chain`
+does (about 4 GB on the device): capture its 56 fused launches with one single-pass metric,
+--kernel-name-base demangled -k 'regex:k_walk<.*512, .int.2,' -c 56.
 """
 from __future__ import annotations
 
@@ -178,8 +182,24 @@ def diffdyn(device='cuda:0'):
     print('diffdyn ok')
 
 
+def chain(device='cuda:0'):
+    """One reconstruction of the chain workload, on the benchmark's own inputs."""
+    import bench
+    from types import SimpleNamespace
+    from nipet_b200 import geometry, mmr_lmproc, mmrhist, mmrrec
+    dev = torch.device(device)
+    p = geometry.get_mmrparams()
+    sp = dict(p, Cnt=dict(p['Cnt'], SPN=11, DEVID=dev.index))
+    lm, mu, comp = bench._chain_inputs(SimpleNamespace(events=200_000_000, duration=600), p, dev, 0)
+    hst = mmrhist.hist_device(lm, sp, pl=mmr_lmproc.plan(lm.cpu().numpy()))
+    mmrrec.osemone({}, mu, hst, sp, recmod=1, itr=4, normcomp=comp)
+    torch.cuda.synchronize(dev)
+    print('chain ok')
+
+
 if __name__ == '__main__':
     {'projectors': projectors, 'hist': hist, 'batch': batch, 'sct': sct, 'diffdyn': diffdyn,
+     'chain': chain,
      'hist200': lambda: hist(nwords=200_000_000, duration=600),
      'hist200s1': lambda: hist(nwords=200_000_000, duration=600, span=1),
      'hist200boot': lambda: hist(nwords=200_000_000, duration=600, nrep=4)}[
