@@ -28,19 +28,16 @@
 // depend on the order.  A ray's own sum, with the fraction terms, is 64 bits wide: it collects
 // from one plane after another and can exceed what any of them holds.
 //   The scale is set by the chunk's hottest plane, so a ray through values decades below it is a
-// sum of few quanta.  At the end of a LOR, rays below 2^20 quanta per chunk whose planes hold
-// weak values, and any below 1.5 x 2^16, are walked again step by step in float32, as the
-// reference walks every ray (walk_weak); so are all rays of an image whose chunk has no scale (a
-// value that is not finite, or above 2^100).  Where they are many, the forward mode first adds a
-// second pass over the values' rounding errors at their own, finer scale.  The fused mode leaves
-// out those whose ratio does not need them: nothing counted, or randoms above 2^20 quanta.
-// Every bin is then good to 1e-5 of its value, but for slivers of a step (a fraction is good to
-// 2^-25 of the step).
+// sum of few quanta.  At the end of a LOR, rays below 2^20 quanta per chunk whose planes hold weak
+// values, and any below 1.5 x 2^16, are walked again step by step in float32, as the reference
+// walks every ray (walk_weak); so are all rays of an image whose chunk has no scale (a value that
+// is not finite, or above 2^100).  The fused mode leaves out those whose ratio does not need them:
+// nothing counted, or randoms above 2^20 quanta.  Every bin is then good to 1e-5 of its value, but
+// for slivers of a step (a fraction is good to 2^-25 of the step).
 //   In the back projection a ray's value is rounded once, by at most 2^-23 of the LOR's largest,
-// and its two parts of a crossing sum to it exactly.  The weights that meet in a plane in one
-// step sum to 255 at the most (checked when the geometry is made: a late crossing has weights
-// outside [0, 1]) and values are below 2^23, so no sum leaves int32.  An image with a value that
-// is not finite goes to the voxels ray by ray in float32.
+// and its two parts of a crossing sum to it exactly.  The weights that meet in a plane in one step
+// sum to 255 at the most (checked when the geometry is made: a late crossing has weights outside
+// [0, 1]) and values are below 2^23, so no sum leaves int32.  An image with a value that is not finite goes to the voxels ray by ray in float32.
 //
 // Jobs.  One block per (LOR, image group); a finished block takes over a block that has not
 // started (cluster launch control), so LORs of 10 to 404 steps even out over the SMs and the
@@ -53,7 +50,7 @@
 // 0.84 ms, a drop-in OSEM iteration 64.4 -> 20.4 ms, 9 images batched 341 -> 161 ms.  Against
 // the FP64 oracle the error is less than half (forward 1.1e-7 -> 5e-8, back 1.7e-7 -> 6e-8
 // relative L2).  An image with 1e-5 around an object in place of zeros, whose weak rays (1000 on a
-// LOR through the object) need the second pass, takes 0.87 ms for 4894 LORs in place of 0.68.
+// LOR through the object) are walked again, takes 1.12 ms for 4894 LORs in place of 0.68.
 // What bounds it: the shared-memory (LSU) pipe at 70 (forward) to 79% of its wavefronts for one
 // image, half of them the crossings' (a warp of 32 pairs spans up to 8 ring differences, whose lanes
 // share banks: 3.1 wavefronts per 8-byte read where 2 would do); of the time the crossings take
@@ -127,7 +124,7 @@ template <int BS, int CH, int NSEG> struct WSmem {
   static constexpr size_t max_off = align128(cs_off + 16ull * NB_STEP_STRIDE);  // [3][NSEG][BS]
   static constexpr size_t obl_off = align128(max_off + 12ull * NSEG * BS);      // [64]
   static constexpr size_t misc_off = obl_off + 256;
-  static constexpr size_t total = misc_off + 256 + 64 * BS;   // (and [16][BS] chunk scales)
+  static constexpr size_t total = misc_off + 256;
   // walk_weak: the rays' integrals [4096][BS], the list of rays, then columns of the image
   static constexpr size_t list_off = 4096ull * 4 * BS;
   static constexpr size_t col_off = list_off + 4096 * 2;
@@ -198,10 +195,6 @@ static __device__ __forceinline__ void lds_tab(uint32_t addr, int *D, int *X) {
   }
 }
 
-// rounding offset of step j of a segment
-static __device__ __forceinline__ constexpr float spread(int j) {
-  return (float)(2 * ((5 * j + 2) % 8) - 7) / 16.f;
-}
 // byte offset of a plane in a row whose planes are `unit` bytes wide (even planes first)
 static __device__ __forceinline__ int plane_off(int P, int unit) {
   return P * (unit / 2) + (P & 1) * (127 * unit / 2);
@@ -606,7 +599,6 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const __grid_constant__ WalkA
   float *sthr = reinterpret_cast<float *>(misc + 96);                // [BS] sum of the quanta
   int *sweak = reinterpret_cast<int *>(misc + 112);                  // [BS] weak values were met
   unsigned *smin = reinterpret_cast<unsigned *>(misc + 128);         // [3][BS] least |value|
-  float *sscale = reinterpret_cast<float *>(misc + 256);             // [16][BS] first pass's scales
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int s = tid & 63;                     // scan: this thread's planes 2 s and 2 s + 1
@@ -620,7 +612,6 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const __grid_constant__ WalkA
     *sflag = 0;
     for (int k = 0; k < 3 * NSEG * BS; k++) smax[k] = 0u;
     for (int k = 0; k < 3 * BS; k++) smin[k] = ~0u;
-    for (int k = 0; k < 16 * BS; k++) sscale[k] = 0.f;   // (a chunk of zeros leaves a finite one)
     for (int k = 0; k < 2 * BS; k++) smaxb[k] = 0u;
     nb_fence_mbar_init();
   }
@@ -787,279 +778,244 @@ __global__ void __launch_bounds__(NT, MINB) k_walk(const __grid_constant__ WalkA
           }
         }
       };
-      bool again;
-      // forward mode: a LOR with many weak rays (in half of its threads) takes a second pass over
-      // what the first one's rounding left of each value, at its own scale, 2^23 and more times
-      // finer, before the weak ones that remain are walked.  4894 LORs of a tenth OSEM iterate of
-      // noisy data 2.3 -> 1.63, 2.4 -> 1.52 and 2.4 -> 1.72 ms per image (one, two, four images); a
-      // third pass took 1.67 / 1.69 / 1.79.
-      for (int pass = 0;; pass++) {
-        for (int c = 0; c < nch; c++) {
-          const int s0 = c * CH, s1 = min(n, s0 + CH);
-          // (holding the next chunk's values through the walk instead hid their latency but
-          // spilled: 1604 against 1487 us for one image's fused subset, 1471 against 1267 for two)
-          load(c);
-          // bound of the chunk's integrals per image: over its segments, the largest integral
-          // of |value| of any plane
-          float lt[SEGL];
-          {
-            step_lengths(s0, lt);
-            if (MODE == MODE_FWD && pass) {
+      for (int c = 0; c < nch; c++) {
+        const int s0 = c * CH, s1 = min(n, s0 + CH);
+        // (holding the next chunk's values through the walk instead hid their latency but
+        // spilled: 1604 against 1487 us for one image's fused subset, 1471 against 1267 for two)
+        load(c);
+        // bound of the chunk's integrals per image: over its segments, the largest integral
+        // of |value| of any plane
+        float lt[SEGL];
+        {
+          step_lengths(s0, lt);
+          float m[BS];
 #pragma unroll
-              for (int v = 0; v < BS; v++) {
-                const float s1 = sscale[c * BS + v], i1 = s1 > 0.f ? __frcp_rn(s1) : 0.f;
+          for (int v = 0; v < BS; v++) m[v] = 0.f;
 #pragma unroll
-                for (int j = 0; j < SEGL; j++) {
-                  const float w = lt[j] * s1;
-                  E[j][v] = fmaf(E[j][v], w, -(float)__float2int_rn(fmaf(E[j][v], w, spread(j)))) * i1;
-                  O[j][v] = fmaf(O[j][v], w, -(float)__float2int_rn(fmaf(O[j][v], w, spread(j)))) * i1;
-                }
-              }
+          for (int v = 0; v < BS; v++) {
+            float me = 0.f, mo = 0.f;
 #pragma unroll
-              for (int j = 0; j < SEGL; j++) lt[j] = 1.f;   // (the rests have their lengths in them)
+            for (int j = 0; j < SEGL; j++) {
+              me = fmaf(lt[j], fabsf(E[j][v]), me);
+              mo = fmaf(lt[j], fabsf(O[j][v]), mo);
             }
+            const unsigned u = __reduce_max_sync(0xffffffffu, max(__float_as_uint(me), __float_as_uint(mo)));
+            if (u == 0u) continue;            // (the whole warp)
+            unsigned lo = ~0u;                // least non-zero |value|, as 2 * bits - 1
+#pragma unroll
+            for (int j = 0; j < SEGL; j++)
+              lo = min(lo, min(2u * __float_as_uint(E[j][v]) - 1u, 2u * __float_as_uint(O[j][v]) - 1u));
+            lo = __reduce_min_sync(0xffffffffu, lo);
+            if (lane == 0) {
+              atomicMax(&smax[(mrot * NSEG + seg) * BS + v], u);
+              atomicMin(&smin[mrot * BS + v], lo);
+            }
+          }
+        }
+        __syncthreads();
+        unsigned any = 0u;
+        float scale[BS], inv[BS], bnd[NSEG * BS];
+#pragma unroll
+        for (int x = 0; x < NSEG * BS; x += 4)
+          ldv<4>(reinterpret_cast<const float *>(smax) + mrot * NSEG * BS + x, bnd + x);
+#pragma unroll
+        for (int k = 0; k < BS; k++) {
+          float bound = 0.f;
+#pragma unroll
+          for (int x = 0; x < NSEG; x++) bound += bnd[x * BS + k];
+          const unsigned bb = __float_as_uint(bound);
+          any |= bb;
+          // bound < 2^e: scale 2^(29 - e), as far as float32 has it.  A bound that is not finite or
+          // above 2^100 has none: the image's rays are all walked again
+          const int x = min(155 - (int)(bb >> 23), 126);
+          const bool none = bb >= 0x71800000u;
+          scale[k] = bb && !none ? __uint_as_float((uint32_t)(127 + x) << 23) : 0.f;
+          inv[k] = bb && !none ? __uint_as_float((uint32_t)(127 - x) << 23) : 0.f;
+          if (bb != 0u && tid == 0) {
+            sthr[k] += none ? __int_as_float(0x7f800000) : inv[k];
+            if (none || smin[mrot * BS + k] < 2u * __float_as_uint(inv[k] * WEAK_VALUE) - 1u) sweak[k] = 1;
+          }
+        }
+        // cleared two chunks before its next use: its last readers are one barrier back
+        if (tid < NSEG * BS) smax[((mrot + 2) % 3) * NSEG * BS + tid] = 0u;
+        if (tid < BS) smin[((mrot + 2) % 3) * BS + tid] = ~0u;
+        mrot = (mrot + 1) % 3;
+        if (any == 0u) continue;              // nothing but zeros
+        {
+          // fixed-point running integrals: within the segment, then the segments before it
+          // (rounded with offsets spread over (-1/2, 1/2), so that the errors of equal values do
+          // not add up; 0 stays 0)
+          int cE[SEGL][BS], cO[SEGL][BS], tE[BS], tO[BS];
+#pragma unroll
+          for (int v = 0; v < BS; v++) tE[v] = tO[v] = 0;
+#pragma unroll
+          for (int j = 0; j < SEGL; j++) {
+            const float off = (float)(2 * ((5 * j + 2) % 8) - 7) / 16.f;
 #pragma unroll
             for (int v = 0; v < BS; v++) {
-              float me = 0.f, mo = 0.f;
+              const float w = lt[j] * scale[v];
+              cE[j][v] = tE[v];
+              cO[j][v] = tO[v];
+              tE[v] += __float2int_rn(fmaf(E[j][v], w, off));
+              tO[v] += __float2int_rn(fmaf(O[j][v], w, off));
+            }
+            if (s == 31) sti<BS>(soc + (seg * (SEGL + 1) + j) * BS, cO[j]);
+          }
+          if (s == 31) sti<BS>(soc + (seg * (SEGL + 1) + SEGL) * BS, tO);
+          sti<BS>(sseg + (seg * 128 + s) * BS, tE);
+          sti<BS>(sseg + (seg * 128 + 64 + s) * BS, tO);
+          __syncthreads();
+          int bE[BS], bO[BS];
 #pragma unroll
-              for (int j = 0; j < SEGL; j++) {
-                me = fmaf(lt[j], fabsf(E[j][v]), me);
-                mo = fmaf(lt[j], fabsf(O[j][v]), mo);
-              }
-              const unsigned u = __reduce_max_sync(0xffffffffu, max(__float_as_uint(me), __float_as_uint(mo)));
-              if (u == 0u) continue;            // (the whole warp)
-              unsigned lo = ~0u;                // least non-zero |value|, as 2 * bits - 1
+          for (int v = 0; v < BS; v++) bE[v] = bO[v] = 0;
+          for (int x = 0; x < seg; x++) {
+            int u[BS], w[BS];
+            ldi<BS>(sseg + (x * 128 + s) * BS, u);
+            ldi<BS>(sseg + (x * 128 + 64 + s) * BS, w);
 #pragma unroll
-              for (int j = 0; j < SEGL; j++)
-                lo = min(lo, min(2u * __float_as_uint(E[j][v]) - 1u, 2u * __float_as_uint(O[j][v]) - 1u));
-              lo = __reduce_min_sync(0xffffffffu, lo);
-              if (lane == 0) {
-                atomicMax(&smax[(mrot * NSEG + seg) * BS + v], u);
-                atomicMin(&smin[mrot * BS + v], lo);
-              }
+            for (int v = 0; v < BS; v++) bE[v] += u[v], bO[v] += w[v];
+          }
+          // the thread of plane 64 gets plane 63's prefixes through shared memory (its neighbour
+          // is another warp's); the thread of plane 0 has no plane below and its D[0] no reader
+          const bool fix = s == 32;
+          int bP[BS];
+#pragma unroll
+          for (int v = 0; v < BS; v++) bP[v] = 0;
+          if (fix)
+            for (int x = 0; x < seg; x++) {
+              int u[BS];
+              ldi<BS>(sseg + (x * 128 + 64 + 31) * BS, u);
+#pragma unroll
+              for (int v = 0; v < BS; v++) bP[v] += u[v];
+            }
+          if (seg == NSEG - 1) {              // the chunk's whole integral per plane
+            int u[BS], w[BS];
+#pragma unroll
+            for (int v = 0; v < BS; v++) u[v] = tE[v] + bE[v], w[v] = tO[v] + bO[v];
+            sti<BS>(srun + s * BS, u);
+            sti<BS>(srun + (64 + s) * BS, w);
+          }
+          // D at the start of each step and its change over the step
+          int De[BS], Do[BS];
+#pragma unroll
+          for (int j = SEGL; j >= 0; j--) {
+            int ne[BS], no[BS];               // D at the end of step j
+#pragma unroll
+            for (int v = 0; v < BS; v++) {
+              ne[v] = De[v];
+              no[v] = Do[v];
+              const int ce = (j < SEGL ? cE[j < SEGL ? j : 0][v] : tE[v]) + bE[v];
+              const int co = (j < SEGL ? cO[j < SEGL ? j : 0][v] : tO[v]) + bO[v];
+              int cp = __shfl_up_sync(0xffffffffu, co, 1);      // plane 2 s - 1
+              if (fix) cp = bP[v] + soc[(seg * (SEGL + 1) + j) * BS + v];
+              De[v] = cp - ce;
+              Do[v] = ce - co;
+              ne[v] -= De[v];
+              no[v] -= Do[v];
+            }
+            if (j == SEGL) continue;
+            unsigned char *r = tab + ((size_t)(seg * SEGL + j) << LOGR) + s * UNIT;
+            if (BS == 1) {
+              *reinterpret_cast<int2 *>(r) = make_int2(De[0], ne[0]);
+              *reinterpret_cast<int2 *>(r + 64 * UNIT) = make_int2(Do[0], no[0]);
+            } else if (BS == 2) {
+              *reinterpret_cast<int4 *>(r) = make_int4(De[0], De[BS - 1], ne[0], ne[BS - 1]);
+              *reinterpret_cast<int4 *>(r + 64 * UNIT) = make_int4(Do[0], Do[BS - 1], no[0], no[BS - 1]);
+            } else {
+              sti<BS>(reinterpret_cast<int *>(r), De);
+              sti<BS>(reinterpret_cast<int *>(r + 64 * UNIT), Do);
+              sti<BS>(reinterpret_cast<int *>(r + 2048), ne);
+              sti<BS>(reinterpret_cast<int *>(r + 2048 + 64 * UNIT), no);
             }
           }
           __syncthreads();
-          unsigned any = 0u;
-          float scale[BS], inv[BS], bnd[NSEG * BS];
-#pragma unroll
-          for (int x = 0; x < NSEG * BS; x += 4)
-            ldv<4>(reinterpret_cast<const float *>(smax) + mrot * NSEG * BS + x, bnd + x);
-#pragma unroll
-          for (int k = 0; k < BS; k++) {
-            float bound = 0.f;
-#pragma unroll
-            for (int x = 0; x < NSEG; x++) bound += bnd[x * BS + k];
-            const unsigned bb = __float_as_uint(bound);
-            any |= bb;
-            // bound < 2^e: scale 2^(29 - e), as far as float32 has it.  A bound that is not finite or
-            // above 2^100 has none: the image's rays are all walked again
-            const int x = min(155 - (int)(bb >> 23), 126);
-            const bool none = bb >= 0x71800000u;
-            scale[k] = bb && !none ? __uint_as_float((uint32_t)(127 + x) << 23) : 0.f;
-            inv[k] = bb && !none ? __uint_as_float((uint32_t)(127 - x) << 23) : 0.f;
-            if (bb != 0u && tid == 0) {
-              sthr[k] += none ? __int_as_float(0x7f800000) : inv[k];
-              if (none || smin[mrot * BS + k] < 2u * __float_as_uint(inv[k] * WEAK_VALUE) - 1u) sweak[k] = 1;
-            }
-          }
-          // cleared two chunks before its next use: its last readers are one barrier back
-          if (tid < NSEG * BS) smax[((mrot + 2) % 3) * NSEG * BS + tid] = 0u;
-          if (tid < BS) smin[((mrot + 2) % 3) * BS + tid] = ~0u;
-          mrot = (mrot + 1) % 3;
-          if (any == 0u) continue;              // nothing but zeros, also in a second pass
-          if (MODE == MODE_FWD && tid == 0 && pass == 0)
-#pragma unroll
-            for (int k = 0; k < BS; k++) sscale[c * BS + k] = scale[k];
-          {
-            // fixed-point running integrals: within the segment, then the segments before it
-            // (rounded with offsets spread over (-1/2, 1/2), so that the errors of equal values do
-            // not add up; 0 stays 0)
-            int cE[SEGL][BS], cO[SEGL][BS], tE[BS], tO[BS];
-#pragma unroll
-            for (int v = 0; v < BS; v++) tE[v] = tO[v] = 0;
-#pragma unroll
-            for (int j = 0; j < SEGL; j++) {
-              const float off = spread(j);
-#pragma unroll
-              for (int v = 0; v < BS; v++) {
-                const float w = lt[j] * scale[v];
-                cE[j][v] = tE[v];
-                cO[j][v] = tO[v];
-                tE[v] += __float2int_rn(fmaf(E[j][v], w, off));
-                tO[v] += __float2int_rn(fmaf(O[j][v], w, off));
-              }
-              if (s == 31) sti<BS>(soc + (seg * (SEGL + 1) + j) * BS, cO[j]);
-            }
-            if (s == 31) sti<BS>(soc + (seg * (SEGL + 1) + SEGL) * BS, tO);
-            sti<BS>(sseg + (seg * 128 + s) * BS, tE);
-            sti<BS>(sseg + (seg * 128 + 64 + s) * BS, tO);
-            __syncthreads();
-            int bE[BS], bO[BS];
-#pragma unroll
-            for (int v = 0; v < BS; v++) bE[v] = bO[v] = 0;
-            for (int x = 0; x < seg; x++) {
-              int u[BS], w[BS];
-              ldi<BS>(sseg + (x * 128 + s) * BS, u);
-              ldi<BS>(sseg + (x * 128 + 64 + s) * BS, w);
-#pragma unroll
-              for (int v = 0; v < BS; v++) bE[v] += u[v], bO[v] += w[v];
-            }
-            // the thread of plane 64 gets plane 63's prefixes through shared memory (its neighbour
-            // is another warp's); the thread of plane 0 has no plane below and its D[0] no reader
-            const bool fix = s == 32;
-            int bP[BS];
-#pragma unroll
-            for (int v = 0; v < BS; v++) bP[v] = 0;
-            if (fix)
-              for (int x = 0; x < seg; x++) {
-                int u[BS];
-                ldi<BS>(sseg + (x * 128 + 64 + 31) * BS, u);
-#pragma unroll
-                for (int v = 0; v < BS; v++) bP[v] += u[v];
-              }
-            if (seg == NSEG - 1) {              // the chunk's whole integral per plane
-              int u[BS], w[BS];
-#pragma unroll
-              for (int v = 0; v < BS; v++) u[v] = tE[v] + bE[v], w[v] = tO[v] + bO[v];
-              sti<BS>(srun + s * BS, u);
-              sti<BS>(srun + (64 + s) * BS, w);
-            }
-            // D at the start of each step and its change over the step
-            int De[BS], Do[BS];
-#pragma unroll
-            for (int j = SEGL; j >= 0; j--) {
-              int ne[BS], no[BS];               // D at the end of step j
-#pragma unroll
-              for (int v = 0; v < BS; v++) {
-                ne[v] = De[v];
-                no[v] = Do[v];
-                const int ce = (j < SEGL ? cE[j < SEGL ? j : 0][v] : tE[v]) + bE[v];
-                const int co = (j < SEGL ? cO[j < SEGL ? j : 0][v] : tO[v]) + bO[v];
-                int cp = __shfl_up_sync(0xffffffffu, co, 1);      // plane 2 s - 1
-                if (fix) cp = bP[v] + soc[(seg * (SEGL + 1) + j) * BS + v];
-                De[v] = cp - ce;
-                Do[v] = ce - co;
-                ne[v] -= De[v];
-                no[v] -= Do[v];
-              }
-              if (j == SEGL) continue;
-              unsigned char *r = tab + ((size_t)(seg * SEGL + j) << LOGR) + s * UNIT;
-              if (BS == 1) {
-                *reinterpret_cast<int2 *>(r) = make_int2(De[0], ne[0]);
-                *reinterpret_cast<int2 *>(r + 64 * UNIT) = make_int2(Do[0], no[0]);
-              } else if (BS == 2) {
-                *reinterpret_cast<int4 *>(r) = make_int4(De[0], De[BS - 1], ne[0], ne[BS - 1]);
-                *reinterpret_cast<int4 *>(r + 64 * UNIT) = make_int4(Do[0], Do[BS - 1], no[0], no[BS - 1]);
-              } else {
-                sti<BS>(reinterpret_cast<int *>(r), De);
-                sti<BS>(reinterpret_cast<int *>(r + 64 * UNIT), Do);
-                sti<BS>(reinterpret_cast<int *>(r + 2048), ne);
-                sti<BS>(reinterpret_cast<int *>(r + 2048 + 64 * UNIT), no);
-              }
-            }
-            __syncthreads();
-          }
+        }
 
-          const unsigned char *kend = rec + NB_REC_KEND;
-          const int krow0 = c * (CH / 8) - 1, krow1 = (s1 - 1) >> 3;
+        const unsigned char *kend = rec + NB_REC_KEND;
+        const int krow0 = c * (CH / 8) - 1, krow1 = (s1 - 1) >> 3;
 #pragma unroll
-          for (int j = 0; j < SPT; j++) {
-            const int zz = (int)zzd[j], d = zz >> 16;
-            const int ka = c ? kend[krow0 * 64 + d] : 0;
-            int cnt = kend[krow1 * 64 + d] - ka;
-            const int e0 = reinterpret_cast<const uint16_t *>(rec + NB_REC_OFF)[d] + ka;
-            const int zA = (zz & 255) + ka, zB = ((zz >> 8) & 255) - ka;
-            const int endA = zA + cnt, endB = zB - cnt;
-            uint32_t ep = rec_u + NB_REC_ENT + e0 * 8;
-            // cursors of the next crossing and the one after (their plane offsets in a row);
-            // two crossings on, both have moved by one unit
-            const uint32_t base = tab_u - ((uint32_t)s0 << LOGR);
-            uint32_t cA0 = base + plane_off(zA + 1, UNIT), cB0 = base + plane_off(zB, UNIT);
-            uint32_t cA1 = cA0 + 64 * UNIT - ((zA + 1) & 1) * (127 * UNIT);
-            uint32_t cB1 = cB0 + 63 * UNIT - (zB & 1) * (127 * UNIT);
-            // sums of D + dD * fraction in 2^-QBITS quanta, 64 bits: a ray that changes planes can
-            // collect more than any plane holds, up to SEGL times 2^29.  Two crossings' D fit 32
-            // (the plane between them cancels but for what the ray collects in it: 3 x 2^29)
-            long long xA[BS], xB[BS];
-            int dA[BS], dB[BS];
+        for (int j = 0; j < SPT; j++) {
+          const int zz = (int)zzd[j], d = zz >> 16;
+          const int ka = c ? kend[krow0 * 64 + d] : 0;
+          int cnt = kend[krow1 * 64 + d] - ka;
+          const int e0 = reinterpret_cast<const uint16_t *>(rec + NB_REC_OFF)[d] + ka;
+          const int zA = (zz & 255) + ka, zB = ((zz >> 8) & 255) - ka;
+          const int endA = zA + cnt, endB = zB - cnt;
+          uint32_t ep = rec_u + NB_REC_ENT + e0 * 8;
+          // cursors of the next crossing and the one after (their plane offsets in a row);
+          // two crossings on, both have moved by one unit
+          const uint32_t base = tab_u - ((uint32_t)s0 << LOGR);
+          uint32_t cA0 = base + plane_off(zA + 1, UNIT), cB0 = base + plane_off(zB, UNIT);
+          uint32_t cA1 = cA0 + 64 * UNIT - ((zA + 1) & 1) * (127 * UNIT);
+          uint32_t cB1 = cB0 + 63 * UNIT - (zB & 1) * (127 * UNIT);
+          // sums of D + dD * fraction in 2^-QBITS quanta, 64 bits: a ray that changes planes can
+          // collect more than any plane holds, up to SEGL times 2^29.  Two crossings' D fit 32
+          // (the plane between them cancels but for what the ray collects in it: 3 x 2^29)
+          long long xA[BS], xB[BS];
+          int dA[BS], dB[BS];
 #pragma unroll
-            for (int k = 0; k < BS; k++) xA[k] = xB[k] = 0;
-            auto cross = [&](int f, uint32_t rA, uint32_t rB) {
-              int X[BS];
-              lds_tab<BS>(rA, dA, X);
+          for (int k = 0; k < BS; k++) xA[k] = xB[k] = 0;
+          auto cross = [&](int f, uint32_t rA, uint32_t rB) {
+            int X[BS];
+            lds_tab<BS>(rA, dA, X);
 #pragma unroll
-              for (int k = 0; k < BS; k++) xA[k] += (long long)X[k] * f;
-              lds_tab<BS>(rB, dB, X);
+            for (int k = 0; k < BS; k++) xA[k] += (long long)X[k] * f;
+            lds_tab<BS>(rB, dB, X);
 #pragma unroll
-              for (int k = 0; k < BS; k++) xB[k] += (long long)X[k] * f;
-            };
-            for (; cnt >= 2; cnt -= 2) {
-              int i0, i1, f0, f1, eA[BS], eB[BS];
-              lds_ent(ep, i0, f0);
-              lds_ent(ep + 8, i1, f1);
-              ep += 16;
-              cross(f0, cA0 + (i0 << LOGR), cB0 + (i0 << LOGR));
+            for (int k = 0; k < BS; k++) xB[k] += (long long)X[k] * f;
+          };
+          for (; cnt >= 2; cnt -= 2) {
+            int i0, i1, f0, f1, eA[BS], eB[BS];
+            lds_ent(ep, i0, f0);
+            lds_ent(ep + 8, i1, f1);
+            ep += 16;
+            cross(f0, cA0 + (i0 << LOGR), cB0 + (i0 << LOGR));
 #pragma unroll
-              for (int k = 0; k < BS; k++) eA[k] = dA[k], eB[k] = dB[k];
-              cross(f1, cA1 + (i1 << LOGR), cB1 + (i1 << LOGR));
-#pragma unroll
-              for (int k = 0; k < BS; k++) {
-                xA[k] += (long long)(eA[k] + dA[k]) * (1 << QBITS);
-                xB[k] += (long long)(eB[k] + dB[k]) * (1 << QBITS);
-              }
-              cA0 += UNIT;
-              cA1 += UNIT;
-              cB0 -= UNIT;
-              cB1 -= UNIT;
-            }
-            if (cnt) {
-              int i0, f0;
-              lds_ent(ep, i0, f0);
-              cross(f0, cA0 + (i0 << LOGR), cB0 + (i0 << LOGR));
-#pragma unroll
-              for (int k = 0; k < BS; k++) {
-                xA[k] += (long long)dA[k] * (1 << QBITS);
-                xB[k] += (long long)dB[k] * (1 << QBITS);
-              }
-            }
-            // the down-going ray leaves C[P] for C[P-1]: its differences count negative
-            int u[BS], w[BS];
-            ldi<BS>(srun + nb_zi(endA) * BS, u);
-            ldi<BS>(srun + nb_zi(endB) * BS, w);
+            for (int k = 0; k < BS; k++) eA[k] = dA[k], eB[k] = dB[k];
+            cross(f1, cA1 + (i1 << LOGR), cB1 + (i1 << LOGR));
 #pragma unroll
             for (int k = 0; k < BS; k++) {
-              FA[j][k] = fmaf(quanta(u[k], xA[k]), inv[k], FA[j][k]);
-              FB[j][k] = fmaf(quanta(w[k], -xB[k]), inv[k], FB[j][k]);
+              xA[k] += (long long)(eA[k] + dA[k]) * (1 << QBITS);
+              xB[k] += (long long)(eB[k] + dB[k]) * (1 << QBITS);
+            }
+            cA0 += UNIT;
+            cA1 += UNIT;
+            cB0 -= UNIT;
+            cB1 -= UNIT;
+          }
+          if (cnt) {
+            int i0, f0;
+            lds_ent(ep, i0, f0);
+            cross(f0, cA0 + (i0 << LOGR), cB0 + (i0 << LOGR));
+#pragma unroll
+            for (int k = 0; k < BS; k++) {
+              xA[k] += (long long)dA[k] * (1 << QBITS);
+              xB[k] += (long long)dB[k] * (1 << QBITS);
             }
           }
-        }
-        // rays whose sums are too few quanta to be good to float32's precision are walked again
-        bool weak = false, scaled = true;
+          // the down-going ray leaves C[P] for C[P-1]: its differences count negative
+          int u[BS], w[BS];
+          ldi<BS>(srun + nb_zi(endA) * BS, u);
+          ldi<BS>(srun + nb_zi(endB) * BS, w);
 #pragma unroll
-        for (int k = 0; k < BS; k++) {
-          const float clip = sthr[k] * CLIP_QUANTA, all = sweak[k] ? sthr[k] * WEAK_QUANTA : 0.f;
-          scaled &= clip < __int_as_float(0x7f800000);
-#pragma unroll
-          for (int j = 0; j < SPT; j++) {
-            const float fA = fabsf(FA[j][k]), fB = fabsf(FB[j][k]);
-            weak |= fA < all || (fA < clip && fA > 0.f) || fB < all || (fB < clip && fB > 0.f);
+          for (int k = 0; k < BS; k++) {
+            FA[j][k] = fmaf(quanta(u[k], xA[k]), inv[k], FA[j][k]);
+            FB[j][k] = fmaf(quanta(w[k], -xB[k]), inv[k], FB[j][k]);
           }
         }
-        // (the walk is done: the table region is free)
-        if (MODE == MODE_FWD) {
-          const int threads = __syncthreads_count(weak);
-          again = threads != 0;
-          if (pass == 0 && scaled && threads >= NT / 2) {
-            if (tid == 0)
-              for (int k = 0; k < BS; k++) sthr[k] = 0.f, sweak[k] = 0;
-            continue;
-          }
-        } else {
-          again = __syncthreads_or(weak);
-        }
-        break;
       }
+      // rays whose sums are too few quanta to be good to float32's precision are walked again
+      bool weak = false;
+#pragma unroll
+      for (int k = 0; k < BS; k++) {
+        const float clip = sthr[k] * CLIP_QUANTA, all = sweak[k] ? sthr[k] * WEAK_QUANTA : 0.f;
+#pragma unroll
+        for (int j = 0; j < SPT; j++) {
+          const float fA = fabsf(FA[j][k]), fB = fabsf(FB[j][k]);
+          weak |= fA < all || (fA < clip && fA > 0.f) || fB < all || (fB < clip && fB > 0.f);
+        }
+      }
+      bool again = __syncthreads_or(weak);    // (the walk is done: the table region is free)
       if (MODE == MODE_OSEM && again) again = __syncthreads_or(bins_matter<BS, NT>(a, sthr, g, lor));
       if (again) {
 #pragma unroll
