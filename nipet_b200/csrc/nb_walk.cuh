@@ -236,17 +236,20 @@ static __device__ __forceinline__ void slot_axial(const nb_slot *slots, int ray,
 
 // Up to NT / 8 rays of `list` step by step in float32, straight from the image: a ray in 8 to 32
 // parts, whose lanes find their start by the crossings alone.  (Staged as below they would wait
-// for five rounds of copies: 33 LORs, which take 22 us, took 30 us longer.)
+// for five rounds of copies: 33 LORs, which take 22 us, took 30 us longer.)  Sums are formed per
+// block of 8 steps and added up in order, as there: a ray's result depends on neither the number
+// of rays nor the lanes.  sums: NB_STEP_STRIDE / 8 blocks a ray.
 template <int BS, int NT>
 static __device__ __noinline__ void walk_few(const float *gimg, size_t stride, bool natural,
                                              const int32_t *scol, const float *sst, int n,
                                              const float4 h, const nb_slot *slots,
-                                             const uint16_t *list, int count, float *vals) {
+                                             const uint16_t *list, int count, float *vals,
+                                             float *sums) {
   constexpr int U = 4;                        // steps whose reads are in flight together
   const int tid = threadIdx.x;
   const int lanes = count <= NT / 32 ? 32 : (count <= NT / 16 ? 16 : 8), sub = tid & (lanes - 1);
   const bool live = tid / lanes < count;
-  const int ray = list[live ? tid / lanes : 0], part = ((n + lanes - 1) / lanes + U - 1) / U * U;
+  const int ray = list[live ? tid / lanes : 0], part = ((n + lanes - 1) / lanes + 7) & ~7;
   const int s0 = min(n, sub * part), s1 = live ? min(n, s0 + part) : 0;
   nb_axial A;
   slot_axial(slots, ray, h, A);
@@ -270,9 +273,11 @@ static __device__ __noinline__ void walk_few(const float *gimg, size_t stride, b
       }
     tp = t[3];
   }
-#pragma unroll
-  for (int k = 0; k < BS; k++) acc[k] = 0.f;
+  float *mine = sums + (size_t)(tid / lanes) * (NB_STEP_STRIDE / 8) * BS;
   for (int s = s0; s < s1; s += U) {
+    if ((s & 7) == 0)
+#pragma unroll
+      for (int k = 0; k < BS; k++) acc[k] = 0.f;
     float v0[U][BS], v1[U][BS], w0[U], w1[U];
 #pragma unroll
     for (int u = 0; u < U; u++) {
@@ -296,13 +301,20 @@ static __device__ __noinline__ void walk_few(const float *gimg, size_t stride, b
     for (int u = 0; u < U; u++)
 #pragma unroll
       for (int k = 0; k < BS; k++) acc[k] = fmaf(w1[u], v1[u][k], fmaf(w0[u], v0[u][k], acc[k]));
-  }
-  for (int o = 1; o < lanes; o <<= 1)
+    if ((s & 4) || s + U >= s1)
 #pragma unroll
-    for (int k = 0; k < BS; k++) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-  if (live && sub == 0)
+      for (int k = 0; k < BS; k++) mine[(s >> 3) * BS + k] = acc[k];
+  }
+  __syncwarp();
+  if (live && sub == 0) {
+#pragma unroll
+    for (int k = 0; k < BS; k++) acc[k] = 0.f;
+    for (int b = 0; b < (n + 7) / 8; b++)
+#pragma unroll
+      for (int k = 0; k < BS; k++) acc[k] += mine[b * BS + k];
 #pragma unroll
     for (int k = 0; k < BS; k++) vals[ray * BS + k] = acc[k];
+  }
 }
 
 // Fused mode: has the LOR a bin whose ratio could need more than 2^20 quanta per chunk?  Not where
@@ -460,7 +472,8 @@ static __device__ __noinline__ bool walk_weak(const WalkArgs &a, unsigned char *
   const int count = *scount;
   if (count == 0) return false;
   if (count <= NT / 8) {
-    walk_few<BS, NT>(gimg, stride, natural, scol, sst, n, h, a.slots, list, count, vals);
+    static_assert(NT / 8 * (NB_STEP_STRIDE / 8) * BS * 4 <= L::region - L::col_off, "block sums fit");
+    walk_few<BS, NT>(gimg, stride, natural, scol, sst, n, h, a.slots, list, count, vals, cols);
     __syncthreads();
     return true;
   }
@@ -474,9 +487,9 @@ static __device__ __noinline__ bool walk_weak(const WalkArgs &a, unsigned char *
     int zo = (natural ? A.w : nb_zi(A.w)) * BS;
     int dz = natural ? A.dir : (A.dir > 0 ? ((A.w & 1) ? -63 : 64) : ((A.w & 1) ? -64 : 63)) * BS;
     const int dsum = natural ? 2 * A.dir : A.dir * BS;
-    float tp = h.x, tzc = A.tzc, acc[BS];
+    float tp = h.x, tzc = A.tzc, acc[BS], sum[BS];   // of a block of 8 steps; of the blocks
 #pragma unroll
-    for (int k = 0; k < BS; k++) acc[k] = 0.f;
+    for (int k = 0; k < BS; k++) sum[k] = 0.f;
     for (int s0 = 0; s0 < n; s0 += L::ncol) {
       const int m = min(L::ncol, n - s0);
       __syncthreads();                        // the columns before have been walked
@@ -512,18 +525,28 @@ static __device__ __noinline__ bool walk_weak(const WalkArgs &a, unsigned char *
         ldv<4>(sst + s0 + i, t);
         ldv<4>(sst + s0 + i + 4, t + 4);
 #pragma unroll
+        for (int k = 0; k < BS; k++) acc[k] = 0.f;
+#pragma unroll
         for (int u = 0; u < 8; u++) step(u, t[u]);
+#pragma unroll
+        for (int k = 0; k < BS; k++) sum[k] += acc[k];
         c += 8 * 128 * BS;
       }
-      for (; i < m; i++) {
-        step(0, sst[s0 + i]);
-        c += 128 * BS;
+      if (i < m) {
+#pragma unroll
+        for (int k = 0; k < BS; k++) acc[k] = 0.f;
+        for (; i < m; i++) {
+          step(0, sst[s0 + i]);
+          c += 128 * BS;
+        }
+#pragma unroll
+        for (int k = 0; k < BS; k++) sum[k] += acc[k];
       }
       zo = (int)(c - cols) - m * 128 * BS;
     }
     if (live)
 #pragma unroll
-      for (int k = 0; k < BS; k++) vals[ray * BS + k] = acc[k];
+      for (int k = 0; k < BS; k++) vals[ray * BS + k] = sum[k];
   }
   __syncthreads();
   return true;

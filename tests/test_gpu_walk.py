@@ -191,6 +191,24 @@ def test_walk_weak_planes(env, nimg, ratio):
     _errors(env, im, subs, nimg, hot * (0.3 * 2.0 ** -25 * im.max()))
 
 
+@pytest.mark.parametrize('seed', [0, 1, 2])
+@pytest.mark.parametrize('nimg', [1, 2, 4])
+def test_walk_planes_of_all_scales(env, nimg, seed):
+    """Planes of random levels over twelve decades, alone and in blocks, with voxel noise: most
+    rays are weak against some plane of their LOR, many of them against a chunk's first pass."""
+    r = np.random.default_rng(seed)
+    level = 10.0 ** r.uniform(-12, 0, 127)
+    if seed:
+        level[:40], level[90:] = 10.0 ** r.uniform(-12, -3), 10.0 ** r.uniform(-12, -3)
+    im = (r.uniform(0.5, 1.5, (320, 320, 127)) * level).astype(np.float32)
+    rno = env['p']['axLUT']['li2rno'].astype(int)
+    slack = np.zeros(4084)
+    for li, (r0, r1) in enumerate(zip(rno.min(1), rno.max(1))):
+        top = level[max(0, 2 * r0 - 1):2 * r1 + 2].max()   # of the planes between the rings
+        slack[env['p']['axLUT']['li2sn1'][li]] = 1.5 * top * 0.3 * 2.0 ** -25
+    _errors(env, im, env['subs'], nimg, slack)
+
+
 @pytest.mark.parametrize('ratio', [100, 300, 700, 2000, 10000])
 def test_walk_equal_weak_values(env, ratio):
     """Equal weak values on LORs of equal steps (along the grid and its diagonals), whose rounding
